@@ -399,64 +399,122 @@ __global__ void __launch_bounds__(256) rope_store_kernel(void* __restrict__ qkv,
 // One block per (row, query head).  Row t with position p sees keys [lo, p] where
 // lo = max(0, p + 1 - window) (window 0 = all).  Keys are taken in chunks of 128 from lo
 // upward with an online softmax; everything is fp32 (src/hip_ops.hip:473-551).
-constexpr int ATT_THREADS = 128;
+//
+// A block's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
+// output element, chunk after chunk.  The keys of a chunk come in slices of 32 elements through two buffers of shared
+// memory (cp.async, whole sectors; a thread reads its own key's slice 16 bytes at a time, rows 144 bytes apart: no bank
+// conflicts), so the chain waits for no load; the values' loads are asked for eight at a time; the trees end in one warp.
+// The order of every sum is that of the element-by-element form, bit for bit.  SEE_FIGURES
+constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_ROW = ATT_SLICE + 4;
+
+template <bool MAX>
+__device__ __forceinline__ float chunk_tree(float v, float* red, int tid) {
+  red[tid] = v;
+  __syncthreads();
+  if (tid < 32) {
+    // (the pairs of a halving tree: tid with tid + 64, then + 32, + 16, ... + 1)
+    auto two = [](float a, float b) { return MAX ? fmaxf(a, b) : a + b; };
+    float x = two(two(red[tid], red[tid + 64]), two(red[tid + 32], red[tid + 96]));
+#pragma unroll
+    for (int st = 16; st > 0; st >>= 1) x = two(x, __shfl_down_sync(0xffffffffu, x, st));
+    if (tid == 0) red[0] = x;
+  }
+  __syncthreads();
+  const float all = red[0];
+  __syncthreads();
+  return all;
+}
+
+template <typename TC>
+__device__ __forceinline__ void stage_keys(float (*dst)[ATT_ROW], const TC* kc, const int* pslot, int cnt, int D, int d0, int tid) {
+  if constexpr (sizeof(TC) == 4) {
+    if (D % 4 == 0 && (uintptr_t)kc % 16 == 0) {
+      for (int i = tid; i < cnt * (ATT_SLICE / 4); i += ATT_THREADS) {
+        const int j = i / (ATT_SLICE / 4), d = d0 + i % (ATT_SLICE / 4) * 4;
+        if (d < D)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&dst[j][d - d0])),
+                       "l"(kc + (size_t)pslot[j] * D + d)
+                       : "memory");
+      }
+      return;
+    }
+  }
+  for (int i = tid; i < cnt * ATT_SLICE; i += ATT_THREADS) {
+    const int j = i / ATT_SLICE, d = d0 + i % ATT_SLICE;
+    if (d < D) dst[j][d - d0] = to_f32(kc[(size_t)pslot[j] * D + d]);
+  }
+}
+
+template <typename TC>
 __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
-    const void* __restrict__ qkv, int dt, int q_stride, const void* __restrict__ kc, const void* __restrict__ vc,
-    int cache_dt, const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_entry,
+    const void* __restrict__ qkv, int dt, int q_stride, const TC* __restrict__ kc, const TC* __restrict__ vc,
+    const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_entry,
     const int* __restrict__ positions, float scale, int window, void* __restrict__ out, int out_dt,
     int Hq, int Hkv, int D, int page) {
   __shared__ float q[256];
   __shared__ float p[ATT_THREADS];
   __shared__ int pslot[ATT_THREADS];   // element offset / D of each key of the chunk
   __shared__ float red[ATT_THREADS];
+  __shared__ __align__(16) float keys[2][ATT_THREADS][ATT_ROW];
+  grid_dep_wait();
+  grid_dep_launch();
   const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int kvh = h / (Hq / Hkv);
   const int n = positions[t] + 1;
   const int lo = window > 0 ? max(0, n - window) : 0;
   const int* bt = block_table + (size_t)row_entry[t] * max_blocks;
   for (int d = tid; d < D; d += ATT_THREADS) q[d] = ld_dt(qkv, dt, (size_t)t * q_stride + (size_t)h * D + d);
-  __syncthreads();
+  const int slices = (D + ATT_SLICE - 1) / ATT_SLICE;
   float m = -1e30f, l = 0.f;
   float o0 = 0.f, o1 = 0.f;  // this thread's output elements d = tid and tid + 128
   for (int c0 = lo; c0 < n; c0 += ATT_THREADS) {
-    const int j = c0 + tid;
-    float s = -1e30f;
-    if (j < n) {
-      int blk = bt[j / page];
-      size_t slot = ((size_t)blk * Hkv + kvh) * page + j % page;
-      pslot[tid] = (int)slot;
-      float acc = 0.f;
-      for (int d = 0; d < D; ++d) acc = fmaf(q[d], ld_dt(kc, cache_dt, slot * D + d), acc);
-      s = acc * scale;
-    }
-    red[tid] = s;
+    const int j = c0 + tid, cnt = min(ATT_THREADS, n - c0);
+    if (j < n) pslot[tid] = (bt[j / page] * Hkv + kvh) * page + j % page;
     __syncthreads();
-    for (int st = ATT_THREADS / 2; st > 0; st >>= 1) {
-      if (tid < st) red[tid] = fmaxf(red[tid], red[tid + st]);
+    stage_keys(keys[0], kc, pslot, cnt, D, 0, tid);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float acc = 0.f;
+    for (int sl = 0; sl < slices; ++sl) {
+      if (sl + 1 < slices) stage_keys(keys[(sl + 1) & 1], kc, pslot, cnt, D, (sl + 1) * ATT_SLICE, tid);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      const int dn = min(ATT_SLICE, D - sl * ATT_SLICE);
+      const float* kr = keys[sl & 1][tid];
+      const float* qr = q + sl * ATT_SLICE;
+      if (j < n) {
+        if (dn == ATT_SLICE) {
+#pragma unroll
+          for (int d = 0; d < ATT_SLICE; d += 4) {
+            const float4 k4 = *(const float4*)(kr + d);
+            acc = fmaf(qr[d], k4.x, acc);
+            acc = fmaf(qr[d + 1], k4.y, acc);
+            acc = fmaf(qr[d + 2], k4.z, acc);
+            acc = fmaf(qr[d + 3], k4.w, acc);
+          }
+        } else {
+          for (int d = 0; d < dn; ++d) acc = fmaf(qr[d], kr[d], acc);
+        }
+      }
       __syncthreads();
     }
-    const float m_new = fmaxf(m, red[0]);
-    __syncthreads();
+    const float s = j < n ? acc * scale : -1e30f;
+    const float m_new = fmaxf(m, chunk_tree<true>(s, red, tid));
     const float e = j < n ? expf(s - m_new) : 0.f;
     p[tid] = e;
-    red[tid] = e;
-    __syncthreads();
-    for (int st = ATT_THREADS / 2; st > 0; st >>= 1) {
-      if (tid < st) red[tid] += red[tid + st];
-      __syncthreads();
-    }
+    const float sum = chunk_tree<false>(e, red, tid);
     const float alpha = expf(m - m_new);
-    l = l * alpha + red[0];
+    l = l * alpha + sum;
     m = m_new;
-    const int cnt = min(ATT_THREADS, n - c0);
     o0 *= alpha;
     o1 *= alpha;
     if (tid < D) {
-      for (int i = 0; i < cnt; ++i) o0 = fmaf(p[i], ld_dt(vc, cache_dt, (size_t)pslot[i] * D + tid), o0);
+#pragma unroll 8
+      for (int i = 0; i < cnt; ++i) o0 = fmaf(p[i], to_f32(vc[(size_t)pslot[i] * D + tid]), o0);
     }
     if (tid + ATT_THREADS < D) {
-      for (int i = 0; i < cnt; ++i)
-        o1 = fmaf(p[i], ld_dt(vc, cache_dt, (size_t)pslot[i] * D + tid + ATT_THREADS), o1);
+#pragma unroll 8
+      for (int i = 0; i < cnt; ++i) o1 = fmaf(p[i], to_f32(vc[(size_t)pslot[i] * D + tid + ATT_THREADS]), o1);
     }
     __syncthreads();
   }
@@ -686,9 +744,14 @@ NV_API int nv_paged_attention_plain(const void* qkv, int dt, int q_stride, const
   if (D > 256 || D <= 0 || Hkv <= 0 || Hq % Hkv) return NV_ERR_UNSUPPORTED;
   if (T == 0) return NV_OK;
   dim3 grid(T, Hq);
-  paged_attention_plain_kernel<<<grid, ATT_THREADS, 0, s>>>(qkv, dt, q_stride, kc, vc, cache_dt, block_table,
-                                                            max_blocks, row_entry, positions, scale, window, out,
-                                                            out_dt, Hq, Hkv, D, page);
+  if (cache_dt == NV_DT_F32)
+    NV_RETURN_IF(launch_dep(paged_attention_plain_kernel<float>, grid, dim3(ATT_THREADS), 0, s, qkv, dt, q_stride, (const float*)kc,
+                            (const float*)vc, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt,
+                            Hq, Hkv, D, page));
+  else
+    NV_RETURN_IF(launch_dep(paged_attention_plain_kernel<bf16>, grid, dim3(ATT_THREADS), 0, s, qkv, dt, q_stride, (const bf16*)kc,
+                            (const bf16*)vc, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt,
+                            Hq, Hkv, D, page));
   NV_RETURN_LAST();
 }
 

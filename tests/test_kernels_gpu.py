@@ -135,6 +135,29 @@ def test_gemm_plain_rows_do_not_depend_on_the_batch():
         assert torch.equal(one[0], full[r])         # bit for bit
 
 
+@pytest.mark.parametrize("K", [4, 127, 128, 129, 333, 516])
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_gemm_plain_forms_give_the_same_bits(K, ta, tw, swiglu):
+    """Blocks of 32 features for many rows, of 16 for few, and every row count of a half-warp: one chain per output."""
+    o = ops()
+    N = 32 * 74 + 5
+    a, w = rnd(130, K, dtype=ta), rnd(2 * N if swiglu else N, K, dtype=tw, seed=1)
+    full = torch.empty(130, N, device=DEV)
+    o.gemm_plain(a, w, full, swiglu=swiglu)
+    z = a.double() @ w.double().T
+    close(full, torch.nn.functional.silu(z[:, :N]) * z[:, N:] if swiglu else z, 2e-6, "wide form")
+    for rows in (1, 7, 8, 9, 16, 17, 32, 33, 63):
+        few = torch.empty(rows, N, device=DEV)
+        o.gemm_plain(a[130 - rows:], w, few, swiglu=swiglu)
+        assert torch.equal(few, full[130 - rows:])
+    shifted = torch.zeros(130, K + 3, dtype=ta, device=DEV)[:, 1:1 + K]        # rows that do not start on 16 bytes
+    shifted.copy_(a)
+    again = torch.empty(130, N, device=DEV)
+    o.gemm_plain(shifted, w, again, swiglu=swiglu)
+    assert torch.equal(again, full)
+
+
 # ------------------------------------------------------------------------------- tensor-core product
 def tc_case(M, N, K, swiglu, bias, out_dtype, splits=None, seed=0):
     o = ops()
