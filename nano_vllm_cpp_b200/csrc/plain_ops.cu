@@ -396,33 +396,38 @@ __global__ void __launch_bounds__(256) rope_store_kernel(void* __restrict__ qkv,
 }
 
 // --------------------------------------------------------------- paged attention (plain)
-// One block per (row, query head).  Row t with position p sees keys [lo, p] where
+// One block per row and HB query heads of one kv head.  Row t with position p sees keys [lo, p] where
 // lo = max(0, p + 1 - window) (window 0 = all).  Keys are taken in chunks of 128 from lo
 // upward with an online softmax; everything is fp32 (src/hip_ops.hip:473-551).
 //
-// A block's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
-// output element, chunk after chunk.  The keys of a chunk come in slices of 32 elements through two buffers of shared
-// memory (cp.async, whole sectors; a thread reads its own key's slice 16 bytes at a time, rows 144 bytes apart: no bank
-// conflicts), so the chain waits for no load; the values' loads are asked for eight at a time; the trees end in one warp.
-// The order of every sum is that of the element-by-element form, bit for bit.  SEE_FIGURES
-constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_ROW = ATT_SLICE + 4;
+// A chunk's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
+// output element.  The heads of a block share the keys and values they read and run their chains side by side.  Keys come
+// in slices of 32 elements through NB buffers of shared memory (cp.async, whole sectors; a thread reads its own key's slice 16 bytes at a
+// time, rows 144 bytes apart: no bank conflicts): two where many blocks hide each other's waits, four, so that a chunk's
+// keys are asked for at once, where a few rows leave multiprocessors idle.  Values are asked for 32 keys ahead, the first
+// before the scores.  The order of every sum is that of the element-by-element form, bit for bit.
+// Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 102 us element by element, 45 with keys in
+// slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.
+constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_ROW = ATT_SLICE + 4, ATT_AHEAD = 32;
 
-template <bool MAX>
-__device__ __forceinline__ float chunk_tree(float v, float* red, int tid) {
-  red[tid] = v;
+template <bool MAX, int HB>
+__device__ __forceinline__ void chunk_trees(float (&v)[HB], float (*red)[ATT_THREADS], int tid) {
+  auto two = [](float a, float b) { return MAX ? fmaxf(a, b) : a + b; };
+#pragma unroll
+  for (int b = 0; b < HB; ++b) red[b][tid] = v[b];
   __syncthreads();
-  if (tid < 32) {
-    // (the pairs of a halving tree: tid with tid + 64, then + 32, + 16, ... + 1)
-    auto two = [](float a, float b) { return MAX ? fmaxf(a, b) : a + b; };
-    float x = two(two(red[tid], red[tid + 64]), two(red[tid + 32], red[tid + 96]));
+  for (int b = tid / 32; b < HB; b += ATT_THREADS / 32) {
+    // (the pairs of a halving tree: i with i + 64, then + 32, + 16, ... + 1)
+    const int i = tid % 32;
+    float x = two(two(red[b][i], red[b][i + 64]), two(red[b][i + 32], red[b][i + 96]));
 #pragma unroll
     for (int st = 16; st > 0; st >>= 1) x = two(x, __shfl_down_sync(0xffffffffu, x, st));
-    if (tid == 0) red[0] = x;
+    if (i == 0) red[b][0] = x;
   }
   __syncthreads();
-  const float all = red[0];
+#pragma unroll
+  for (int b = 0; b < HB; ++b) v[b] = red[b][0];
   __syncthreads();
-  return all;
 }
 
 template <typename TC>
@@ -445,83 +450,141 @@ __device__ __forceinline__ void stage_keys(float (*dst)[ATT_ROW], const TC* kc, 
   }
 }
 
-template <typename TC>
+template <typename TC, int HB, int NB>
 __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     const void* __restrict__ qkv, int dt, int q_stride, const TC* __restrict__ kc, const TC* __restrict__ vc,
     const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_entry,
     const int* __restrict__ positions, float scale, int window, void* __restrict__ out, int out_dt,
     int Hq, int Hkv, int D, int page) {
-  __shared__ float q[256];
-  __shared__ float p[ATT_THREADS];
+  extern __shared__ __align__(16) float att_keys[];
+  __shared__ __align__(16) float q[HB][256];
+  __shared__ float p[HB][ATT_THREADS];
   __shared__ int pslot[ATT_THREADS];   // element offset / D of each key of the chunk
-  __shared__ float red[ATT_THREADS];
-  __shared__ __align__(16) float keys[2][ATT_THREADS][ATT_ROW];
+  __shared__ float red[HB][ATT_THREADS];
+  float(*keys)[ATT_THREADS][ATT_ROW] = (float(*)[ATT_THREADS][ATT_ROW])att_keys;
   grid_dep_wait();
   grid_dep_launch();
-  const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  const int kvh = h / (Hq / Hkv);
+  const int t = blockIdx.x, h0 = blockIdx.y * HB, tid = threadIdx.x;
+  const int kvh = h0 / (Hq / Hkv);
   const int n = positions[t] + 1;
   const int lo = window > 0 ? max(0, n - window) : 0;
   const int* bt = block_table + (size_t)row_entry[t] * max_blocks;
-  for (int d = tid; d < D; d += ATT_THREADS) q[d] = ld_dt(qkv, dt, (size_t)t * q_stride + (size_t)h * D + d);
+  for (int i = tid; i < HB * D; i += ATT_THREADS) q[i / D][i % D] = ld_dt(qkv, dt, (size_t)t * q_stride + (size_t)h0 * D + i);
   const int slices = (D + ATT_SLICE - 1) / ATT_SLICE;
-  float m = -1e30f, l = 0.f;
-  float o0 = 0.f, o1 = 0.f;  // this thread's output elements d = tid and tid + 128
+  const int halves = (D + ATT_THREADS - 1) / ATT_THREADS;    // output elements of a thread: d = tid and, above 128, tid + 128
+  float m[HB], l[HB], o[2][HB];
+#pragma unroll
+  for (int b = 0; b < HB; ++b) { m[b] = -1e30f; l[b] = 0.f; o[0][b] = o[1][b] = 0.f; }
   for (int c0 = lo; c0 < n; c0 += ATT_THREADS) {
     const int j = c0 + tid, cnt = min(ATT_THREADS, n - c0);
     if (j < n) pslot[tid] = (bt[j / page] * Hkv + kvh) * page + j % page;
     __syncthreads();
-    stage_keys(keys[0], kc, pslot, cnt, D, 0, tid);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    float acc = 0.f;
-    for (int sl = 0; sl < slices; ++sl) {
-      if (sl + 1 < slices) stage_keys(keys[(sl + 1) & 1], kc, pslot, cnt, D, (sl + 1) * ATT_SLICE, tid);
+    for (int sl = 0; sl < NB - 1; ++sl) {
+      if (sl < slices) stage_keys(keys[sl], kc, pslot, cnt, D, sl * ATT_SLICE, tid);
       asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
+    float val[ATT_AHEAD];
+#pragma unroll
+    for (int i = 0; i < ATT_AHEAD; ++i) val[i] = tid < D && i < cnt ? to_f32(vc[(size_t)pslot[i] * D + tid]) : 0.f;
+    float s[HB];
+#pragma unroll
+    for (int b = 0; b < HB; ++b) s[b] = 0.f;
+    for (int sl = 0; sl < slices; ++sl) {
+      if (sl + NB - 1 < slices) stage_keys(keys[(sl + NB - 1) % NB], kc, pslot, cnt, D, (sl + NB - 1) * ATT_SLICE, tid);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group %0;" ::"n"(NB - 1) : "memory");
       __syncthreads();
       const int dn = min(ATT_SLICE, D - sl * ATT_SLICE);
-      const float* kr = keys[sl & 1][tid];
-      const float* qr = q + sl * ATT_SLICE;
+      const float* kr = keys[sl % NB][tid];
       if (j < n) {
         if (dn == ATT_SLICE) {
 #pragma unroll
           for (int d = 0; d < ATT_SLICE; d += 4) {
             const float4 k4 = *(const float4*)(kr + d);
-            acc = fmaf(qr[d], k4.x, acc);
-            acc = fmaf(qr[d + 1], k4.y, acc);
-            acc = fmaf(qr[d + 2], k4.z, acc);
-            acc = fmaf(qr[d + 3], k4.w, acc);
+#pragma unroll
+            for (int b = 0; b < HB; ++b) {
+              const float4 q4 = *(const float4*)(q[b] + sl * ATT_SLICE + d);
+              s[b] = fmaf(q4.x, k4.x, s[b]);
+              s[b] = fmaf(q4.y, k4.y, s[b]);
+              s[b] = fmaf(q4.z, k4.z, s[b]);
+              s[b] = fmaf(q4.w, k4.w, s[b]);
+            }
           }
         } else {
-          for (int d = 0; d < dn; ++d) acc = fmaf(qr[d], kr[d], acc);
+          for (int d = 0; d < dn; ++d)
+#pragma unroll
+            for (int b = 0; b < HB; ++b) s[b] = fmaf(q[b][sl * ATT_SLICE + d], kr[d], s[b]);
         }
       }
       __syncthreads();
     }
-    const float s = j < n ? acc * scale : -1e30f;
-    const float m_new = fmaxf(m, chunk_tree<true>(s, red, tid));
-    const float e = j < n ? expf(s - m_new) : 0.f;
-    p[tid] = e;
-    const float sum = chunk_tree<false>(e, red, tid);
-    const float alpha = expf(m - m_new);
-    l = l * alpha + sum;
-    m = m_new;
-    o0 *= alpha;
-    o1 *= alpha;
-    if (tid < D) {
-#pragma unroll 8
-      for (int i = 0; i < cnt; ++i) o0 = fmaf(p[i], to_f32(vc[(size_t)pslot[i] * D + tid]), o0);
+    float top[HB], sum[HB];
+#pragma unroll
+    for (int b = 0; b < HB; ++b) top[b] = s[b] = j < n ? s[b] * scale : -1e30f;
+    chunk_trees<true, HB>(top, red, tid);
+#pragma unroll
+    for (int b = 0; b < HB; ++b) {
+      const float m_new = fmaxf(m[b], top[b]);
+      p[b][tid] = sum[b] = j < n ? expf(s[b] - m_new) : 0.f;
+      top[b] = expf(m[b] - m_new);                           // what the sums so far are worth now
+      m[b] = m_new;
     }
-    if (tid + ATT_THREADS < D) {
-#pragma unroll 8
-      for (int i = 0; i < cnt; ++i) o1 = fmaf(p[i], to_f32(vc[(size_t)pslot[i] * D + tid + ATT_THREADS]), o1);
+    chunk_trees<false, HB>(sum, red, tid);
+#pragma unroll
+    for (int b = 0; b < HB; ++b) {
+      l[b] = l[b] * top[b] + sum[b];
+      o[0][b] *= top[b];
+      o[1][b] *= top[b];
+    }
+    for (int half = 0; half < halves; ++half) {
+      const int d = tid + half * ATT_THREADS;
+      for (int i0 = 0; i0 < cnt; i0 += ATT_AHEAD) {
+        float now[ATT_AHEAD];
+#pragma unroll
+        for (int i = 0; i < ATT_AHEAD; ++i) now[i] = val[i];
+        const bool wrap = i0 + ATT_AHEAD >= cnt;             // the values after this half's are the next half's first
+        const int nd = wrap ? d + ATT_THREADS : d, ni = wrap ? 0 : i0 + ATT_AHEAD;
+        if (!wrap || half + 1 < halves) {
+#pragma unroll
+          for (int i = 0; i < ATT_AHEAD; ++i)
+            val[i] = nd < D && ni + i < cnt ? to_f32(vc[(size_t)pslot[ni + i] * D + nd]) : 0.f;
+        }
+        const int k = min(ATT_AHEAD, cnt - i0);
+#pragma unroll
+        for (int i = 0; i < ATT_AHEAD; ++i)
+          if (i < k) {
+#pragma unroll
+            for (int b = 0; b < HB; ++b) {
+              const float w = p[b][i0 + i];
+              if (half == 0) o[0][b] = fmaf(w, now[i], o[0][b]);
+              else o[1][b] = fmaf(w, now[i], o[1][b]);
+            }
+          }
+      }
     }
     __syncthreads();
   }
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  const size_t ob = (size_t)t * Hq * D + (size_t)h * D;
-  if (tid < D) st_dt(out, out_dt, ob + tid, o0 * inv);
-  if (tid + ATT_THREADS < D) st_dt(out, out_dt, ob + tid + ATT_THREADS, o1 * inv);
+#pragma unroll
+  for (int b = 0; b < HB; ++b) {
+    const float inv = l[b] > 0.f ? 1.f / l[b] : 0.f;
+    const size_t ob = (size_t)t * Hq * D + (size_t)(h0 + b) * D;
+    if (tid < D) st_dt(out, out_dt, ob + tid, o[0][b] * inv);
+    if (tid + ATT_THREADS < D) st_dt(out, out_dt, ob + tid + ATT_THREADS, o[1][b] * inv);
+  }
+}
+
+template <typename TC, int HB>
+int launch_plain_attention(const void* qkv, int dt, int q_stride, const TC* kc, const TC* vc, const int* block_table,
+                           int max_blocks, const int* row_entry, const int* positions, float scale, int window, void* out,
+                           int out_dt, int T, int Hq, int Hkv, int D, int page, cudaStream_t s) {
+  const dim3 grid(T, Hq / HB);
+  const bool few = (long long)T * (Hq / HB) <= 2 * 148;      // (four buffers leave a multiprocessor room for three blocks)
+  const size_t smem = (few ? 4 : 2) * sizeof(float) * ATT_THREADS * ATT_ROW;
+  auto* kernel = few ? paged_attention_plain_kernel<TC, HB, 4> : paged_attention_plain_kernel<TC, HB, 2>;
+  if (few) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NV_RETURN_IF(launch_dep(kernel, grid, dim3(ATT_THREADS), smem, s, qkv, dt, q_stride, kc, vc, block_table, max_blocks, row_entry,
+                          positions, scale, window, out, out_dt, Hq, Hkv, D, page));
+  NV_RETURN_LAST();
 }
 
 // ----------------------------------------------------------------------- router, expert permutation
@@ -743,16 +806,19 @@ NV_API int nv_paged_attention_plain(const void* qkv, int dt, int q_stride, const
   if (!dt_ok(dt) || !dt_ok(cache_dt) || !dt_ok(out_dt)) return NV_ERR_BAD_DTYPE;
   if (D > 256 || D <= 0 || Hkv <= 0 || Hq % Hkv) return NV_ERR_UNSUPPORTED;
   if (T == 0) return NV_OK;
-  dim3 grid(T, Hq);
-  if (cache_dt == NV_DT_F32)
-    NV_RETURN_IF(launch_dep(paged_attention_plain_kernel<float>, grid, dim3(ATT_THREADS), 0, s, qkv, dt, q_stride, (const float*)kc,
-                            (const float*)vc, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt,
-                            Hq, Hkv, D, page));
-  else
-    NV_RETURN_IF(launch_dep(paged_attention_plain_kernel<bf16>, grid, dim3(ATT_THREADS), 0, s, qkv, dt, q_stride, (const bf16*)kc,
-                            (const bf16*)vc, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt,
-                            Hq, Hkv, D, page));
-  NV_RETURN_LAST();
+  auto go = [&](auto* k, auto* v) {
+    // (a few rows: a block per head, since there are multiprocessors for all of them; many: heads share what they read)
+    const int group = (long long)T * Hq <= 4 * 148 ? 1 : Hq / Hkv;
+    if (group % 4 == 0)
+      return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 4>(
+          qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
+    if (group % 2 == 0)
+      return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 2>(
+          qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
+    return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 1>(
+        qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
+  };
+  return cache_dt == NV_DT_F32 ? go((const float*)kc, (const float*)vc) : go((const bf16*)kc, (const bf16*)vc);
 }
 
 NV_API int nv_router_topk(const float* logits, long long ld, int T, int E, int K, int renorm, int* idx,
