@@ -150,6 +150,32 @@ __device__ __forceinline__ void chunk_pair(float (&g)[W], const float (&u)[W], f
   for (int j = 0; j < W; ++j) g[j] = pair_mul(PAIR, g[j], u[j], p0, p1);
 }
 
+template <int W, bool RAGGED>
+__device__ __forceinline__ void store_chunk(const TcArgs& a, const Tile& t, size_t row, int n, int n2, bool n2_ok,
+                                            const float (&g)[W], const float (&u)[W], int valid) {
+  if (a.out_dt == NV_DT_BF16) {
+    bf16* o = (bf16*)a.out + row * a.ldo + t.o_col0;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (!RAGGED || j < valid) o[(size_t)j * a.ldo + n] = __float2bfloat16_rn(g[j]);
+    if (n2_ok) {
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        if (!RAGGED || j < valid) o[(size_t)j * a.ldo + n2] = __float2bfloat16_rn(u[j]);
+    }
+  } else {
+    float* o = (float*)a.out + row * a.ldo + t.o_col0;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (!RAGGED || j < valid) o[(size_t)j * a.ldo + n] = g[j];
+    if (n2_ok) {
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        if (!RAGGED || j < valid) o[(size_t)j * a.ldo + n2] = u[j];
+    }
+  }
+}
+
 template <int W>
 __device__ __forceinline__ void epilogue_chunk(const TcArgs& a, const Tile& t, int two, uint32_t taddr, int c0, int n,
                                                int n2, bool n_ok, bool n2_ok, float bias, float bias2) {
@@ -189,8 +215,8 @@ __device__ __forceinline__ void epilogue_chunk(const TcArgs& a, const Tile& t, i
     }
     return;
   }
-  if (valid < W) {
-    // a ragged chunk (the few rows of an expert's tile while decoding): only the rows that exist are worked out
+  if (valid <= W / 4) {
+    // a short chunk (the few rows of an expert's tile while decoding): only the rows that exist are worked out
 #pragma unroll
     for (int j = 0; j < W; ++j) {
       if (j < valid) {
@@ -232,22 +258,11 @@ __device__ __forceinline__ void epilogue_chunk(const TcArgs& a, const Tile& t, i
       break;
     default: chunk_act<W, NV_EPI_RELU2>(g, u, a.act_p0, a.act_p1); break;
   }
-  if (a.out_dt == NV_DT_BF16) {
-    bf16* o = (bf16*)a.out + row * a.ldo + t.o_col0;
-#pragma unroll
-    for (int j = 0; j < W; ++j) o[(size_t)j * a.ldo + n] = __float2bfloat16_rn(g[j]);
-    if (n2_ok) {
-#pragma unroll
-      for (int j = 0; j < W; ++j) o[(size_t)j * a.ldo + n2] = __float2bfloat16_rn(u[j]);
-    }
+  if (valid < W) {       // (a ragged chunk stores fewer rows: element by element through the codes it made a prompt of
+                         // 1,500 rows slower than one of 2,048, 39 against 22 us for 2,048 x 2,048)
+    store_chunk<W, true>(a, t, row, n, n2, n2_ok, g, u, valid);
   } else {
-    float* o = (float*)a.out + row * a.ldo + t.o_col0;
-#pragma unroll
-    for (int j = 0; j < W; ++j) o[(size_t)j * a.ldo + n] = g[j];
-    if (n2_ok) {
-#pragma unroll
-      for (int j = 0; j < W; ++j) o[(size_t)j * a.ldo + n2] = u[j];
-    }
+    store_chunk<W, false>(a, t, row, n, n2, n2_ok, g, u, valid);
   }
 }
 
@@ -685,6 +700,11 @@ NV_API int nv_tc_gemm_splits(int M_tok, int N, int K, int n_tile, int num_sms) {
   int s = (M_tok <= 64 ? 2 * num_sms : num_sms) / ctas;
   if (s > k_steps / 4) s = k_steps / 4;
   if (s > 16) s = 16;
+  // With tiles of 128 tokens and more a k-step takes some 0.48 us and the partial sums are big: what the parts save of
+  // the chain of k-steps has to pay for writing and reading them and for the second kernel.  (Measured, float32 out: 1,000 rows,
+  // 2,048 x 2,048 in two parts 36 us, whole 22; 1,500 rows, 1,024 x 1,024 in three 31, whole 15; 512 rows, 1,024 x 4,096
+  // in nine 22, whole 32.)
+  if (M_tok >= 128 && s > 1 && 0.48 * k_steps * (s - 1) / s < 8.0 + 1.5e-6 * s * M_tok * N) return 1;
   return s < 1 ? 1 : s;
 }
 

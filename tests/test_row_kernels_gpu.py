@@ -1,0 +1,137 @@
+"""Kernels over many rows where they can go wrong: edges of their blocks and vectors, rows that begin a sequence inside a
+block, and the general forms beside the wide ones."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from nano_vllm_cpp_b200.csrc import ops as o
+    return o
+
+
+def rnd(*shape, seed=0, dtype=torch.float32):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV).to(dtype)
+
+
+@pytest.mark.parametrize("lens", [[1], [1, 1, 2, 3, 4], [5, 9, 1, 17, 8], [700, 1, 2, 490]])
+@pytest.mark.parametrize("C,unit_heads,unit_dim,col0", [(96, 2, 16, 0), (3072, 8, 128, 4), (40, 0, 1, 8), (42, 1, 8, 0), (96, 2, 16, 1)])
+def test_convolution_of_four_taps(lens, C, unit_heads, unit_dim, col0):
+    """Every entry continues from a state of its own; sizes and columns off 16 bytes take the general kernel."""
+    o, T, S = ops(), sum(lens), len(lens)
+    src, w, state = rnd(T, C + 12, seed=1), rnd(C, 4, seed=2), rnd(S, 3, C, seed=3)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    entry = torch.repeat_interleave(torch.arange(S), torch.tensor(lens)).to(torch.int32).to(DEV)
+    slot = torch.arange(S, dtype=torch.int32, device=DEV).flip(0).contiguous()
+    out = torch.empty(T, C, device=DEV)
+    o.conv_silu_norm(src, col0, C, w, 4, types.SimpleNamespace(row_entry=entry, cu_rows=cu, entry_slot=slot), state, out,
+                     unit_heads=unit_heads, unit_dim=unit_dim, unit_eps=1e-6, scaled_heads=unit_heads // 2, scale=0.25)
+    want = []
+    for e, n in enumerate(lens):
+        x = torch.cat([state[int(slot[e])], src[int(cu[e]):int(cu[e]) + n, col0:col0 + C]]).double()
+        want.append(torch.nn.functional.silu(sum(x[d:d + n] * w[:, d].double() for d in range(4))))
+    want = torch.cat(want)
+    for h in range(unit_heads):
+        y = want[:, h * unit_dim:(h + 1) * unit_dim]
+        y /= torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6)
+        y *= 0.25 if h < unit_heads // 2 else 1.0
+    # four products, a sigmoid and a sum of unit_dim squares in float32: some ten roundings
+    assert float((out.double() - want).abs().max()) <= 2e-6 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("T,H,G,D", [(1, 4, 4, 16), (3, 4, 2, 24), (70, 16, 4, 128), (5, 16, 2, 64), (4, 6, 2, 16), (3, 4, 2, 10)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_mixed_queries(T, H, G, D, dtype):
+    o = ops()
+    q, mix = rnd(T, H * D, seed=1), rnd(H, H, seed=2)
+    out = torch.empty(T, H * G * D, dtype=dtype, device=DEV)
+    o.mix_query_heads(q, mix, out, H, G, D)
+    rep = H // G
+    want = torch.einsum("hcg,tcgd->thcd", mix.double().view(H, G, rep), q.double().view(T, G, rep, D)).reshape(T, -1)
+    bound = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-6 * float(want.abs().max())
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("T,H,D,dims", [(1, 2, 16, 16), (300, 16, 128, 64), (7, 3, 20, 6), (2, 2, 8, 0)])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_turned_heads(T, H, D, dims, sign):
+    o = ops()
+    x, pos = rnd(T, H * D, seed=1), torch.randint(0, 3000, (T,), dtype=torch.int32, device=DEV)
+    inv = (10.0 ** -(torch.arange(max(1, dims // 2)) / 4.0)).float().to(DEV)
+    out = torch.empty_like(x)
+    o.rotate_heads(x, pos, inv, dims, sign, out, H, D)
+    ang = (sign * pos.float()[:, None] * inv[None, :dims // 2]).double()[:, None]       # (the angle is a float32 product)
+    v, half = x.double().view(T, H, D), dims // 2
+    a, b = v[..., :half], v[..., half:dims]
+    want = torch.cat([a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin(), v[..., dims:]], -1).reshape(T, -1)
+    assert float((out.double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("T,H,N", [(1, 1, 4), (300, 16, 128), (5, 3, 6), (3, 2, 5)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_heads(T, H, N, dtype):
+    o = ops()
+    x, gate = rnd(T, H * N, seed=1), rnd(T, H + 3, seed=2)
+    out = torch.empty(T, H * N, dtype=dtype, device=DEV)
+    o.head_gate(x, gate, 2, out, H, N)
+    want = (x.double().view(T, H, N) * gate[:, 2:2 + H].double().sigmoid()[..., None]).reshape(T, -1)
+    bound = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-6 * float(want.abs().max())
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M", [129, 255, 257, 300, 1500])
+@pytest.mark.parametrize("N,K", [(256, 128), (1024, 1024), (3000, 264)])
+@pytest.mark.parametrize("how", ["plain", "swiglu", "gelu_erf"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_ragged_token_tiles_of_the_tensor_core_product(M, N, K, how, dtype):
+    o = ops()
+    a, w = rnd(M, K, seed=1, dtype=torch.bfloat16), rnd(2 * N if how == "swiglu" else N, K, seed=2, dtype=torch.bfloat16) * 0.03125
+    out = torch.full((M + 1, N), 7.0, dtype=dtype, device=DEV)
+    o.gemm_fast(a, w, out[:M], swiglu=how == "swiglu", act="gelu_erf" if how == "gelu_erf" else None)
+    z = a.double() @ w.double().T
+    want = z if how == "plain" else torch.nn.functional.silu(z[:, :N]) * z[:, N:] if how == "swiglu" else torch.nn.functional.gelu(z)
+    # bfloat16 rounds by 2^-9 of the value; K / 16 partial sums are each off by at most 2^-23 of the largest
+    bound = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + K / 8 * 2.0 ** -23 * float(want.abs().max()) + 2e-6
+    assert bool(((out[:M].double() - want).abs() <= bound).all()) and bool((out[M] == 7.0).all())
+
+
+def paged(lens, Hkv, D, seed, page=16):
+    blocks = [(n + page - 1) // page for n in lens]
+    bt = torch.full((len(lens), max(blocks)), -1, dtype=torch.int32)
+    at = 0
+    for i, b in enumerate(blocks):
+        bt[i, :b] = torch.arange(at, at + b)
+        at += b
+    kc, vc = rnd(at, Hkv, page, D, seed=seed, dtype=torch.bfloat16), rnd(at, Hkv, page, D, seed=seed + 1, dtype=torch.bfloat16)
+    return kc, vc, bt.to(DEV)
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D", [([1, 16, 17, 530], 4, 2, 64), ([3, 700] * 40, 16, 16, 128), ([1500], 8, 2, 128)])
+@pytest.mark.parametrize("sink", [None, 0.0, 4.0])
+@pytest.mark.parametrize("float_weights", [False, True])
+def test_decode_attention_with_a_sink_and_short_rows(lens, Hq, Hkv, D, sink, float_weights):
+    """The tensor-core form: a sink in the denominator with one split and with several, rows far shorter than the
+    longest (the second case has splits that are left empty)."""
+    o, B = ops(), len(lens)
+    kc, vc, bt = paged(lens, Hkv, D, 3)
+    q = rnd(B, Hq * D, seed=5, dtype=torch.bfloat16)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    err, out = o.ErrorFlag(DEV), torch.empty(B, Hq * D, dtype=torch.bfloat16, device=DEV)
+    o.attention_decode(q, kc, vc, bt, torch.arange(B, dtype=torch.int32, device=DEV), pos, D ** -0.5, 0, out, Hq, Hkv, D,
+                       2048, err=err, sink_score=sink, float_weights=float_weights)
+    err.check("decode")
+    for i in [i for i in range(B) if i < 4 or i > B - 3]:
+        n = lens[i]
+        rows = bt[i].long().clamp(min=0)
+        k, v = (c[rows].transpose(1, 2).reshape(-1, Hkv, D)[:n].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        s = torch.einsum("hd,nhd->hn", q[i].double().view(Hq, D), k) * D ** -0.5
+        if sink is not None:
+            s = torch.cat([s, torch.full((Hq, 1), sink, device=DEV).double()], 1)
+        want = torch.einsum("hn,nhd->hd", s.softmax(-1)[:, :n], v)
+        # one term: the weights are rounded to bfloat16, 2^-9 of a sum of weighted values of order one; the output too
+        bound = 2.0 ** -8 * want.abs() + (2e-5 if float_weights else 4e-3)
+        assert bool(((out[i].double().view(Hq, D) - want).abs() <= bound).all())
