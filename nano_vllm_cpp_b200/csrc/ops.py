@@ -1011,6 +1011,21 @@ def channel_scan_usable(dk: int, dv: int) -> bool:
     return bool(lib().nv_channel_scan_usable(dk, dv))
 
 
+# Steps with at least this many rows beyond one per entry take the memories in chunks of eight rows (memory_chunks.cuh); a
+# step of a row or two per entry would work out chunks of which one row counts (8 rows: 24 us row by row).
+CHUNK_MIN_ROWS = 32
+
+
+def _chunk_buf(out, batch, H: int, dk: int, lstm: bool):
+    """Scratch for the chunked form of a memory, or None for a step that goes row by row: one of few rows, and any step
+    of a float32 run, whose sums must not depend on how a sequence is cut into steps."""
+    T = out.shape[0]
+    if out.dtype != torch.bfloat16 or T - batch.S < CHUNK_MIN_ROWS:
+        return None
+    return torch.empty(int(lib().nv_memory_chunk_floats(T, batch.S, H, dk, 1 if lstm else 0)), dtype=torch.float32,
+                       device=out.device)
+
+
 def mlstm_scan(proj, cols: dict, batch, S, n, m, H: int, dk: int, dv: int, cap: float, eps: float, norm_w, out,
                *, den_eps: float = 1e-6, columns: bool = True) -> None:
     """The matrix memory with exponential gating, row by row per entry, from and to the entries' states.
@@ -1024,11 +1039,13 @@ def mlstm_scan(proj, cols: dict, batch, S, n, m, H: int, dk: int, dv: int, cap: 
         T = proj.shape[0]
         raw = torch.empty((T, H, dv + 2), dtype=torch.float32, device=proj.device)
         gate_buf = torch.empty((T, H, 2), dtype=torch.float32, device=proj.device)
+        chunk_buf = _chunk_buf(out, batch, H, dk, True)
         _check(lib().nv_mlstm_col_scan(_p(proj), proj.stride(0), cols["q"], cols["k"], cols["v"], cols["g"], cols["i"],
                                        cols["f"], _p(batch.cu_rows), _p(batch.entry_slot), _p(S), _slot_stride(S), _p(n),
                                        _slot_stride(n), _p(m), _slot_stride(m), H, dk, dv, cap, float(dk) ** -0.5,
                                        den_eps, eps, _p(norm_w), (1 if norm_w.numel() == H * dv and H > 1 else 0),
-                                       _p(raw), _p(gate_buf), _p(out), dt(out), batch.S, T, _stream()), "mlstm_col_scan")
+                                       _p(raw), _p(gate_buf), _p(chunk_buf), _p(out), dt(out), batch.S, T, _stream()),
+               "mlstm_col_scan")
         return
     _check(lib().nv_mlstm_scan(_p(proj), proj.stride(0), cols["q"], cols["k"], cols["v"], cols["g"], cols["i"],
                                cols["f"], _p(batch.cu_rows), _p(batch.entry_slot), _p(S), _slot_stride(S), _p(n),
@@ -1061,14 +1078,18 @@ def gated_delta_scan(qkv, cols: dict, G: int, proj, pcols: dict, A_log, dt_bias,
         if columns and col_scan_usable(dk, dv) and dec is not None and channel_scan_usable(dk, dv):
             T = qkv.shape[0]
             raw = torch.empty((T, H, dv), dtype=torch.float32, device=qkv.device)
-            gate_buf = torch.empty((T, H, 2), dtype=torch.float32, device=qkv.device)
-            decays = torch.empty((T, H * dk), dtype=torch.float32, device=qkv.device)
+            chunk_buf = _chunk_buf(out, batch, H, dk, False)
+            gate_buf = decays = None
+            if chunk_buf is None:
+                gate_buf = torch.empty((T, H, 2), dtype=torch.float32, device=qkv.device)
+                decays = torch.empty((T, H * dk), dtype=torch.float32, device=qkv.device)
             _check(lib().nv_channel_delta_scan(_p(qkv), qkv.shape[1], cols["q"], cols["k"], cols["v"], G, _p(proj),
                                                dt(proj), proj.stride(0), pcols["b"], _p(dec), dec.stride(0), pcols["a"],
                                                _p(gs), dt(gs), gs.stride(0), pcols["g"], (1 if gate == "sigmoid" else 0),
                                                _p(A_log), _p(dt_bias), _p(batch.cu_rows), _p(batch.entry_slot), _p(S),
                                                _slot_stride(S), H, dk, dv, eps, _p(norm_w), _p(raw), _p(gate_buf),
-                                               _p(decays), _p(out), dt(out), batch.S, T, _stream()), "channel_delta_scan")
+                                               _p(decays), _p(chunk_buf), _p(out), dt(out), batch.S, T, _stream()),
+                   "channel_delta_scan")
             return
         _check(lib().nv_gated_delta_scan(_p(qkv), qkv.shape[1], cols["q"], cols["k"], cols["v"], G, _p(proj), dt(proj),
                                          proj.stride(0), pcols["g"], pcols["b"], (0 if dec is not None else pcols["a"]),
@@ -1082,11 +1103,12 @@ def gated_delta_scan(qkv, cols: dict, G: int, proj, pcols: dict, A_log, dt_bias,
         T = qkv.shape[0]
         raw = torch.empty((T, H, dv), dtype=torch.float32, device=qkv.device)
         gate_buf = torch.empty((T, H, 2), dtype=torch.float32, device=qkv.device)
+        chunk_buf = _chunk_buf(out, batch, H, dk, False)
         _check(lib().nv_gated_delta_col_scan(_p(qkv), qkv.shape[1], cols["q"], cols["k"], cols["v"], G, _p(proj),
                                              dt(proj), proj.stride(0), pcols["g"], pcols["b"], pcols["a"], _p(A_log),
                                              _p(dt_bias), _p(batch.cu_rows), _p(batch.entry_slot), _p(S),
-                                             _slot_stride(S), H, dk, dv, eps, _p(norm_w), _p(raw), _p(gate_buf), _p(out),
-                                             dt(out), batch.S, T, _stream()), "gated_delta_col_scan")
+                                             _slot_stride(S), H, dk, dv, eps, _p(norm_w), _p(raw), _p(gate_buf),
+                                             _p(chunk_buf), _p(out), dt(out), batch.S, T, _stream()), "gated_delta_col_scan")
         return
     _check(lib().nv_gated_delta_scan(_p(qkv), qkv.shape[1], cols["q"], cols["k"], cols["v"], G, _p(proj), dt(proj),
                                      proj.stride(0), pcols["g"], pcols["b"], pcols["a"], _p(A_log), _p(dt_bias),

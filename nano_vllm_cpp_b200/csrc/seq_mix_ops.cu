@@ -882,7 +882,7 @@ struct ColArgs {
   long long S_stride;
   float* n;                 // matrix LSTM: [slots][H, dk]
   long long n_stride;
-  float* m;                 // matrix LSTM: [slots][H]
+  const float* m;           // matrix LSTM: [slots][H]; the new maximum goes to raw (see head_finish_kernel)
   long long m_stride;
   const float* qk;          // rows that hold q and k: [T, qk_ld]
   long long qk_ld;
@@ -1143,17 +1143,36 @@ __global__ void __launch_bounds__(COL_THREADS) col_scan_kernel(ColArgs a) {
     for (int r = 0; r < DKH; ++r)
       if (row_of(r) < dk) colp[(size_t)row_of(r) * cstride] = Sreg[r];
   }
-  if (MODE == 0 && blockIdx.z == 0 && tid == 0) a.m[(size_t)slot * a.m_stride + h] = m;
 }
 
+#include "memory_chunks.cuh"
+
 // A row and head per warp: o = raw (divided, for the matrix LSTM, by max(|n . q|, exp(-m)) + den_eps), then
-// o / sqrt(mean(o^2) + eps) * w * act(gate), act the sigmoid (gate_act 0) or silu (1).
+// o / sqrt(mean(o^2) + eps) * w * act(gate), act the sigmoid (gate_act 0) or silu (1).  Behind the blocks of the rows
+// the matrix LSTM has blocks that move the running maximum after every entry's last row to the entry's state: the scan's
+// blocks all begin with the old one, so none of them may write it.
+struct MaxState {
+  float* m;
+  long long stride;
+  const int* cu_rows;
+  const int* entry_slot;
+  int S;
+};
 __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restrict__ raw, int RW, int has_den,
                                                           float den_eps, const void* __restrict__ gate, int gate_dt,
                                                           long long gate_ld, int g0, int gate_act,
                                                           const float* __restrict__ w, int w_per_head, float eps,
-                                                          void* __restrict__ out, int out_dt, int T, int H, int dv) {
+                                                          void* __restrict__ out, int out_dt, int T, int H, int dv,
+                                                          MaxState top) {
   const int lane = threadIdx.x & 31;
+  const unsigned row_blocks = (unsigned)(((long long)T * H + 7) / 8);
+  if (blockIdx.x >= row_blocks) {
+    const long long i = (long long)(blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
+    if (i >= (long long)top.S * H) return;
+    const int e = (int)(i / H), h = (int)(i % H), last = top.cu_rows[e + 1] - 1;
+    if (last >= top.cu_rows[e]) top.m[(size_t)top.entry_slot[e] * top.stride + h] = raw[((size_t)last * H + h) * RW + dv + 1];
+    return;
+  }
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)T * H) return;
   const int t = (int)(item / H), h = (int)(item % H);
@@ -1488,66 +1507,114 @@ NV_API int nv_head_gate(const float* x, const float* gate, long long gate_ld, in
 NV_API int nv_col_scan_usable(int dk, int dv) { return dk >= 1 && dk <= 128 && dv >= 1; }
 NV_API int nv_channel_scan_usable(int dk, int dv) { return nv_col_scan_usable(dk, dv); }
 
-// The matrix LSTM through col_scan_kernel; raw: [T, H, dv + 2] and gate_buf: [T, H, 2] float32 scratch.
+// Floats of scratch that the chunked form of a memory takes (chunk_buf below); `lstm`: the matrix LSTM's.
+NV_API long long nv_memory_chunk_floats(int T, int S, int H, int dk, int lstm) {
+  const int DK = dk <= 64 ? 64 : 128;
+  return mc_records(T, S) * H * mc_record(DK, lstm != 0);
+}
+
+// The matrix LSTM through col_scan_kernel, or with `chunk_buf` through memory_chunks.cuh; raw: [T, H, dv + 2] and gate_buf:
+// [T, H, 2] float32 scratch (gate_buf is not touched by the chunked form).
 NV_API int nv_mlstm_col_scan(const float* proj, long long ld, int q0, int k0, int v0, int g0, int i0, int f0,
                              const int* cu_rows, const int* entry_slot, float* S, long long S_stride, float* n,
                              long long n_stride, float* m, long long m_stride, int H, int dk, int dv, float cap,
                              float q_scale, float den_eps, float eps, const float* norm_w, int norm_per_head,
-                             float* raw, float* gate_buf, void* out, int out_dt, int num_entries, int T,
-                             cudaStream_t s) {
+                             float* raw, float* gate_buf, float* chunk_buf, void* out, int out_dt, int num_entries,
+                             int T, cudaStream_t s) {
   if (!dt_ok(out_dt)) return NV_ERR_BAD_DTYPE;
   if (!nv_col_scan_usable(dk, dv) || H <= 0) return NV_ERR_UNSUPPORTED;
   if (num_entries == 0 || T == 0) return NV_OK;
+  int rc;
+  if (chunk_buf) {
+    ChunkArgs p = {};
+    p.cu_rows = cu_rows; p.S_entries = num_entries; p.qk = proj; p.qk_ld = ld; p.q0 = q0; p.k0 = k0; p.G = H; p.gates = proj;
+    p.gates_dt = NV_DT_F32; p.gates_ld = ld; p.ga0 = i0; p.gb0 = f0; p.cap = cap; p.rec = chunk_buf; p.H = H; p.dk = dk;
+    ChunkScanArgs a = {};
+    a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.rec = chunk_buf; a.S = S; a.S_stride = S_stride; a.n = n;
+    a.n_stride = n_stride; a.m = m; a.m_stride = m_stride; a.vsrc = proj; a.v_ld = ld; a.v0 = v0; a.q_scale = q_scale;
+    a.raw = raw; a.RW = dv + 2; a.H = H; a.dk = dk; a.dv = dv;
+    rc = launch_chunks_of<true>(p, a, T, s);
+  } else {
   ColArgs a = {};
   a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.n = n; a.n_stride = n_stride;
   a.m = m; a.m_stride = m_stride; a.qk = proj; a.qk_ld = ld; a.q0 = q0; a.k0 = k0; a.G = H; a.vsrc = proj; a.v_ld = ld;
   a.v0 = v0; a.gates = proj; a.gates_dt = NV_DT_F32; a.gates_ld = ld; a.ga0 = i0; a.gb0 = f0; a.cap = cap;
   a.q_scale = q_scale; a.raw = raw; a.RW = dv + 2; a.H = H; a.dk = dk; a.dv = dv;
-  int rc = launch_col_scan<0>(a, num_entries, T, gate_buf, s);
+  rc = launch_col_scan<0>(a, num_entries, T, gate_buf, s);
+  }
   if (rc) return rc;
   const long long items = (long long)T * H;
-  head_finish_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(raw, dv + 2, 1, den_eps, proj, NV_DT_F32, ld, g0, 0,
-                                                                 norm_w, norm_per_head, eps, out, out_dt, T, H, dv);
+  const unsigned max_blocks = (unsigned)(((long long)num_entries * H + 255) / 256);
+  head_finish_kernel<<<(unsigned)((items + 7) / 8) + max_blocks, 256, 0, s>>>(
+      raw, dv + 2, 1, den_eps, proj, NV_DT_F32, ld, g0, 0, norm_w, norm_per_head, eps, out, out_dt, T, H, dv,
+      MaxState{m, m_stride, cu_rows, entry_slot, num_entries});
   NV_RETURN_LAST();
 }
 
-// The gated delta rule through col_scan_kernel; raw: [T, H, dv] and gate_buf: [T, H, 2] float32 scratch.
+// Both delta rules in chunks; `dec` null: one decay per head, its pre-activation at column a0 of `proj`.
+static int delta_chunks(const float* qkv, int C, int q0, int k0, int v0, int G, const void* proj, int proj_dt, long long ld,
+                        int b0, int a0, const float* dec, long long dec_ld, int dec0, const float* A_log,
+                        const float* dt_bias, const int* cu_rows, const int* entry_slot, float* S, long long S_stride,
+                        int H, int dk, int dv, float* raw, float* chunk_buf, int num_entries, int T, cudaStream_t s) {
+  ChunkArgs p = {};
+  p.cu_rows = cu_rows; p.S_entries = num_entries; p.qk = qkv; p.qk_ld = C; p.q0 = q0; p.k0 = k0; p.G = G; p.gates = proj;
+  p.gates_dt = proj_dt; p.gates_ld = ld; p.ga0 = b0; p.gb0 = a0; p.dec = dec; p.dec_ld = dec_ld; p.dec0 = dec0;
+  p.A_log = A_log; p.dt_bias = dt_bias; p.rec = chunk_buf; p.H = H; p.dk = dk;
+  ChunkScanArgs a = {};
+  a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.rec = chunk_buf; a.S = S; a.S_stride = S_stride; a.vsrc = qkv;
+  a.v_ld = C; a.v0 = v0; a.q_scale = 1.f; a.raw = raw; a.RW = dv; a.H = H; a.dk = dk; a.dv = dv;
+  return launch_chunks_of<false>(p, a, T, s);
+}
+
+// The gated delta rule through col_scan_kernel, or with `chunk_buf` in chunks; raw: [T, H, dv] and gate_buf: [T, H, 2] float32
+// scratch.
 NV_API int nv_gated_delta_col_scan(const float* qkv, int C, int q0, int k0, int v0, int G, const void* proj,
                                    int proj_dt, long long ld, int g0, int b0, int a0, const float* A_log,
                                    const float* dt_bias, const int* cu_rows, const int* entry_slot, float* S,
                                    long long S_stride, int H, int dk, int dv, float eps, const float* norm_w,
-                                   float* raw, float* gate_buf, void* out, int out_dt, int num_entries, int T,
-                                   cudaStream_t s) {
+                                   float* raw, float* gate_buf, float* chunk_buf, void* out, int out_dt,
+                                   int num_entries, int T, cudaStream_t s) {
   if (!dt_ok(out_dt) || proj_dt != NV_DT_F32) return NV_ERR_BAD_DTYPE;
   if (!nv_col_scan_usable(dk, dv) || H <= 0 || G <= 0 || H % G) return NV_ERR_UNSUPPORTED;
   if (num_entries == 0 || T == 0) return NV_OK;
+  int rc;
+  if (chunk_buf) {
+    rc = delta_chunks(qkv, C, q0, k0, v0, G, proj, proj_dt, ld, b0, a0, nullptr, 0, 0, A_log, dt_bias, cu_rows, entry_slot,
+                      S, S_stride, H, dk, dv, raw, chunk_buf, num_entries, T, s);
+  } else {
   ColArgs a = {};
   a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.qk = qkv; a.qk_ld = C; a.q0 = q0;
   a.k0 = k0; a.G = G; a.vsrc = qkv; a.v_ld = C; a.v0 = v0; a.gates = proj; a.gates_dt = proj_dt; a.gates_ld = ld;
   a.ga0 = b0; a.gb0 = a0; a.A_log = A_log; a.dt_bias = dt_bias; a.q_scale = 1.f; a.raw = raw; a.RW = dv; a.H = H;
   a.dk = dk; a.dv = dv;
-  int rc = launch_col_scan<1>(a, num_entries, T, gate_buf, s);
+  rc = launch_col_scan<1>(a, num_entries, T, gate_buf, s);
+  }
   if (rc) return rc;
   const long long items = (long long)T * H;
   head_finish_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(raw, dv, 0, 0.f, proj, proj_dt, ld, g0, 1, norm_w, 0,
-                                                                 eps, out, out_dt, T, H, dv);
+                                                                 eps, out, out_dt, T, H, dv, MaxState{});
   NV_RETURN_LAST();
 }
 
 // The delta rule with a decay per head and key channel through col_scan_kernel.  `dec` [T, dec_ld] float32 holds the
 // decays' pre-activations at column dec0 (head h's at dec0 + h dk); `gsrc` the output gate's at g0, gate_mode 1: a
-// sigmoid, 0: silu.  Scratch, all float32: raw [T, H, dv], gate_buf [T, H, 2], decays [T, H dk].
+// sigmoid, 0: silu.  Scratch, all float32: raw [T, H, dv] and either gate_buf [T, H, 2] and decays [T, H dk], or chunk_buf.
 NV_API int nv_channel_delta_scan(const float* qkv, int C, int q0, int k0, int v0, int G, const void* proj, int proj_dt,
                                  long long ld, int b0, const float* dec, long long dec_ld, int dec0, const void* gsrc,
                                  int gsrc_dt, long long gsrc_ld, int g0, int gate_mode, const float* A_log,
                                  const float* dt_bias, const int* cu_rows, const int* entry_slot, float* S,
                                  long long S_stride, int H, int dk, int dv, float eps, const float* norm_w, float* raw,
-                                 float* gate_buf, float* decays, void* out, int out_dt, int num_entries, int T,
-                                 cudaStream_t s) {
+                                 float* gate_buf, float* decays, float* chunk_buf, void* out, int out_dt,
+                                 int num_entries, int T, cudaStream_t s) {
   if (!dt_ok(out_dt) || !dt_ok(proj_dt) || !dt_ok(gsrc_dt)) return NV_ERR_BAD_DTYPE;
   if (!nv_channel_scan_usable(dk, dv) || H <= 0 || G <= 0 || H % G) return NV_ERR_UNSUPPORTED;
-  if (!dec || !raw || !gate_buf || !decays || gate_mode < 0 || gate_mode > 1) return NV_ERR_BAD_SIZE;
+  if (!dec || !raw || (!chunk_buf && (!gate_buf || !decays)) || gate_mode < 0 || gate_mode > 1) return NV_ERR_BAD_SIZE;
   if (num_entries == 0 || T == 0) return NV_OK;
+  int rc;
+  if (chunk_buf) {
+    rc = delta_chunks(qkv, C, q0, k0, v0, G, proj, proj_dt, ld, b0, 0, dec, dec_ld, dec0, A_log, dt_bias, cu_rows, entry_slot,
+                      S, S_stride, H, dk, dv, raw, chunk_buf, num_entries, T, s);
+  } else {
   const long long n = (long long)T * H * dk;
   channel_gates_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dec, dec_ld, dec0, proj, proj_dt, ld, b0, A_log,
                                                                   dt_bias, H, dk, decays, gate_buf, n);
@@ -1560,11 +1627,12 @@ NV_API int nv_channel_delta_scan(const float* qkv, int C, int q0, int k0, int v0
   a.RW = dv; a.H = H; a.dk = dk; a.dv = dv; a.dec = decays; a.dec_ld = (long long)H * dk;
   a.vec16 = (((uintptr_t)qkv & 15) == 0 && C % 4 == 0 && q0 % 4 == 0 && k0 % 4 == 0 && dk % 4 == 0 &&
              ((uintptr_t)decays & 15) == 0) ? 1 : 0;
-  int rc = launch_col_scan_p<2, true>(a, num_entries, s);
+  rc = launch_col_scan_p<2, true>(a, num_entries, s);
+  }
   if (rc) return rc;
   const long long items = (long long)T * H;
   head_finish_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(raw, dv, 0, 0.f, gsrc, gsrc_dt, gsrc_ld, g0,
                                                                  gate_mode == 1 ? 0 : 1, norm_w, 0, eps, out, out_dt, T,
-                                                                 H, dv);
+                                                                 H, dv, MaxState{});
   NV_RETURN_LAST();
 }

@@ -1,0 +1,159 @@
+"""The matrix memories in chunks of eight rows against float64 token by token: sequences that end inside a chunk, single
+rows beside long ones, head sizes below and at the padded ones, decays from none to nearly everything, and a state
+that is carried from one step to the next."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def batch_of(lens):
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV).flip(0).contiguous()
+    return types.SimpleNamespace(cu_rows=cu, entry_slot=slots, S=len(lens))
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def rms(x):
+    return x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6)
+
+
+def delta_plain(q, k, v, beta, g, S):
+    """float64; q, k [T, H, dk], v [T, H, dv], beta [T, H], g [T, H, dk]; S [H, dk, dv] changed in place."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S *= g[t][..., None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S += k[t][..., None] * u[:, None, :]
+        out[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return out
+
+
+def lstm_plain(q, k, v, gi, gf, S, n, m):
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        new = torch.maximum(gf[t] + m, gi[t])
+        keep, take = torch.exp(gf[t] + m - new), torch.exp(gi[t] - new)
+        S *= keep[:, None, None]
+        S += (take[:, None] * k[t])[..., None] * v[t][:, None, :]
+        n *= keep[:, None]
+        n += take[:, None] * k[t]
+        m.copy_(new)
+        den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+        out[t] = torch.einsum("hkv,hk->hv", S, q[t]) / den[:, None]
+    return out
+
+
+LENS = [[33], [40, 1, 7, 8, 9], [1, 1, 64, 1], [130, 3, 77] * 16]
+SIZES = [(4, 2, 128, 128), (3, 3, 16, 40), (2, 1, 64, 33), (4, 4, 72, 128)]        # heads, q/k heads, dk, dv
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("H,G,dk,dv", SIZES)
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("decay", [-6.0, 0.0, 4.0])
+def test_delta_rule_in_chunks(lens, H, G, dk, dv, channel, decay):
+    from nano_vllm_cpp_b200.csrc import ops
+    g = torch.Generator().manual_seed(len(lens) + dk)
+    b, T = batch_of(lens), sum(lens)
+    C = 2 * G * dk + H * dv
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)                                        # noqa: E731
+    q, k = unit(torch.randn(T, G, dk, generator=g)) * dk ** -0.5, unit(torch.randn(T, G, dk, generator=g))
+    v = torch.randn(T, H, dv, generator=g)
+    qkv = torch.cat([q.flatten(1), k.flatten(1), v.flatten(1)], 1).to(DEV)
+    proj = torch.randn(T, 2 * H + H * dv, generator=g).to(DEV)
+    dec = (torch.randn(T, H * dk, generator=g) + decay).to(DEV)
+    proj[:, H:2 * H] += decay
+    A_log, dt_bias = (0.3 * torch.randn(H, generator=g)).to(DEV), (0.3 * torch.randn(H * dk if channel else H, generator=g)).to(DEV)
+    norm = torch.ones(dv, device=DEV)
+    S = (0.3 * torch.randn(len(lens), H, dk, dv, generator=g)).to(DEV)
+    S64 = S.double()
+    rate = A_log.double().exp()
+    pre = dec.double().view(T, H, dk) + dt_bias.double().view(H, dk) if channel else \
+        (proj[:, H:2 * H].double() + dt_bias.double())[..., None].expand(T, H, dk)
+    gam = torch.exp(-rate[:, None] * torch.nn.functional.softplus(pre))
+    rep = H // G
+    q64, k64 = (qkv[:, i * G * dk:(i + 1) * G * dk].double().view(T, G, dk).repeat_interleave(rep, 1) for i in (0, 1))
+    want, cu = torch.empty(T, H, dv, dtype=torch.float64, device=DEV), b.cu_rows.tolist()
+    for e, slot in enumerate(b.entry_slot.tolist()):
+        r = slice(cu[e], cu[e + 1])
+        want[r] = delta_plain(q64[r], k64[r], qkv[r, 2 * G * dk:].double().view(-1, H, dv),
+                              proj[r, :H].double().sigmoid(), gam[r], S64[slot])
+    gate = proj[:, 2 * H:].double().sigmoid() if channel else torch.nn.functional.silu(proj[:, 2 * H:].double())
+    y64 = rms(want).flatten(1) * gate
+    kw = dict(channel_decay=dec, gate_src=proj, gate="sigmoid") if channel else {}
+    pcols = {"b": 0, "a": 0 if channel else H, "g": 2 * H}
+    errs = []
+    for dtype in (torch.float32, torch.bfloat16):       # row by row, then in chunks
+        S2, out = S.clone(), torch.empty(T, H * dv, dtype=dtype, device=DEV)
+        ops.gated_delta_scan(qkv, {"q": 0, "k": G * dk, "v": 2 * G * dk}, G, proj, pcols, A_log, dt_bias, b, S2, H, dk, dv,
+                             1e-6, norm, out, **kw)
+        errs.append((rel(S2, S64), rel(out, y64)))
+    print(errs)
+    # float32 sums of some hundred terms each way; the memory forgets, so errors do not pile up
+    assert errs[1][0] < max(1.5 * errs[0][0], 5e-7)
+    assert errs[1][1] < 2.0 ** -8                       # (the rounding of the output to bfloat16)
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("H,dk,dv", [(4, 128, 128), (3, 16, 40), (2, 64, 33), (4, 72, 128)])
+def test_matrix_lstm_in_chunks(lens, H, dk, dv):
+    from nano_vllm_cpp_b200.csrc import ops
+    g = torch.Generator().manual_seed(len(lens) + dk)
+    b, T = batch_of(lens), sum(lens)
+    cols = {"q": 0, "k": H * dk, "v": 2 * H * dk, "g": 2 * H * dk + H * dv, "i": 2 * H * dk + 2 * H * dv,
+            "f": 2 * H * dk + 2 * H * dv + H}
+    proj = torch.randn(T, cols["f"] + H, generator=g).to(DEV)
+    proj[:, cols["i"]:] *= 4.0
+    norm = torch.ones(dv, device=DEV)
+    S = (0.3 * torch.randn(len(lens), H, dk, dv, generator=g)).to(DEV)
+    n = torch.randn(len(lens), H, dk, generator=g).to(DEV)
+    m = torch.randn(len(lens), H, generator=g).to(DEV)
+    S64, n64, m64 = S.double(), n.double(), m.double()
+    col = lambda name, w: proj[:, cols[name]:cols[name] + w].double()                        # noqa: E731
+    gi = 15 * torch.tanh(col("i", H) / 15)
+    gf = torch.nn.functional.logsigmoid(15 * torch.tanh(col("f", H) / 15))
+    want, cu = torch.empty(T, H, dv, dtype=torch.float64, device=DEV), b.cu_rows.tolist()
+    for e, slot in enumerate(b.entry_slot.tolist()):
+        r = slice(cu[e], cu[e + 1])
+        want[r] = lstm_plain(col("q", H * dk)[r].view(-1, H, dk) * dk ** -0.5, col("k", H * dk)[r].view(-1, H, dk),
+                             col("v", H * dv)[r].view(-1, H, dv), gi[r], gf[r], S64[slot], n64[slot], m64[slot])
+    y64 = rms(want).flatten(1) * col("g", H * dv).sigmoid()
+    errs = []
+    for dtype in (torch.float32, torch.bfloat16):
+        S2, n2, m2, out = S.clone(), n.clone(), m.clone(), torch.empty(T, H * dv, dtype=dtype, device=DEV)
+        ops.mlstm_scan(proj, cols, b, S2, n2, m2, H, dk, dv, 15.0, 1e-6, norm, out)
+        errs.append((rel(S2, S64), rel(n2, n64), rel(m2, m64), rel(out, y64)))
+    print(errs)
+    for i in range(3):
+        assert errs[1][i] < max(1.5 * errs[0][i], 5e-7)
+    assert errs[1][3] < 2.0 ** -8
+
+
+def test_matrix_lstm_of_many_single_rows():
+    """More blocks than fit the GPU at once: every block of a head starts from the maximum before the step."""
+    from nano_vllm_cpp_b200.csrc import ops
+    g = torch.Generator().manual_seed(3)
+    B, H, dk, dv = 96, 16, 128, 128
+    b = batch_of([1] * B)
+    cols = {"q": 0, "k": H * dk, "v": 2 * H * dk, "g": 2 * H * dk + H * dv, "i": 2 * H * dk + 2 * H * dv,
+            "f": 2 * H * dk + 2 * H * dv + H}
+    proj = torch.randn(B, cols["f"] + H, generator=g).to(DEV)
+    norm = torch.ones(dv, device=DEV)
+    state = [(torch.randn(B, H, dk, dv, generator=g)).to(DEV), torch.randn(B, H, dk, generator=g).to(DEV),
+             (4 * torch.randn(B, H, generator=g)).to(DEV)]
+    one = [x.clone() for x in state]
+    out = torch.empty(B, H * dv, device=DEV)
+    ops.mlstm_scan(proj, cols, b, *state, H, dk, dv, 15.0, 1e-6, norm, out)
+    for e in range(0, B, 19):                  # a step of the entry alone gives the same bits
+        slot = int(b.entry_slot[e])
+        single = batch_of([1])
+        own, y = [x[slot:slot + 1].clone() for x in one], torch.empty(1, H * dv, device=DEV)
+        ops.mlstm_scan(proj[e:e + 1].contiguous(), cols, single, *own, H, dk, dv, 15.0, 1e-6, norm, y)
+        assert all(torch.equal(x[0], z[slot]) for x, z in zip(own, state)) and torch.equal(y[0], out[e])
