@@ -69,7 +69,8 @@ struct DecArgs {
                           // fetches a page once, and a stage of its ring is half as large
   float softcap;          // > 0: a scaled score s becomes softcap * tanh(s / softcap) (lane-per-chunk kernel only)
   int has_sink;           // the softmax's denominator also holds exp(sink): a key with that score and no value
-  float sink;             // (the lane-per-chunk kernel and the merges add it; the tensor-core form does not know it)
+  float sink;
+  int min_pages;          // tensor-core form: a split takes at least so many pages (a short row then has fewer splits)
   HeadGate gate;          // multiplies a head's output where its final value is written (here or in the merge)
   int chunk;              // > 0: a row sees its own chunk of so many positions (and there is no window)
   ScoreBias bias;         // what the distance gives to a score, after the cap
@@ -388,9 +389,20 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
   const int n = a.positions[t] + 1;
   const int lo = first_visible(n - 1, a.window, a.chunk);
   const int p_lo = lo / a.page, p_hi = (n - 1) / a.page + 1;
-  const int per = (p_hi - p_lo + a.splits - 1) / a.splits;
+  const int per = max((p_hi - p_lo + a.splits - 1) / a.splits, a.min_pages);
   const int pb = p_lo + split * per;
   const int n_pages = max(0, min(p_hi, pb + per) - pb);
+  if (n_pages == 0 && a.splits > 1) {                // nothing for this split: say so and leave
+    grid_dep_wait();
+    grid_dep_launch();
+    for (int i = threadIdx.x; i < ng * a.D; i += (WARPS + 1) * 32) {
+      const size_t pi = ((size_t)r * a.Hq + kvh * G + g0 + i / a.D) * a.splits + split;
+      a.part_o[pi * a.D + i % a.D] = 0.f;
+      if (i % a.D == 0) { a.part_ml[pi * 2] = -1e30f; a.part_ml[pi * 2 + 1] = 0.f; }
+    }
+    if (a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, a.D);
+    return;
+  }
   const uint32_t box_bytes = (uint32_t)a.page * 128;           // one box: `page` keys x 64 elements
   const uint32_t half_stage = box_bytes * (D / 64);            // keys of one page; values follow
   const uint32_t stage_bytes = a.same_kv ? half_stage : 2 * half_stage;
@@ -644,6 +656,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
     }
     const int h = kvh * G + g0 + gg;
     if (a.splits == 1) {
+      if (a.has_sink) ll += exp2f(a.sink * 1.4426950408889634f - mms);
       st_dt(a.out, a.out_dt, ((size_t)t * a.Hq + h) * a.D + d, ll > 0.f ? ov / ll * head_gate_of(a.gate, t, h) : 0.f);
     } else {
       const size_t pi = ((size_t)r * a.Hq + h) * a.splits + split;
@@ -793,8 +806,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // softcap > 0: scaled scores are capped, s -> softcap * tanh(s / softcap).  chunk > 0: a row at position p sees the
   // positions from p / chunk * chunk on (and there is no window).  slopes [Hq]: head h's score with a key at distance n loses
   // slopes[h] * n; bias_table [Hq, 64 + bias_len + 64] (see ScoreBias): it gains bias_table[h][min(n, bias_len - 1)]; both after the cap.
-  // has_sink: a further key with the score sink_score and no value in every softmax; it keeps the tensor-core form
-  // out.  float_weights: the weights keep all their bits in their product with the values (the lane-per-chunk
+  // has_sink: a further key with the score sink_score and no value in every softmax.  float_weights: the weights keep all their bits in their product with the values (the lane-per-chunk
   // kernel multiplies in float32; the tensor-core form takes them as three bfloat16 terms instead of one).
   if (!dt_ok(q_dt) || !dt_ok(cache_dt) || !dt_ok(out_dt)) return NV_ERR_BAD_DTYPE;
   if (D <= 0 || D > 256 || D % 8 || Hkv <= 0 || Hq % Hkv || page % 16) return NV_ERR_UNSUPPORTED;
@@ -810,6 +822,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   a.qkv = qkv; a.kc = kc; a.vc = vc; a.block_table = block_table; a.row_entry = row_entry; a.positions = positions;
   a.rows = rows; a.out = out; a.scale = scale; a.q_dt = q_dt; a.out_dt = out_dt; a.q_stride = q_stride;
   a.max_blocks = max_blocks; a.window = window; a.Hq = Hq; a.Hkv = Hkv; a.D = D; a.page = page; a.splits = splits;
+  a.min_pages = 1;
   a.part_o = scratch;
   a.part_ml = scratch ? scratch + (size_t)R * Hq * splits * D : nullptr;
   a.err = err;
@@ -851,8 +864,13 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
       a.same_kv = 1;
     }
   }
-  if (cache_dt == NV_DT_BF16 && D >= 32 && D % 16 == 0 && page <= 256 && num_pages > 0 && tc_stages >= WARPS && !has_sink) {
+  if (cache_dt == NV_DT_BF16 && D >= 32 && D % 16 == 0 && page <= 256 && num_pages > 0 && tc_stages >= WARPS) {
     a.stages = tc_stages;
+    // Rows of different lengths: the split count fills the GPU if all rows are as long as the longest may be, so where
+    // there are blocks for several waves anyway a short row is not cut into shares that cost more to begin than to
+    // read (a share of 512 keys of 128 elements is 256 KB).  Measured: 64 rows of 67 to 2,048 tokens, 16 heads, eight layers, four steps:
+    // 10.93 -> 10.73 ms.
+    a.min_pages = (long long)R * Hkv * ((G + 15) / 16) * splits > 2 * 3 * 148 ? (512 + page - 1) / page : 1;
     // tensor-core form (a page of keys per warp); its blocks take up to 16 query heads of a kv head; with
     // float_weights the weights enter the product with the values as three bfloat16 terms
     const bool mod = a.softcap > 0.f || slopes || bias_table;
