@@ -788,7 +788,9 @@ class StaticTiles:
     T * K routed pairs: what ``moe_route_small(static=True)`` leaves out of its list."""
 
     def __init__(self, T: int, K: int, E: int, C: int, device):
-        self.tile_m = 16 if T <= 16 else (32 if T <= 32 else (64 if T <= 64 else 128))
+        # (4,523 rows of eight chunks of 2,560, width 3,584: 1,399 + 753 us in tiles of 128, 1,199 + 573 in tiles of 256; 2,048 rows of
+        # four of 1,408 108 + 59 against 114 + 50, 508 rows 53 + 25 against 53 + 29)
+        self.tile_m = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128 if T < 3072 else 256
         experts, row0, rows = [], [], []
         for c in range(C):
             for r in range(0, T, self.tile_m):
@@ -1523,13 +1525,16 @@ def grouped_token_tile(TK: int, E: int, swiglu: bool = False) -> int:
     """Token tile of the grouped tensor-core product for TK (row, expert) pairs over E experts: the most rows of
     one expert that a CTA takes at once.  The product's instruction is as wide as a tile's rows need (in steps
     of 16) and so are its token loads (in boxes of 64 rows), so a short last tile of an expert is cheap.  Tiles
-    of 256 rows are accepted but lose (one accumulator set instead of two: 23.9 against 20.5 ms for a prompt of
-    2,048 tokens).  ``swiglu`` lets the two products of an expert layer choose differently; they agree."""
+    of 256 rows leave one accumulator set instead of two but read an expert's weights from L2 half as often: they win once
+    an expert has several hundred rows (64 experts of 2,560, width 3,584, 565 rows each: 1,341 + 709 us in tiles of 128, 1,181 +
+    581 in tiles of 256; at 136 rows each of 60 experts of 1,408 124 + 72 against 138 + 71).  ``swiglu`` lets the two products of an expert layer choose differently; they agree."""
     avg = (TK + E - 1) // E
     if avg <= 12:
         return 16
     if avg <= 24:
         return 32
+    if avg >= 384:
+        return 256
     return 128 if avg >= 96 else 64
 
 
