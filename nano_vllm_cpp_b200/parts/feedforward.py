@@ -6,7 +6,7 @@ import torch
 
 from ..csrc import ops
 from .base import FeedForward, RowMix, TensorSpec
-from .linear import linear, grouped_linear, small_linear
+from .linear import linear, grouped_linear, small_linear, side_stream
 from .registry import register_part
 
 # Batches of up to this many rows run the shared expert's chunks on a second stream beside the routing.
@@ -354,7 +354,7 @@ class SparseMoeSwiGLU(FeedForward):
             self._static_kept.add(key)
         act = torch.empty((T * KT, self.inter), dtype=ctx.act_dtype, device=dev)
         y = torch.empty((T * KT, self.hidden), dtype=torch.float32, device=dev)
-        main, side = torch.cuda.current_stream(dev), _side_stream(dev)
+        main, side = torch.cuda.current_stream(dev), side_stream(dev)
         fork, join = torch.cuda.Event(), torch.cuda.Event()
         fork.record(main)
         side.wait_event(fork)
@@ -388,19 +388,6 @@ class SparseMoeSwiGLU(FeedForward):
         ops.gemm_fast_grouped(act, self.w_down, y, al, err=ctx.err, tiles_ready=True, counter=c1)
         main.wait_event(join)
         return RowMix(y, al.pair_pos[:T * KT].view(T, KT), score, None, None)
-
-
-_side = {}
-
-
-def _side_stream(dev):
-    """One second stream per device for work that runs beside a step's main stream."""
-    if ops.timing():                 # per-kernel timers are running: one stream, one kernel after the other
-        return torch.cuda.current_stream(dev)
-    key = torch.device(dev)
-    if key not in _side:
-        _side[key] = torch.cuda.Stream(device=key)
-    return _side[key]
 
 
 def _cat(ts):

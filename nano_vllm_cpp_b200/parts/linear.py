@@ -70,3 +70,16 @@ def grouped_linear(ctx, a, w, out_dtype, align, *, a_rows=None, swiglu=False, ti
     else:
         ops.gemm_plain(a, w, out, a_rows=a_rows, swiglu=swiglu, M=align.TK, tiles=align.tiles, act=act)
     return out
+
+
+_side = {}
+
+
+def side_stream(dev):
+    """One second stream per device for work that runs beside a step's main stream."""
+    if ops.timing():                 # per-kernel timers are running: one stream, one kernel after the other
+        return torch.cuda.current_stream(dev)
+    key = torch.device(dev)
+    if key not in _side:
+        _side[key] = torch.cuda.Stream(device=key)
+    return _side[key]
