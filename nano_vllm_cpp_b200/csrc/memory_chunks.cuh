@@ -20,7 +20,8 @@
 // holding row i's.  The matrix LSTM is the same without the first product and with weights exp(F_i - F_j + i_j - m_i) for
 // the quotients (F the running sum of the log forget gates, m_i the running maximum).
 // Measured (heads of 128 x 128, preparation, gates and head norm included): 1,500 rows of one sequence, 8 heads: delta rule 576 ->
-// 286 us, matrix LSTM 531 -> 277; eight sequences of 200 to 2,048 rows, 16 heads, a decay per channel: 1,870 -> 830 us.  Against float64
+// 281 us, matrix LSTM 531 -> 277; eight sequences of 200 to 2,048 rows, 16 heads, a decay per channel: 1,870 -> 734 us
+// (825 before two FMAs went into one instruction and the longest sequences first).  Against float64
 // the states are off by no more than row by row (tests/test_memory_chunks_gpu.py).
 
 constexpr int MC_R = 8;                                   // rows of a chunk
@@ -197,15 +198,40 @@ __device__ __forceinline__ float own_row_sum(const float (&x)[MC_R], int l) {
   return w + __shfl_xor_sync(0xffffffffu, w, 8);
 }
 
+// Two float32 FMAs, each rounded as one, in one instruction.
+__device__ __forceinline__ void fma2(float2& d, float2 a, float2 b, float2 c) {
+  unsigned long long r, x = *(unsigned long long*)&a, y = *(unsigned long long*)&b, z = *(unsigned long long*)&c;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  d = *(float2*)&r;
+}
+
 constexpr int MC_CT = 4, MC_LANES = 16;                   // columns of a lane, lanes of a column
 
 template <int DK, bool LSTM, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a) {
   constexpr int REC = mc_record(DK, LSTM), NP = DK / 64, CT = MC_CT;      // a lane's rows: NP pieces of four, 64 apart
   extern __shared__ __align__(16) float ring[];
-  const int e = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, l = tid % MC_LANES, row = l % MC_R, group = tid / MC_LANES;
+  const int h = blockIdx.y, tid = threadIdx.x, l = tid % MC_LANES, row = l % MC_R, group = tid / MC_LANES;
+  // Longest sequences first: a sequence is one walk however many blocks share its columns, so the last to begin should be
+  // short (eight sequences of 200 to 2,048 rows in order of their numbers left some multiprocessors three of the longest).
+  int e = blockIdx.z;
+  if (gridDim.z <= 32 * WARPS) {
+    __shared__ int chosen;
+    const int S_n = gridDim.z;
+    if (tid < S_n) {
+      const int mine = a.cu_rows[tid + 1] - a.cu_rows[tid];
+      int rank = 0;
+      for (int j = 0; j < S_n; ++j) {
+        const int other = a.cu_rows[j + 1] - a.cu_rows[j];
+        rank += other > mine || (other == mine && j < tid);
+      }
+      if (rank == e) chosen = tid;
+    }
+    __syncthreads();
+    e = chosen;
+  }
   const int dk = a.dk, dv = a.dv, ncols = LSTM ? dv + 1 : dv;
-  const int col = (blockIdx.z * 2 * WARPS + group) * CT;
+  const int col = (blockIdx.x * 2 * WARPS + group) * CT;
   const int row0 = a.cu_rows[e], rows = a.cu_rows[e + 1] - row0, chunks = (rows + MC_R - 1) / MC_R;
   const int slot = a.entry_slot[e];
   const float* rec = a.rec + ((long long)(row0 / MC_R + e) * a.H + h) * REC;
@@ -217,7 +243,7 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
   };
   for (int c = 0; c < MC_RING - 1; ++c) fetch(c);
 
-  float S[NP][4][CT];
+  float2 S[NP][2][CT];                             // rows 4 (l + 16 p) + 0, 1 and + 2, 3 of every column
   auto place = [&](int t, int r) -> float* {
     return LSTM && col + t == dv ? a.n + (size_t)slot * a.n_stride + (size_t)h * dk + r
                                  : a.S + (size_t)slot * a.S_stride + ((size_t)h * dk + r) * dv + col + t;
@@ -225,10 +251,11 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
 #pragma unroll
   for (int p = 0; p < NP; ++p)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 4 * (l + MC_LANES * p) + i;
+    for (int i = 0; i < 2; ++i) {
+      const int r = 4 * (l + MC_LANES * p) + 2 * i;
 #pragma unroll
-      for (int t = 0; t < CT; ++t) S[p][i][t] = col + t < ncols && r < dk ? *place(t, r) : 0.f;
+      for (int t = 0; t < CT; ++t)
+        S[p][i][t] = make_float2(col + t < ncols && r < dk ? *place(t, r) : 0.f, col + t < ncols && r + 1 < dk ? *place(t, r + 1) : 0.f);
     }
   float m0 = LSTM ? a.m[(size_t)slot * a.m_stride + h] : 0.f;
   const float* vp = a.vsrc + (size_t)(row0 + row) * a.v_ld + a.v0 + (size_t)h * dv + col;
@@ -258,8 +285,9 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
     float pk[CT][MC_R], pq[CT][MC_R];
 #pragma unroll
     for (int i = 0; i < MC_R; ++i) {
+      float2 sk[CT], sq[CT];
 #pragma unroll
-      for (int t = 0; t < CT; ++t) pk[t][i] = pq[t][i] = 0.f;
+      for (int t = 0; t < CT; ++t) sk[t] = sq[t] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const float4 qq = q4[i * (DK / 4) + MC_LANES * p];
@@ -267,18 +295,16 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
         if (!LSTM) kk = k4[i * (DK / 4) + MC_LANES * p];
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
-          pq[t][i] = fmaf(S[p][0][t], qq.x, pq[t][i]);
-          pq[t][i] = fmaf(S[p][1][t], qq.y, pq[t][i]);
-          pq[t][i] = fmaf(S[p][2][t], qq.z, pq[t][i]);
-          pq[t][i] = fmaf(S[p][3][t], qq.w, pq[t][i]);
+          fma2(sq[t], S[p][0][t], make_float2(qq.x, qq.y), sq[t]);
+          fma2(sq[t], S[p][1][t], make_float2(qq.z, qq.w), sq[t]);
           if (!LSTM) {
-            pk[t][i] = fmaf(S[p][0][t], kk.x, pk[t][i]);
-            pk[t][i] = fmaf(S[p][1][t], kk.y, pk[t][i]);
-            pk[t][i] = fmaf(S[p][2][t], kk.z, pk[t][i]);
-            pk[t][i] = fmaf(S[p][3][t], kk.w, pk[t][i]);
+            fma2(sk[t], S[p][0][t], make_float2(kk.x, kk.y), sk[t]);
+            fma2(sk[t], S[p][1][t], make_float2(kk.z, kk.w), sk[t]);
           }
         }
       }
+#pragma unroll
+      for (int t = 0; t < CT; ++t) { pq[t][i] = sq[t].x + sq[t].y; pk[t][i] = sk[t].x + sk[t].y; }
     }
     float qkr[MC_R], u[CT][MC_R], o[CT], scale = 1.f, keep = 1.f;
     *(float4*)qkr = *(const float4*)(tri + 64 + 8 * row);
@@ -308,7 +334,7 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
           u[t][j] = w7 * vj;
         }
       }
-      if (blockIdx.z == 0 && tid < MC_R && c * MC_R + row < rows) out[dv + 1] = m;
+      if (blockIdx.x == 0 && tid < MC_R && c * MC_R + row < rows) out[dv + 1] = m;
       m0 = __shfl_sync(0xffffffffu, m, MC_R - 1, MC_LANES);
       keep = __shfl_sync(0xffffffffu, keep, MC_R - 1, MC_LANES);
       scale = a.q_scale;
@@ -339,16 +365,17 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
       float4 dd = make_float4(keep, keep, keep, keep);
       if (!LSTM) dd = ((const float4*)(rc + 3 * MC_R * DK) + l)[MC_LANES * p];
 #pragma unroll
-      for (int t = 0; t < CT; ++t) { S[p][0][t] *= dd.x; S[p][1][t] *= dd.y; S[p][2][t] *= dd.z; S[p][3][t] *= dd.w; }
+      for (int t = 0; t < CT; ++t) {
+        S[p][0][t].x *= dd.x; S[p][0][t].y *= dd.y; S[p][1][t].x *= dd.z; S[p][1][t].y *= dd.w;
+      }
 #pragma unroll
       for (int j = 0; j < MC_R; ++j) {
         const float4 kk = t4[j * (DK / 4) + MC_LANES * p];
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
-          S[p][0][t] = fmaf(kk.x, u[t][j], S[p][0][t]);
-          S[p][1][t] = fmaf(kk.y, u[t][j], S[p][1][t]);
-          S[p][2][t] = fmaf(kk.z, u[t][j], S[p][2][t]);
-          S[p][3][t] = fmaf(kk.w, u[t][j], S[p][3][t]);
+          const float2 uu = make_float2(u[t][j], u[t][j]);
+          fma2(S[p][0][t], make_float2(kk.x, kk.y), uu, S[p][0][t]);
+          fma2(S[p][1][t], make_float2(kk.z, kk.w), uu, S[p][1][t]);
         }
       }
     }
@@ -357,11 +384,14 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
 #pragma unroll
   for (int p = 0; p < NP; ++p)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 4 * (l + MC_LANES * p) + i;
+    for (int i = 0; i < 2; ++i) {
+      const int r = 4 * (l + MC_LANES * p) + 2 * i;
 #pragma unroll
       for (int t = 0; t < CT; ++t)
-        if (col + t < ncols && r < dk) *place(t, r) = S[p][i][t];
+        if (col + t < ncols) {
+          if (r < dk) *place(t, r) = S[p][i][t].x;
+          if (r + 1 < dk) *place(t, r + 1) = S[p][i][t].y;
+        }
     }
 }
 
@@ -373,14 +403,14 @@ int launch_chunk_scan(const ChunkScanArgs& a, int S, cudaStream_t s) {
   const size_t smem = sizeof(float) * MC_RING * mc_record(DK, LSTM);
   auto* kernel = chunk_scan_kernel<DK, LSTM, WARPS>;
   if (smem > 48 * 1024) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<dim3(S, a.H, (ncols + per - 1) / per), 32 * WARPS, smem, s>>>(a);
+  kernel<<<dim3((ncols + per - 1) / per, a.H, S), 32 * WARPS, smem, s>>>(a);
   NV_RETURN_LAST();
 }
 
 template <int DK, bool LSTM>
 int launch_chunks(const ChunkArgs& p, const ChunkScanArgs& a, int T, cudaStream_t s) {
   const int S = p.S_entries;
-  if (mc_records(T, S) > 0x7fffffff || a.H > 65535) return NV_ERR_BAD_SIZE;
+  if (mc_records(T, S) > 0x7fffffff || a.H > 65535 || S > 65535) return NV_ERR_BAD_SIZE;
   chunk_prepare_kernel<DK, LSTM><<<dim3((unsigned)mc_records(T, S), a.H), DK, 0, s>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;

@@ -1281,6 +1281,8 @@ __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restric
                                                           void* __restrict__ out, int out_dt, int T, int H, int dv,
                                                           MaxState top) {
   const int lane = threadIdx.x & 31;
+  const bool four = out_dt == NV_DT_BF16 && gate_dt == NV_DT_F32 && dv % 4 == 0 && RW % 4 == 0 && gate_ld % 4 == 0 && g0 % 4 == 0 &&
+                    (((uintptr_t)raw | (uintptr_t)gate | (uintptr_t)w) & 15) == 0 && ((uintptr_t)out & 7) == 0;
   const unsigned row_blocks = (unsigned)(((long long)T * H + 7) / 8);
   if (blockIdx.x >= row_blocks) {
     const long long i = (long long)(blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
@@ -1299,6 +1301,17 @@ __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restric
   for (int i = lane; i < dv; i += 32) { const float o = x[i] * inv; ss = fmaf(o, o, ss); }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / (float)dv + eps);
+  if (four) {                          // (element by element: 65 us for 6,737 rows of 16 heads of 128)
+    for (int i = 4 * lane; i < dv; i += 128) {
+      const float4 v = *(const float4*)(x + i), g = *(const float4*)((const float*)gate + (size_t)t * gate_ld + g0 + h * dv + i);
+      const float4 wv = *(const float4*)(w + (w_per_head ? h * dv + i : i));
+      auto one = [&](float a, float b, float c) { return a * inv * r * b * (gate_act == 0 ? sigmoidf_(c) : siluf_(c)); };
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(one(v.x, wv.x, g.x), one(v.y, wv.y, g.y));
+      const __nv_bfloat162 hi = __floats2bfloat162_rn(one(v.z, wv.z, g.z), one(v.w, wv.w, g.w));
+      *(uint2*)((bf16*)out + (size_t)t * H * dv + (size_t)h * dv + i) = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+    }
+    return;
+  }
   for (int i = lane; i < dv; i += 32) {
     const float gv = ld_dt(gate, gate_dt, (size_t)t * gate_ld + g0 + h * dv + i);
     const float act = gate_act == 0 ? sigmoidf_(gv) : siluf_(gv);
