@@ -67,7 +67,7 @@ struct DecArgs {
   int q_dt, out_dt, q_stride, max_blocks, window, Hq, Hkv, D, page, splits, stages;
   int same_kv;            // the values are read where the keys are (one array is both): the tensor-core form then
                           // fetches a page once, and a stage of its ring is half as large
-  float softcap;          // > 0: a scaled score s becomes softcap * tanh(s / softcap) (lane-per-chunk kernel only)
+  float softcap;          // > 0: a scaled score s becomes softcap * tanh(s / softcap)
   int has_sink;           // the softmax's denominator also holds exp(sink): a key with that score and no value
   float sink;
   int min_pages;          // tensor-core form: a split takes at least so many pages (a short row then has fewer splits)

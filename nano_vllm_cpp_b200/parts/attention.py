@@ -302,7 +302,7 @@ class PagedAttention(Mixer):
     def _attend_general(self, q, cache, bt, batch, att, P, gate):
         """Entries of one row go to the split-key decode kernel (with weights that keep their float32 bits, or as one
         rounded term), the others to a tensor-core kernel (tcgen05, else mma.sync), where float32 weights enter the product
-        with the values as three bfloat16 terms; the decode kernel and the mma.sync kernel add the sink to the softmax's
+        with the values as three bfloat16 terms; each of them adds the sink to the softmax's
         denominator.  ``q``: rows whose first Hq * P elements are the query heads."""
         ctx, Hq, Hkv = self.ctx, self.Hq, self.Hkv
         scored = dict(softcap=self.softcap, gate=gate, chunk=self.chunk, slopes=self.slopes, bias_table=self.bias_table)
@@ -403,13 +403,15 @@ class PagedAttention(Mixer):
                                       self.window, att, self.Hq, self.Hkv, self.D, err=ctx.err, min_rows=min_rows)
         if side is not None:
             join.record(side)
-        if single:
-            ops.attention_decode(qkv, cache.k, cache.v, bt, batch.row_entry, batch.positions, self.scale, self.window,
-                                 att, self.Hq, self.Hkv, self.D,
-                                 batch.max_context if batch.decode_only else batch.max_single_context,
-                                 rows=None if batch.decode_only else batch.single_rows, err=ctx.err)
-        if side is not None:
-            main.wait_event(join)
+        try:
+            if single:
+                ops.attention_decode(qkv, cache.k, cache.v, bt, batch.row_entry, batch.positions, self.scale, self.window,
+                                     att, self.Hq, self.Hkv, self.D,
+                                     batch.max_context if batch.decode_only else batch.max_single_context,
+                                     rows=None if batch.decode_only else batch.single_rows, err=ctx.err)
+        finally:                # (a refused call, too, leaves no reader of these buffers behind the main stream's back)
+            if side is not None:
+                main.wait_event(join)
 
 
 def distance_buckets(rows: int, far: int) -> list:
