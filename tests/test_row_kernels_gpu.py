@@ -135,3 +135,39 @@ def test_decode_attention_with_a_sink_and_short_rows(lens, Hq, Hkv, D, sink, flo
         # one term: the weights are rounded to bfloat16, 2^-9 of a sum of weighted values of order one; the output too
         bound = 2.0 ** -8 * want.abs() + (2e-5 if float_weights else 4e-3)
         assert bool(((out[i].double().view(Hq, D) - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("D", [32, 64, 112, 128])
+@pytest.mark.parametrize("sink", [-200.0, 0.5, 6.0, 200.0])
+@pytest.mark.parametrize("lens,window", [([2, 63, 64, 65], 0), ([300], 0), ([129, 2], 50)])
+def test_prompt_attention_with_a_sink_and_three_terms(D, sink, lens, window):
+    """The sink beside sums whose reference lies far below, near and far above it.  Bound: the result is rounded once to
+    bfloat16 (2^-8 of it); the float32 steps before it move a weight by less than 2^-14 (scores of up to 8: 64 x 2^-24 in
+    the exponent, twice for the product's sum), so the output by 2^-13 of the largest value."""
+    o, T, Hq, Hkv, page, S = ops(), sum(lens), 4, 2, 16, len(lens)
+    q, k, v = (rnd(T, h, D, seed=7 + i).to(torch.bfloat16) for i, h in enumerate((Hq, Hkv, Hkv)))
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    n_pages = (max(lens) + page - 1) // page
+    bt = torch.arange(S * n_pages, dtype=torch.int32, device=DEV).flip(0).view(S, n_pages).contiguous()
+    kc = torch.zeros(S * n_pages, Hkv, page, D, dtype=torch.bfloat16, device=DEV)
+    vc = torch.zeros_like(kc)
+    want, scale = torch.empty(T, Hq, D, dtype=torch.float64, device=DEV), D ** -0.5
+    for e, n in enumerate(lens):
+        a = int(cu[e])
+        for j in range(n):
+            kc[int(bt[e, j // page]), :, j % page] = k[a + j]
+            vc[int(bt[e, j // page]), :, j % page] = v[a + j]
+        kk, vv = (t[a:a + n].double().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        s = torch.einsum("thd,jhd->htj", q[a:a + n].double(), kk) * scale
+        i = torch.arange(n, device=DEV)
+        seen = (i[None, :] <= i[:, None]) & ((i[:, None] - i[None, :] < window) if window else True)
+        s = torch.cat([s.masked_fill(~seen, -torch.inf), torch.full((Hq, n, 1), sink, dtype=torch.float64, device=DEV)], 2)
+        want[a:a + n] = torch.einsum("htj,jhd->thd", torch.softmax(s, 2)[:, :, :n], vv)
+    err, tiles = o.ErrorFlag(DEV), T // o.attention_prefill_tile_rows() + S
+    for kernel in ("auto", "mma"):
+        out = torch.zeros(T, Hq * D, dtype=torch.bfloat16, device=DEV)
+        o.attention_prefill(q.reshape(T, -1), kc, vc, bt, cu, torch.zeros(S, dtype=torch.int32, device=DEV), tiles, scale,
+                            window, out, Hq, Hkv, D, err=err, kernel=kernel, sink_score=sink, weight_terms=3)
+        err.check(kernel)
+        bound = 2.0 ** -8 * want.abs() + 2.0 ** -13 * float(v.abs().max())
+        assert bool(((out.view(T, Hq, D).double() - want).abs() <= bound).all()), kernel
