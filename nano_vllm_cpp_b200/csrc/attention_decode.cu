@@ -77,6 +77,7 @@ struct DecArgs {
   ScoreMap map;           // MOD kernels: how a raw score becomes a capped one in base-2 units
 };
 
+  float cap_in;           // MOD 2: scale / softcap
 // Called by every thread of a block once the block has written its split's partial results for the query heads
 // h0 .. h0 + nh - 1 of row r (batch row t): the block that arrives last for this (row, group of heads) adds the splits
 // up, in split order and with the arithmetic of attention_decode_merge_kernel, and writes the result; the others
@@ -363,8 +364,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 constexpr int TC_ROWS = 16;      // query heads per block (rows of the MMA)
 
 // D: head dimension rounded up to a multiple of 64 (compile time: it sizes the fragments); a.D: the head's own elements.
-// MOD: scores pass a cap and a bias by distance; they are then in base-2 units (and a.scale is 1).
-template <int D, int TERMS, bool MOD>
+// MOD 1: scores pass a cap and a bias by distance; they are then in base-2 units (and a.scale is 1).  MOD 2: the same with a
+// cap whose tangent is tanhf's (capped_log2 is off by some 2^-22 of the cap, however small the score).
+template <int D, int TERMS, int MOD>
 __global__ void __launch_bounds__((WARPS + 1) * 32, D <= 128 ? 3 : 1)
 attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                            DecArgs a) {
@@ -524,7 +526,10 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int na = n - 1 - (j0 + 2 * tq + c), nb = na - 8;         // distances (negative ones are masked below)
-            if (a.map.cap1 > 0.f) {
+            if (MOD == 2) {
+              s0[c] = a.map.cap1 * tanhf(s0[c] * a.cap_in); s0[2 + c] = a.map.cap1 * tanhf(s0[2 + c] * a.cap_in);
+              s1[c] = a.map.cap1 * tanhf(s1[c] * a.cap_in); s1[2 + c] = a.map.cap1 * tanhf(s1[2 + c] * a.cap_in);
+            } else if (a.map.cap1 > 0.f) {
               s0[c] = capped_log2(a.map, s0[c]); s0[2 + c] = capped_log2(a.map, s0[2 + c]);
               s1[c] = capped_log2(a.map, s1[c]); s1[2 + c] = capped_log2(a.map, s1[2 + c]);
             } else {
@@ -711,7 +716,7 @@ int launch_decode(const DecArgs& a, int R, int G, size_t smem, cudaStream_t s) {
   return G == 1 ? launch_decode_g<TC, CPL, 1>(a, R, G, smem, s) : launch_decode_g<TC, CPL, 4>(a, R, G, smem, s);
 }
 
-template <int D, int TERMS, bool MOD>
+template <int D, int TERMS, int MOD>
 int launch_decode_tc(DecArgs a, int R, const void* kc, const void* vc, int num_pages, float scale, cudaStream_t s) {
   const int G = a.Hq / a.Hkv;
   CUtensorMap tm_k, tm_v;
@@ -740,7 +745,7 @@ int launch_decode_tc(DecArgs a, int R, const void* kc, const void* vc, int num_p
   NV_RETURN_LAST();
 }
 
-template <int TERMS, bool MOD>
+template <int TERMS, int MOD>
 int launch_decode_tc_d(const DecArgs& a, int DT, int R, const void* kc, const void* vc, int num_pages, float scale, cudaStream_t s) {
   return DT == 64 ? launch_decode_tc<64, TERMS, MOD>(a, R, kc, vc, num_pages, scale, s)
        : DT == 128 ? launch_decode_tc<128, TERMS, MOD>(a, R, kc, vc, num_pages, scale, s)
@@ -806,8 +811,9 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // softcap > 0: scaled scores are capped, s -> softcap * tanh(s / softcap).  chunk > 0: a row at position p sees the
   // positions from p / chunk * chunk on (and there is no window).  slopes [Hq]: head h's score with a key at distance n loses
   // slopes[h] * n; bias_table [Hq, 64 + bias_len + 64] (see ScoreBias): it gains bias_table[h][min(n, bias_len - 1)]; both after the cap.
-  // has_sink: a further key with the score sink_score and no value in every softmax.  float_weights: the weights keep all their bits in their product with the values (the lane-per-chunk
-  // kernel multiplies in float32; the tensor-core form takes them as three bfloat16 terms instead of one).
+  // has_sink: a further key with the score sink_score and no value in every softmax.
+  // float_weights: the weights keep all their bits in their product with the values (the lane-per-chunk kernel multiplies
+  // in float32; the tensor-core form takes them as three bfloat16 terms instead of one).  With a sink they always do.
   if (!dt_ok(q_dt) || !dt_ok(cache_dt) || !dt_ok(out_dt)) return NV_ERR_BAD_DTYPE;
   if (D <= 0 || D > 256 || D % 8 || Hkv <= 0 || Hq % Hkv || page % 16) return NV_ERR_UNSUPPORTED;
   const int esize = cache_dt == NV_DT_BF16 ? 2 : 4;
@@ -837,6 +843,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // the last blocks' sums lengthen the kernel's tail by more than the second kernel's launch costs (measured per
   // decode step: batch 1 507 -> 511 tokens/s, batch 8 2,209 -> 2,212, batch 64 6,252 -> 6,192).
   a.split_count = (split_count && (long long)R * Hq <= split_count_len && R * Hq <= 256) ? split_count : nullptr;
+  a.cap_in = a.softcap > 0.f ? scale / a.softcap : 0.f;
   // ... and only while the last block's sum is short: a thread of it adds its outputs one after the other, each a chain
   // of loads from the second-level cache, so with sixteen heads of 256 elements on one kv head (4,096 outputs for 160
   // threads) that one block ran for 50 of the kernel's 64 us; the second kernel has a block per row and head.
@@ -864,7 +871,12 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
       a.same_kv = 1;
     }
   }
-  if (cache_dt == NV_DT_BF16 && D >= 32 && D % 16 == 0 && page <= 256 && num_pages > 0 && tc_stages >= WARPS) {
+  // Calls with a sink keep what the lane-per-chunk kernel gives: weights with all their bits, a cap by tanhf, float32 queries as
+  // they are (the tensor-core form rounds queries to bfloat16) and any scale (it takes the largest raw score for the
+  // largest scaled one).
+  const bool tc = cache_dt == NV_DT_BF16 && D >= 32 && D % 16 == 0 && page <= 256 && num_pages > 0 && tc_stages >= WARPS &&
+                  !(has_sink && (q_dt == NV_DT_F32 || !(scale > 0.f)));
+  if (tc) {
     a.stages = tc_stages;
     // Rows of different lengths: the split count fills the GPU if all rows are as long as the longest may be, so where
     // there are blocks for several waves anyway a short row is not cut into shares that cost more to begin than to
@@ -872,14 +884,15 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
     // 10.93 -> 10.73 ms.
     a.min_pages = (long long)R * Hkv * ((G + 15) / 16) * splits > 2 * 3 * 148 ? (512 + page - 1) / page : 1;
     // tensor-core form (a page of keys per warp); its blocks take up to 16 query heads of a kv head; with
-    // float_weights the weights enter the product with the values as three bfloat16 terms
+    // float_weights or a sink the weights enter the product with the values as three bfloat16 terms
     const bool mod = a.softcap > 0.f || slopes || bias_table;
-    if (float_weights)
-      rc = mod ? launch_decode_tc_d<3, true>(a, DT, R, kc, vc, num_pages, scale, stream)
-               : launch_decode_tc_d<3, false>(a, DT, R, kc, vc, num_pages, scale, stream);
+    if (float_weights || has_sink)
+      rc = has_sink && a.softcap > 0.f ? launch_decode_tc_d<3, 2>(a, DT, R, kc, vc, num_pages, scale, stream)
+           : mod ? launch_decode_tc_d<3, 1>(a, DT, R, kc, vc, num_pages, scale, stream)
+                 : launch_decode_tc_d<3, 0>(a, DT, R, kc, vc, num_pages, scale, stream);
     else
-      rc = mod ? launch_decode_tc_d<1, true>(a, DT, R, kc, vc, num_pages, scale, stream)
-               : launch_decode_tc_d<1, false>(a, DT, R, kc, vc, num_pages, scale, stream);
+      rc = mod ? launch_decode_tc_d<1, 1>(a, DT, R, kc, vc, num_pages, scale, stream)
+               : launch_decode_tc_d<1, 0>(a, DT, R, kc, vc, num_pages, scale, stream);
   } else if (cache_dt == NV_DT_BF16) {
     a.same_kv = 0;
     rc = D <= 64 ? launch_decode<bf16, 1>(a, R, G, smem, stream)

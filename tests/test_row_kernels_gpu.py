@@ -137,6 +137,32 @@ def test_decode_attention_with_a_sink_and_short_rows(lens, Hq, Hkv, D, sink, flo
         assert bool(((out[i].double().view(Hq, D) - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("lens,Hq,Hkv,D", [([1, 16, 17, 530], 4, 2, 64), ([700], 24, 4, 96), ([900] * 3, 8, 2, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("softcap", [0.0, 5.0])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_decode_attention_with_a_sink_keeps_weights_and_queries(lens, Hq, Hkv, D, dtype, softcap, sign):
+    """Without ``float_weights`` too: neither weights nor float32 queries are rounded to bfloat16 beside a sink.  Bound: scores of up
+    to 8 are off by 64 x 2^-24 and an exponential by 2^-21, the sums of weighted values of up to 5 by as much: 2e-5."""
+    o, B = ops(), len(lens)
+    kc, vc, bt = paged(lens, Hkv, D, 3)
+    q, scale = rnd(B, Hq * D, seed=5, dtype=dtype), sign * D ** -0.5
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    err, out = o.ErrorFlag(DEV), torch.empty(B, Hq * D, device=DEV)
+    o.attention_decode(q, kc, vc, bt, torch.arange(B, dtype=torch.int32, device=DEV), pos, scale, 0, out, Hq, Hkv, D, 2048,
+                       err=err, sink_score=0.5, softcap=softcap)
+    err.check("decode")
+    for i, n in enumerate(lens):
+        rows = bt[i].long().clamp(min=0)
+        k, v = (c[rows].transpose(1, 2).reshape(-1, Hkv, D)[:n].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        s = torch.einsum("hd,nhd->hn", q[i].double().view(Hq, D), k) * scale
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        s = torch.cat([s, torch.full((Hq, 1), 0.5, dtype=torch.float64, device=DEV)], 1)
+        want = torch.einsum("hn,nhd->hd", s.softmax(-1)[:, :n], v)
+        assert float((out[i].double().view(Hq, D) - want).abs().max()) <= 2e-5
+
+
 @pytest.mark.parametrize("D", [32, 64, 112, 128])
 @pytest.mark.parametrize("sink", [-200.0, 0.5, 6.0, 200.0])
 @pytest.mark.parametrize("lens,window", [([2, 63, 64, 65], 0), ([300], 0), ([129, 2], 50)])
