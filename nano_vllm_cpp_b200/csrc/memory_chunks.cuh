@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
           const float vj = __shfl_sync(0xffffffffu, v[t], j, MC_LANES);
-          o[t] = fmaf(g[j] * qkr[j], vj, o[t]);
+          if (j <= row) o[t] = fmaf(g[j] * qkr[j], vj, o[t]);        // (a later row's value may not be finite)
           u[t][j] = w7 * vj;
         }
       }
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
         for (int t = 0; t < CT; ++t) {
           u[t][j] = __shfl_sync(0xffffffffu, beta * acc[t], j, MC_LANES);       // (what rows before j take off has been taken off)
           acc[t] = fmaf(-kkr[j], u[t][j], acc[t]);
-          o[t] = fmaf(qkr[j], u[t][j], o[t]);
+          if (j <= row) o[t] = fmaf(qkr[j], u[t][j], o[t]);          // (0 times a later row's infinity would be NaN)
         }
     }
     if (l < MC_R && c * MC_R + row < rows) {

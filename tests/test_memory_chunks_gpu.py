@@ -157,3 +157,40 @@ def test_matrix_lstm_of_many_single_rows():
         own, y = [x[slot:slot + 1].clone() for x in one], torch.empty(1, H * dv, device=DEV)
         ops.mlstm_scan(proj[e:e + 1].contiguous(), cols, single, *own, H, dk, dv, 15.0, 1e-6, norm, y)
         assert all(torch.equal(x[0], z[slot]) for x, z in zip(own, state)) and torch.equal(y[0], out[e])
+
+
+def chunked(kind, T, H, dk, dv, spoil=None):
+    """One sequence through the chunked form of a memory: its output and states.  ``spoil`` = (row, part, value): that row's
+    first element of q, k or v becomes the value."""
+    from nano_vllm_cpp_b200.csrc import ops
+    g = torch.Generator().manual_seed(11)
+    b, lstm = batch_of([T]), kind == "lstm"
+    cols = {"q": 0, "k": H * dk, "v": 2 * H * dk, "g": 2 * H * dk + H * dv, "i": 2 * H * dk + 2 * H * dv,
+            "f": 2 * H * dk + 2 * H * dv + H}
+    src = torch.randn(T, cols["f"] + H, generator=g).to(DEV) * 0.3
+    if spoil:
+        src[spoil[0], cols[spoil[1]]] = spoil[2]
+    S = (0.3 * torch.randn(1, H, dk, dv, generator=g)).to(DEV)
+    out, norm = torch.empty(T, H * dv, dtype=torch.bfloat16, device=DEV), torch.ones(dv, device=DEV)
+    assert ops._chunk_buf(out, b, H, dk, lstm) is not None
+    if lstm:
+        n, m = torch.randn(1, H, dk, generator=g).to(DEV), torch.randn(1, H, generator=g).to(DEV)
+        ops.mlstm_scan(src, cols, b, S, n, m, H, dk, dv, 15.0, 1e-6, norm, out)
+        return out
+    qkv = src[:, :cols["g"]].contiguous()
+    gates, dec = src[:, cols["g"]:].contiguous(), torch.randn(T, H * dk, generator=g).to(DEV)
+    A, bias = torch.zeros(H, device=DEV), torch.zeros(H * dk if kind == "channel" else H, device=DEV)
+    kw = dict(channel_decay=dec, gate_src=gates, gate="sigmoid") if kind == "channel" else {}
+    ops.gated_delta_scan(qkv, cols, H, gates, {"g": 0, "b": H * dv, "a": 0 if kind == "channel" else H * dv + H}, A, bias, b, S, H, dk, dv, 1e-6, norm,
+                         out, **kw)
+    return out
+
+
+@pytest.mark.parametrize("kind", ["head", "channel", "lstm"])
+@pytest.mark.parametrize("row,part,value", [(15, "v", float("inf")), (12, "v", float("nan")), (15, "k", float("inf")),
+                                            (9, "q", float("nan")), (39, "v", float("-inf")), (32, "k", float("nan"))])
+def test_a_row_that_is_not_finite_leaves_the_rows_before_it(kind, row, part, value):
+    """Rows see no later row, also within a chunk, whatever the later row holds: the bits of the rows before it."""
+    want, got = chunked(kind, 45, 2, 64, 40), chunked(kind, 45, 2, 64, 40, (row, part, value))
+    assert bool(want.isfinite().all())
+    assert torch.equal(got[:row], want[:row]) and not bool(got[row].isfinite().all())
