@@ -70,14 +70,16 @@ struct DecArgs {
   float softcap;          // > 0: a scaled score s becomes softcap * tanh(s / softcap)
   int has_sink;           // the softmax's denominator also holds exp(sink): a key with that score and no value
   float sink;
-  int min_pages;          // tensor-core form: a split takes at least so many pages (a short row then has fewer splits)
+  // tensor-core form: a row that has many_shares of long_pages takes no shorter ones, another whose even share is below
+  // short_pages takes mid_pages (and either has fewer splits)
+  int long_pages, many_shares, short_pages, mid_pages;
   HeadGate gate;          // multiplies a head's output where its final value is written (here or in the merge)
   int chunk;              // > 0: a row sees its own chunk of so many positions (and there is no window)
   ScoreBias bias;         // what the distance gives to a score, after the cap
   ScoreMap map;           // MOD kernels: how a raw score becomes a capped one in base-2 units
+  float cap_in;           // MOD 2: scale / softcap
 };
 
-  float cap_in;           // MOD 2: scale / softcap
 // Called by every thread of a block once the block has written its split's partial results for the query heads
 // h0 .. h0 + nh - 1 of row r (batch row t): the block that arrives last for this (row, group of heads) adds the splits
 // up, in split order and with the arithmetic of attention_decode_merge_kernel, and writes the result; the others
@@ -391,7 +393,10 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
   const int n = a.positions[t] + 1;
   const int lo = first_visible(n - 1, a.window, a.chunk);
   const int p_lo = lo / a.page, p_hi = (n - 1) / a.page + 1;
-  const int per = max((p_hi - p_lo + a.splits - 1) / a.splits, a.min_pages);
+  const int pages = p_hi - p_lo;
+  int per = (pages + a.splits - 1) / a.splits;
+  if ((pages + a.long_pages - 1) / a.long_pages >= a.many_shares) per = max(per, a.long_pages);
+  else if (per < a.short_pages) per = a.mid_pages;
   const int pb = p_lo + split * per;
   const int n_pages = max(0, min(p_hi, pb + per) - pb);
   if (n_pages == 0 && a.splits > 1) {                // nothing for this split: say so and leave
@@ -828,7 +833,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   a.qkv = qkv; a.kc = kc; a.vc = vc; a.block_table = block_table; a.row_entry = row_entry; a.positions = positions;
   a.rows = rows; a.out = out; a.scale = scale; a.q_dt = q_dt; a.out_dt = out_dt; a.q_stride = q_stride;
   a.max_blocks = max_blocks; a.window = window; a.Hq = Hq; a.Hkv = Hkv; a.D = D; a.page = page; a.splits = splits;
-  a.min_pages = 1;
+  a.long_pages = 1; a.many_shares = 0x7fffffff; a.short_pages = a.mid_pages = 0;      // even shares
   a.part_o = scratch;
   a.part_ml = scratch ? scratch + (size_t)R * Hq * splits * D : nullptr;
   a.err = err;
@@ -838,12 +843,12 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   a.chunk = chunk;
   a.bias = ScoreBias{slopes, bias_table, bias_len - 1};
   a.map = score_map(scale, a.softcap);
+  a.cap_in = a.softcap > 0.f ? scale / a.softcap : 0.f;
   // `split_count`: zeros (R * Hq of them are enough), kept zero from launch to launch by the kernel: the splits are
   // then added up by the block that finishes last instead of by a second kernel.  For a few rows only: with many,
   // the last blocks' sums lengthen the kernel's tail by more than the second kernel's launch costs (measured per
   // decode step: batch 1 507 -> 511 tokens/s, batch 8 2,209 -> 2,212, batch 64 6,252 -> 6,192).
   a.split_count = (split_count && (long long)R * Hq <= split_count_len && R * Hq <= 256) ? split_count : nullptr;
-  a.cap_in = a.softcap > 0.f ? scale / a.softcap : 0.f;
   // ... and only while the last block's sum is short: a thread of it adds its outputs one after the other, each a chain
   // of loads from the second-level cache, so with sixteen heads of 256 elements on one kv head (4,096 outputs for 160
   // threads) that one block ran for 50 of the kernel's 64 us; the second kernel has a block per row and head.
@@ -878,11 +883,21 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
                   !(has_sink && (q_dt == NV_DT_F32 || !(scale > 0.f)));
   if (tc) {
     a.stages = tc_stages;
-    // Rows of different lengths: the split count fills the GPU if all rows are as long as the longest may be, so where
-    // there are blocks for several waves anyway a short row is not cut into shares that cost more to begin than to
-    // read (a share of 512 keys of 128 elements is 256 KB).  Measured: 64 rows of 67 to 2,048 tokens, 16 heads, eight layers, four steps:
-    // 10.93 -> 10.73 ms.
-    a.min_pages = (long long)R * Hkv * ((G + 15) / 16) * splits > 2 * 3 * 148 ? (512 + page - 1) / page : 1;
+    // The split count fills the GPU if all rows are as long as the longest may be; a share of such a row holds 256 keys and
+    // more.  Where there are blocks for two waves anyway, shares of 512 keys cost less (256 KB at 128 elements; a share has
+    // its start-up and its part in the merge), as long as a row's length gives three waves of them.  Else the waves decide:
+    // rows of the limit's length keep their even shares, shorter ones (shares below 256 keys) take 384 keys.
+    // Measured, even shares and these: 64 rows of 67 to 2,048 tokens, 16 heads, 97 and 93 us, with a limit of 8,192 169 and
+    // 106; 128 rows 239 and 171; 24 rows of 4,096 191 and 165; 16 rows of 512, limit 8,192, 70 and 49.  With 512 keys always,
+    // 16 rows of 2,048 on 16 heads 70 and 78, 20 rows of 1,536 on 8 heads, limit 2,048, 47 and 53.
+    const int slots = 3 * num_multiprocessors();
+    const long long blocks = (long long)R * Hkv * ((G + 15) / 16);
+    if (blocks * splits > 2 * slots) {
+      a.long_pages = (512 + page - 1) / page;
+      a.many_shares = (int)((3 * slots + blocks - 1) / blocks);
+      a.short_pages = (256 + page - 1) / page;
+      a.mid_pages = (384 + page - 1) / page;
+    }
     // tensor-core form (a page of keys per warp); its blocks take up to 16 query heads of a kv head; with
     // float_weights or a sink the weights enter the product with the values as three bfloat16 terms
     const bool mod = a.softcap > 0.f || slopes || bias_table;

@@ -175,6 +175,17 @@ __device__ __forceinline__ float capped_log2(const ScoreMap& m, float s) {
   return fmaf(-m.cap2, rcp_fast(ex2_fast(s * m.cap_k) + 1.f), m.cap1);
 }
 
+// Multiprocessors of the current device at the first call (the launchers' rules ask how many blocks fill the GPU).
+static inline int num_multiprocessors() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+      v = 148;
+    return v;
+  }();
+  return n;
+}
+
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialization attribute may start
 // while the kernel before it in the stream still runs; what it reads of that kernel's results, and whatever it
 // writes, must come after grid_dep_wait(), which returns once the earlier kernel has finished and its writes

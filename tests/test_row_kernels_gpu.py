@@ -197,3 +197,20 @@ def test_prompt_attention_with_a_sink_and_three_terms(D, sink, lens, window):
         err.check(kernel)
         bound = 2.0 ** -8 * want.abs() + 2.0 ** -13 * float(v.abs().max())
         assert bool(((out.view(T, Hq, D).double() - want).abs() <= bound).all()), kernel
+
+
+@pytest.mark.parametrize("R,Hq,Hkv,lens", [(16, 16, 16, [2048] * 16), (20, 8, 8, [1536] * 20), (64, 16, 16, [67, 300, 700, 2048] * 16)])
+def test_decode_splits_of_rows_as_long_as_the_limit(R, Hq, Hkv, lens):
+    """Rows that use the split count made for them keep its shares; shorter ones have longer shares and empty splits."""
+    o, D = ops(), 128
+    kc, vc, bt = paged(lens, Hkv, D, 3)
+    q, out = rnd(R, Hq * D, seed=5, dtype=torch.bfloat16), torch.empty(R, Hq * D, device=DEV)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    o.attention_decode(q, kc, vc, bt, torch.arange(R, dtype=torch.int32, device=DEV), pos, D ** -0.5, 0, out, Hq, Hkv, D, 2048,
+                       float_weights=True)
+    for i in (0, 1, R - 1):
+        rows = bt[i].long().clamp(min=0)
+        k, v = (c[rows].transpose(1, 2).reshape(-1, Hkv, D)[:lens[i]].double() for c in (kc, vc))
+        s = torch.einsum("hd,nhd->hn", q[i].double().view(Hq, D), k) * D ** -0.5
+        want = torch.einsum("hn,nhd->hd", s.softmax(-1), v)
+        assert float((out[i].double().view(Hq, D) - want).abs().max()) <= 2e-5      # (as in the test above)
