@@ -71,6 +71,20 @@ def test_turned_heads(T, H, D, dims, sign):
     assert float((out.double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("H,D,dims", [(3, 20, 6), (16, 128, 64), (40, 192, 192)])
+def test_turned_heads_have_the_bits_of_their_row(H, D, dims):
+    """A row's heads are shared out among fewer blocks the more rows there are: no bit depends on how many."""
+    o, T = ops(), 1500
+    x, pos = rnd(T, H * D, seed=1), torch.randint(0, 3000, (T,), dtype=torch.int32, device=DEV)
+    inv = (10.0 ** -(torch.arange(dims // 2) / 16.0)).float().to(DEV)
+    full = torch.empty_like(x)
+    o.rotate_heads(x, pos, inv, dims, 1.0, full, H, D)
+    for rows in (1, 2, 37, 148, 149, 700):
+        few = torch.empty(rows, H * D, device=DEV)
+        o.rotate_heads(x[T - rows:], pos[T - rows:], inv, dims, 1.0, few, H, D)
+        assert torch.equal(few, full[T - rows:])
+
+
 @pytest.mark.parametrize("T,H,N", [(1, 1, 4), (300, 16, 128), (5, 3, 6), (3, 2, 5)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gated_heads(T, H, N, dtype):
