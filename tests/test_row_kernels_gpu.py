@@ -43,6 +43,34 @@ def test_convolution_of_four_taps(lens, C, unit_heads, unit_dim, col0):
     assert float((out.double() - want).abs().max()) <= 2e-6 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("T", [1184, 1185, 1700])
+@pytest.mark.parametrize("C,unit_heads,unit_dim", [(96, 2, 16), (2560, 8, 128)])
+def test_convolution_forms_give_the_same_bits(T, C, unit_heads, unit_dim):
+    """Rows one at a time, in eights, and by the general kernel (columns off 16 bytes): a float32 run must not see which."""
+    o, S = ops(), 3
+    src, w, state = rnd(T, C + 4, seed=1), rnd(C, 4, seed=2), rnd(S, 3, C, seed=3)
+    ends = [0, 5, T - 2, T]
+    cu = torch.tensor(ends, dtype=torch.int32, device=DEV)
+    entry = torch.repeat_interleave(torch.arange(S), cu.cpu().diff()).to(torch.int32).to(DEV)
+    slot = torch.arange(S, dtype=torch.int32, device=DEV)
+    kw = dict(unit_heads=unit_heads, unit_dim=unit_dim, unit_eps=1e-6, scaled_heads=1, scale=0.25)
+
+    def run(x, col0, rows, cu, entry, slot):
+        out = torch.empty(rows, C, device=DEV)
+        o.conv_silu_norm(x, col0, C, w, 4, types.SimpleNamespace(row_entry=entry, cu_rows=cu, entry_slot=slot), state, out, **kw)
+        return out
+
+    full = run(src, 0, T, cu, entry, slot)
+    moved = torch.zeros(T, C + 4, device=DEV)
+    moved[:, 1:C + 1] = src[:, :C]
+    assert torch.equal(run(moved, 1, T, cu, entry, slot), full)
+    for e in range(S):                             # (up to T - 7 rows: the other form, on its own entry)
+        rows = ends[e + 1] - ends[e]
+        one = run(src[ends[e]:ends[e + 1]].contiguous(), 0, rows, torch.tensor([0, rows], dtype=torch.int32, device=DEV),
+                  torch.zeros(rows, dtype=torch.int32, device=DEV), slot[e:e + 1])
+        assert torch.equal(one, full[ends[e]:ends[e + 1]])
+
+
 @pytest.mark.parametrize("T,H,G,D", [(1, 4, 4, 16), (3, 4, 2, 24), (70, 16, 4, 128), (5, 16, 2, 64), (4, 6, 2, 16), (3, 4, 2, 10)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_mixed_queries(T, H, G, D, dtype):
