@@ -1013,16 +1013,22 @@ def channel_scan_usable(dk: int, dv: int) -> bool:
     return bool(lib().nv_channel_scan_usable(dk, dv))
 
 
-# Steps with at least this many rows beyond one per entry take the memories in chunks of eight rows (memory_chunks.cuh); a
-# step of a row or two per entry would work out chunks of which one row counts (8 rows: 24 us row by row).
-CHUNK_MIN_ROWS = 32
+def memory_chunks_pay(T: int, S: int, n_single: int, H: int) -> bool:
+    """Whether a step of T rows in S entries, ``n_single`` of them of one row, takes its memories in chunks of eight rows
+    (memory_chunks.cuh).  Chunks halve the time of the longest entry's chain, 0.36 us a row row by row; they cost every entry a
+    record of eight rows and a state read by fewer blocks, which counts where entries fill the GPU.  Measured, row by row
+    against chunks, 16 heads of 128 x 128: one entry of 40 rows 30 and 30 us, of 256 116 and 71; 64 rows beside a portion of
+    40 73 and 130, of 128 126 and 134, of 512 361 and 196; 8 entries of 40 58 and 58, 32 of 17 87 and 110; 2 heads, 64 rows
+    beside 128: 69 and 54.  Over 546 such points the rule is on average within a percent of the faster of both."""
+    portions = S - n_single
+    return portions > 0 and 8 * (T - n_single) > portions * (240 + S * H)
 
 
 def _chunk_buf(out, batch, H: int, dk: int, lstm: bool):
-    """Scratch for the chunked form of a memory, or None for a step that goes row by row: one of few rows, and any step
-    of a float32 run, whose sums must not depend on how a sequence is cut into steps."""
+    """Scratch for the chunked form of a memory, or None for a step that goes row by row: one that is faster so, and any
+    step of a float32 run, whose sums must not depend on how a sequence is cut into steps."""
     T = out.shape[0]
-    if out.dtype != torch.bfloat16 or T - batch.S < CHUNK_MIN_ROWS:
+    if out.dtype != torch.bfloat16 or not memory_chunks_pay(T, batch.S, getattr(batch, "n_single", 0), H):
         return None
     return torch.empty(int(lib().nv_memory_chunk_floats(T, batch.S, H, dk, 1 if lstm else 0)), dtype=torch.float32,
                        device=out.device)

@@ -1,0 +1,13 @@
+"""Rules that choose between two forms of a kernel by the sizes of a step, at sizes where both were measured."""
+import pytest
+
+from nano_vllm_cpp_b200.csrc import ops
+
+
+@pytest.mark.parametrize("rows,entries,singles,heads,chunks", [
+    (40, 1, 0, 16, True), (1500, 1, 0, 8, True), (7898, 8, 0, 16, True), (576, 65, 64, 16, True), (192, 65, 64, 2, True),
+    (600, 6, 0, 16, True), (104, 65, 64, 16, False), (104, 65, 64, 8, False), (192, 65, 64, 16, False),
+    (296, 257, 256, 16, False), (512, 257, 256, 8, False), (128, 64, 0, 16, False), (512, 256, 0, 8, False),
+    (544, 32, 0, 16, False), (1800, 200, 0, 16, False), (96, 32, 0, 8, False), (64, 64, 64, 16, False)])
+def test_memories_go_in_chunks_where_that_is_faster(rows, entries, singles, heads, chunks):
+    assert ops.memory_chunks_pay(rows, entries, singles, heads) is chunks

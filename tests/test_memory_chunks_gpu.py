@@ -10,6 +10,13 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
+@pytest.fixture(autouse=True)
+def always_chunks(monkeypatch):
+    """The chunked form also where the rule of sizes would go row by row."""
+    from nano_vllm_cpp_b200.csrc import ops
+    monkeypatch.setattr(ops, "memory_chunks_pay", lambda T, S, n_single, H: True)
+
+
 def batch_of(lens):
     cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
     slots = torch.arange(len(lens), dtype=torch.int32, device=DEV).flip(0).contiguous()
@@ -194,3 +201,71 @@ def test_a_row_that_is_not_finite_leaves_the_rows_before_it(kind, row, part, val
     want, got = chunked(kind, 45, 2, 64, 40), chunked(kind, 45, 2, 64, 40, (row, part, value))
     assert bool(want.isfinite().all())
     assert torch.equal(got[:row], want[:row]) and not bool(got[row].isfinite().all())
+
+
+def run_step(kind, src, cols, dec, lens, H, dk, dv, state, dtype):
+    """A step over sequences of ``lens`` rows from and to ``state``; (output, rows before the head norm)."""
+    from nano_vllm_cpp_b200.csrc import ops
+    b, out, raws = batch_of(lens), torch.empty(sum(lens), H * dv, dtype=dtype, device=DEV), []
+    norm, empty = torch.ones(dv, device=DEV), torch.empty
+
+    def kept(*a, **kw):
+        t = empty(*a, **kw)
+        if len(a) and a[0] in ((sum(lens), H, dv), (sum(lens), H, dv + 2)):
+            raws.append(t)
+        return t
+
+    torch.empty = kept
+    try:
+        if kind == "lstm":
+            ops.mlstm_scan(src, cols, b, *state, H, dk, dv, 15.0, 1e-6, norm, out)
+        else:
+            A, bias = torch.zeros(H, device=DEV), torch.zeros(H * dk if kind == "channel" else H, device=DEV)
+            gates = src[:, cols["g"]:].contiguous()
+            kw = dict(channel_decay=dec, gate_src=gates, gate="sigmoid") if kind == "channel" else {}
+            ops.gated_delta_scan(src[:, :cols["g"]].contiguous(), cols, H, gates,
+                                 {"g": 0, "b": H * dv, "a": 0 if kind == "channel" else H * dv + H}, A, bias, b, state[0], H, dk,
+                                 dv, 1e-6, norm, out, **kw)
+    finally:
+        torch.empty = empty
+    return out, raws[0][..., :dv]
+
+
+@pytest.mark.parametrize("kind", ["head", "channel", "lstm"])
+@pytest.mark.parametrize("dk,dv", [(64, 40), (128, 128)])
+def test_a_state_that_chunks_and_rows_hand_to_each_other(kind, dk, dv):
+    """A portion in chunks, three single rows, a portion in chunks over one state, beside the whole row by row (a float32
+    run) and float64: states (the LSTM's maximum among them) and the float32 rows before the head norm."""
+    H, T, g = 2, 91, torch.Generator().manual_seed(5)
+    cols = {"q": 0, "k": H * dk, "v": 2 * H * dk, "g": 2 * H * dk + H * dv, "i": 2 * H * dk + 2 * H * dv,
+            "f": 2 * H * dk + 2 * H * dv + H}
+    src = torch.randn(T, cols["f"] + H, generator=g).to(DEV)
+    if kind != "lstm":
+        src[:, :cols["v"]] = torch.nn.functional.normalize(src[:, :cols["v"]].reshape(T, 2 * H, dk), dim=-1).flatten(1)
+    dec = torch.randn(T, H * dk, generator=g).to(DEV)
+    first = [(0.3 * torch.randn(1, H, dk, dv, generator=g)).to(DEV)]
+    if kind == "lstm":
+        first += [torch.randn(1, H, dk, generator=g).to(DEV), torch.randn(1, H, generator=g).to(DEV)]
+    cut, rows, state = [44, 1, 1, 1, 44], [], [x.clone() for x in first]
+    at = 0
+    for n in cut:
+        # (single rows as a decode step runs them: row by row, in a bfloat16 run too)
+        rows.append(run_step(kind, src[at:at + n].contiguous(), cols, dec[at:at + n].contiguous(), [n], H, dk, dv, state,
+                             torch.bfloat16 if n > 1 else torch.float32)[1])
+        at += n
+    by_row = [x.clone() for x in first]
+    raw = run_step(kind, src, cols, dec, [T], H, dk, dv, by_row, torch.float32)[1]
+    exact = [x.double() for x in first]
+    part = lambda name, w: src[:, cols[name]:cols[name] + w].double().view(T, H, -1)        # noqa: E731
+    q, k, v, b, a = part("q", H * dk), part("k", H * dk), part("v", H * dv), part("i", H), part("f", H)
+    if kind == "lstm":
+        cap = lambda z: 15 * torch.tanh(z[..., 0] / 15)                                       # noqa: E731
+        lstm_plain(q * dk ** -0.5, k, v, cap(b), torch.nn.functional.logsigmoid(cap(a)), *(x[0] for x in exact))
+    else:
+        pre = dec.double().view(T, H, dk) if kind == "channel" else a.expand(T, H, dk)
+        want = delta_plain(q, k, v, b[..., 0].sigmoid(), torch.exp(-torch.nn.functional.softplus(pre)), exact[0][0])
+        # (the delta rules' float32 rows themselves: no bfloat16 in between)
+        assert rel(torch.cat(rows), want) < max(1.5 * rel(raw, want), 1e-6)
+    assert rel(torch.cat(rows), raw.double()) < 2e-6         # two orders of sums of some hundred float32 terms
+    for got, ref, x in zip(state, by_row, exact):
+        assert rel(got, x) < max(1.5 * rel(ref, x), 1e-6)
