@@ -402,13 +402,15 @@ __global__ void __launch_bounds__(256) rope_store_kernel(void* __restrict__ qkv,
 //
 // A chunk's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
 // output element.  The heads of a block share the keys and values they read and run their chains side by side.  Keys come
-// in slices of 32 elements through NB buffers of shared memory (cp.async, whole sectors; a thread reads its own key's slice 16 bytes at a
-// time, rows 144 bytes apart: no bank conflicts): two where many blocks hide each other's waits, four, so that a chunk's
+// in slices of 32 elements through NB buffers of shared memory (cp.async, whole sectors; a thread reads its own key's slice
+// 16 bytes at a time, rows 144 bytes apart, 80 for bfloat16 keys: no bank conflicts): two where many blocks hide each other's waits, four, so that a chunk's
 // keys are asked for at once, where a few rows leave multiprocessors idle.  Values are asked for 32 keys ahead, the first
 // before the scores.  The order of every sum is that of the element-by-element form, bit for bit.
 // Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 102 us element by element, 45 with keys in
-// slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.
-constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_ROW = ATT_SLICE + 4, ATT_AHEAD = 32;
+// slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.  bfloat16 caches (copied as they are
+// and widened from shared memory; element by element a slice was waited for 32 times over): one row at 4,096 keys 750 us
+// element by element from memory, 2,004 through slices copied so, 351 now.
+constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_AHEAD = 32;
 
 template <bool MAX, int HB>
 __device__ __forceinline__ void chunk_trees(float (&v)[HB], float (*red)[ATT_THREADS], int tid) {
@@ -430,24 +432,46 @@ __device__ __forceinline__ void chunk_trees(float (&v)[HB], float (*red)[ATT_THR
   __syncthreads();
 }
 
+// One slice of the chunk's keys as they lie in the cache: rows of ATT_SLICE elements and 16 bytes of padding.
 template <typename TC>
-__device__ __forceinline__ void stage_keys(float (*dst)[ATT_ROW], const TC* kc, const int* pslot, int cnt, int D, int d0, int tid) {
-  if constexpr (sizeof(TC) == 4) {
-    if (D % 4 == 0 && (uintptr_t)kc % 16 == 0) {
-      for (int i = tid; i < cnt * (ATT_SLICE / 4); i += ATT_THREADS) {
-        const int j = i / (ATT_SLICE / 4), d = d0 + i % (ATT_SLICE / 4) * 4;
-        if (d < D)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&dst[j][d - d0])),
-                       "l"(kc + (size_t)pslot[j] * D + d)
-                       : "memory");
-      }
-      return;
+struct KeySlice {
+  static constexpr int PER = 16 / sizeof(TC), ROW = ATT_SLICE + PER;
+  TC k[ATT_THREADS][ROW];
+};
+template <typename TC>
+__device__ __forceinline__ void stage_keys(KeySlice<TC>& dst, const TC* kc, const int* pslot, int cnt, int D, int d0, int tid) {
+  constexpr int PER = KeySlice<TC>::PER, PIECES = ATT_SLICE / PER;
+  if (D % PER == 0 && (uintptr_t)kc % 16 == 0) {
+    for (int i = tid; i < cnt * PIECES; i += ATT_THREADS) {
+      const int j = i / PIECES, d = d0 + i % PIECES * PER;
+      if (d < D)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&dst.k[j][d - d0])),
+                     "l"(kc + (size_t)pslot[j] * D + d)
+                     : "memory");
     }
+    return;
   }
   for (int i = tid; i < cnt * ATT_SLICE; i += ATT_THREADS) {
     const int j = i / ATT_SLICE, d = d0 + i % ATT_SLICE;
-    if (d < D) dst[j][d - d0] = to_f32(kc[(size_t)pslot[j] * D + d]);
+    if (d < D) dst.k[j][d - d0] = kc[(size_t)pslot[j] * D + d];
   }
+}
+// A value as it comes from memory, widened where it is used (widened at once, bfloat16 values are waited for at once).
+__device__ __forceinline__ uint32_t raw_value(const float* p) { return __float_as_uint(*p); }
+__device__ __forceinline__ uint32_t raw_value(const bf16* p) { return *(const unsigned short*)p; }
+template <typename TC>
+__device__ __forceinline__ float wide_value(uint32_t raw) { return __uint_as_float(sizeof(TC) == 4 ? raw : raw << 16); }
+
+// 16 bytes of a key as float32
+__device__ __forceinline__ void key_piece(const float* p, float (&v)[4]) {
+  const float4 f = *(const float4*)p;
+  v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+__device__ __forceinline__ void key_piece(const bf16* p, float (&v)[8]) {
+  const uint4 u = *(const uint4*)p;
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 
 template <typename TC, int HB, int NB>
@@ -456,12 +480,13 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_entry,
     const int* __restrict__ positions, float scale, int window, void* __restrict__ out, int out_dt,
     int Hq, int Hkv, int D, int page) {
-  extern __shared__ __align__(16) float att_keys[];
+  extern __shared__ __align__(16) uint8_t att_keys[];
   __shared__ __align__(16) float q[HB][256];
   __shared__ float p[HB][ATT_THREADS];
   __shared__ int pslot[ATT_THREADS];   // element offset / D of each key of the chunk
   __shared__ float red[HB][ATT_THREADS];
-  float(*keys)[ATT_THREADS][ATT_ROW] = (float(*)[ATT_THREADS][ATT_ROW])att_keys;
+  KeySlice<TC>* keys = (KeySlice<TC>*)att_keys;
+  constexpr int PER = KeySlice<TC>::PER;
   grid_dep_wait();
   grid_dep_launch();
   const int t = blockIdx.x, h0 = blockIdx.y * HB, tid = threadIdx.x;
@@ -483,9 +508,9 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
       if (sl < slices) stage_keys(keys[sl], kc, pslot, cnt, D, sl * ATT_SLICE, tid);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    float val[ATT_AHEAD];
+    uint32_t val[ATT_AHEAD];
 #pragma unroll
-    for (int i = 0; i < ATT_AHEAD; ++i) val[i] = tid < D && i < cnt ? to_f32(vc[(size_t)pslot[i] * D + tid]) : 0.f;
+    for (int i = 0; i < ATT_AHEAD; ++i) val[i] = tid < D && i < cnt ? raw_value(vc + (size_t)pslot[i] * D + tid) : 0u;
     float s[HB];
 #pragma unroll
     for (int b = 0; b < HB; ++b) s[b] = 0.f;
@@ -495,26 +520,32 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
       asm volatile("cp.async.wait_group %0;" ::"n"(NB - 1) : "memory");
       __syncthreads();
       const int dn = min(ATT_SLICE, D - sl * ATT_SLICE);
-      const float* kr = keys[sl % NB][tid];
+      const TC* kr = keys[sl % NB].k[tid];
       if (j < n) {
+        auto piece = [&](int d) {
+          float kv[PER];
+          key_piece(kr + d, kv);
+#pragma unroll
+          for (int b = 0; b < HB; ++b)
+#pragma unroll
+            for (int u = 0; u < PER; u += 4) {
+              const float4 q4 = *(const float4*)(q[b] + sl * ATT_SLICE + d + u);
+              s[b] = fmaf(q4.x, kv[u], s[b]);
+              s[b] = fmaf(q4.y, kv[u + 1], s[b]);
+              s[b] = fmaf(q4.z, kv[u + 2], s[b]);
+              s[b] = fmaf(q4.w, kv[u + 3], s[b]);
+            }
+        };
+        int d = 0;
         if (dn == ATT_SLICE) {
 #pragma unroll
-          for (int d = 0; d < ATT_SLICE; d += 4) {
-            const float4 k4 = *(const float4*)(kr + d);
-#pragma unroll
-            for (int b = 0; b < HB; ++b) {
-              const float4 q4 = *(const float4*)(q[b] + sl * ATT_SLICE + d);
-              s[b] = fmaf(q4.x, k4.x, s[b]);
-              s[b] = fmaf(q4.y, k4.y, s[b]);
-              s[b] = fmaf(q4.z, k4.z, s[b]);
-              s[b] = fmaf(q4.w, k4.w, s[b]);
-            }
-          }
+          for (; d < ATT_SLICE; d += PER) piece(d);
         } else {
-          for (int d = 0; d < dn; ++d)
-#pragma unroll
-            for (int b = 0; b < HB; ++b) s[b] = fmaf(q[b][sl * ATT_SLICE + d], kr[d], s[b]);
+          for (; d + PER <= dn; d += PER) piece(d);
         }
+        for (; d < dn; ++d)
+#pragma unroll
+          for (int b = 0; b < HB; ++b) s[b] = fmaf(q[b][sl * ATT_SLICE + d], to_f32(kr[d]), s[b]);
       }
       __syncthreads();
     }
@@ -539,7 +570,7 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     for (int half = 0; half < halves; ++half) {
       const int d = tid + half * ATT_THREADS;
       for (int i0 = 0; i0 < cnt; i0 += ATT_AHEAD) {
-        float now[ATT_AHEAD];
+        uint32_t now[ATT_AHEAD];
 #pragma unroll
         for (int i = 0; i < ATT_AHEAD; ++i) now[i] = val[i];
         const bool wrap = i0 + ATT_AHEAD >= cnt;             // the values after this half's are the next half's first
@@ -547,7 +578,7 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
         if (!wrap || half + 1 < halves) {
 #pragma unroll
           for (int i = 0; i < ATT_AHEAD; ++i)
-            val[i] = nd < D && ni + i < cnt ? to_f32(vc[(size_t)pslot[ni + i] * D + nd]) : 0.f;
+            val[i] = nd < D && ni + i < cnt ? raw_value(vc + (size_t)pslot[ni + i] * D + nd) : 0u;
         }
         const int k = min(ATT_AHEAD, cnt - i0);
 #pragma unroll
@@ -556,8 +587,8 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
 #pragma unroll
             for (int b = 0; b < HB; ++b) {
               const float w = p[b][i0 + i];
-              if (half == 0) o[0][b] = fmaf(w, now[i], o[0][b]);
-              else o[1][b] = fmaf(w, now[i], o[1][b]);
+              if (half == 0) o[0][b] = fmaf(w, wide_value<TC>(now[i]), o[0][b]);
+              else o[1][b] = fmaf(w, wide_value<TC>(now[i]), o[1][b]);
             }
           }
       }
@@ -578,8 +609,8 @@ int launch_plain_attention(const void* qkv, int dt, int q_stride, const TC* kc, 
                            int max_blocks, const int* row_entry, const int* positions, float scale, int window, void* out,
                            int out_dt, int T, int Hq, int Hkv, int D, int page, cudaStream_t s) {
   const dim3 grid(T, Hq / HB);
-  const bool few = (long long)T * (Hq / HB) <= 2 * 148;      // (four buffers leave a multiprocessor room for three blocks)
-  const size_t smem = (few ? 4 : 2) * sizeof(float) * ATT_THREADS * ATT_ROW;
+  const bool few = (long long)T * (Hq / HB) <= 2 * num_multiprocessors();      // (four buffers leave a multiprocessor room for three blocks)
+  const size_t smem = (few ? 4 : 2) * sizeof(KeySlice<TC>);
   auto* kernel = few ? paged_attention_plain_kernel<TC, HB, 4> : paged_attention_plain_kernel<TC, HB, 2>;
   if (few) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   NV_RETURN_IF(launch_dep(kernel, grid, dim3(ATT_THREADS), smem, s, qkv, dt, q_stride, kc, vc, block_table, max_blocks, row_entry,
@@ -808,7 +839,7 @@ NV_API int nv_paged_attention_plain(const void* qkv, int dt, int q_stride, const
   if (T == 0) return NV_OK;
   auto go = [&](auto* k, auto* v) {
     // (a few rows: a block per head, since there are multiprocessors for all of them; many: heads share what they read)
-    const int group = (long long)T * Hq <= 4 * 148 ? 1 : Hq / Hkv;
+    const int group = (long long)T * Hq <= 4 * num_multiprocessors() ? 1 : Hq / Hkv;
     if (group % 4 == 0)
       return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 4>(
           qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);

@@ -256,3 +256,33 @@ def test_decode_splits_of_rows_as_long_as_the_limit(R, Hq, Hkv, lens):
         s = torch.einsum("hd,nhd->hn", q[i].double().view(Hq, D), k) * D ** -0.5
         want = torch.einsum("hn,nhd->hd", s.softmax(-1), v)
         assert float((out[i].double().view(Hq, D) - want).abs().max()) <= 2e-5      # (as in the test above)
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,window", [(4, 2, 48, 0), (8, 2, 128, 0), (8, 1, 256, 90), (6, 2, 20, 0), (12, 12, 64, 33)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_plain_attention_forms_give_the_same_bits(Hq, Hkv, D, window, dtype):
+    """One, two and four heads a block, two and four buffers of keys, by how many rows a call has: the same bits, and float64's
+    sums.  Bound: chains of D and of 300 float32 FMAs, 2^-24 of their largest terms each; bfloat16 outputs are rounded once."""
+    o, n = ops(), 300
+    q = rnd(n, Hq * D, seed=1, dtype=dtype)
+    kc, vc, bt = paged([n], Hkv, D, 3)
+    kc, vc = (rnd(*kc.shape, seed=s, dtype=dtype) for s in (3, 4))
+    pos, entry = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    scale = D ** -0.5
+
+    def run(a, b):
+        out = torch.empty(b - a, Hq * D, dtype=dtype, device=DEV)
+        o.paged_attention_plain(q[a:b].contiguous(), kc, vc, bt, entry[a:b].contiguous(), pos[a:b].contiguous(), scale, window,
+                                out, Hq, Hkv, D)
+        return out
+
+    full = run(0, n)
+    for a, b in ((0, 1), (127, 129), (200, 237), (150, 300), (299, 300)):
+        assert torch.equal(run(a, b), full[a:b])
+    k, v = (c[bt[0].long()].transpose(1, 2).reshape(-1, Hkv, D)[:n].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+    s = torch.einsum("thd,jhd->htj", q.double().view(n, Hq, D), k) * scale
+    i = torch.arange(n, device=DEV)
+    seen = (i[None, :] <= i[:, None]) & ((i[:, None] - i[None, :] < window) if window else True)
+    want = torch.einsum("htj,jhd->thd", s.masked_fill(~seen, -torch.inf).softmax(-1), v).reshape(n, -1)
+    bound = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-5
+    assert bool(((full.double() - want).abs() <= bound).all())
