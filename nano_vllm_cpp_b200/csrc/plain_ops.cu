@@ -551,19 +551,20 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     }
     float top[HB], sum[HB];
 #pragma unroll
-    for (int b = 0; b < HB; ++b) top[b] = s[b] = j < n ? s[b] * scale : -1e30f;
+    for (int b = 0; b < HB; ++b) top[b] = s[b] = j < n ? __fmul_rn(s[b], scale) : -1e30f;
     chunk_trees<true, HB>(top, red, tid);
 #pragma unroll
     for (int b = 0; b < HB; ++b) {
       const float m_new = fmaxf(m[b], top[b]);
-      p[b][tid] = sum[b] = j < n ? expf(s[b] - m_new) : 0.f;
-      top[b] = expf(m[b] - m_new);                           // what the sums so far are worth now
+      // (every rounding is spelled out: the forms with one, two and four heads must not be contracted differently)
+      p[b][tid] = sum[b] = j < n ? expf(__fsub_rn(s[b], m_new)) : 0.f;
+      top[b] = expf(__fsub_rn(m[b], m_new));                 // what the sums so far are worth now
       m[b] = m_new;
     }
     chunk_trees<false, HB>(sum, red, tid);
 #pragma unroll
     for (int b = 0; b < HB; ++b) {
-      l[b] = l[b] * top[b] + sum[b];
+      l[b] = fmaf(l[b], top[b], sum[b]);
       o[0][b] *= top[b];
       o[1][b] *= top[b];
     }
