@@ -58,13 +58,17 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
 // dependent FFMAs of an output (4 cycles each; it may not be cut, see above) and the stream of W; with many the FFMA
 // rate.  So W and A pass through a ring of ST stages of KC elements a row (cp.async: the loads of ST - 1 stages are
 // under way while one is summed), blocks are narrow (N / 16 of them keep the multiprocessors busy for a handful of
-// rows), and a thread's outputs are RT rows x FT features: two LDS.128 of W and eight of A feed 64 FFMAs in the widest
+// rows), and a thread's outputs are RT rows x FT features: four LDS.128 of W and eight of A feed 128 FFMAs in the widest
 // form.  Rows are dealt to half-warps in steps of eight, so that RT is no larger than the tile's rows need (the lanes
 // of a half-warp read one row of A together, its 16 rows of W lie 16 bytes apart modulo 128: no bank conflicts).
 // Measured (float32, four layers of width 1,024 with 16 experts of 512; prompts of 75 and 333 tokens and eight decoded tokens
 // of each, 225 products): 24.2 ms with tiles of 64 x 64 x 16 loaded element by element, 6.1 so; the whole 27.5 -> 7.1 ms.
-// Tried and slower (408 rows): 64 x 64 outputs in blocks of 64 or 128 threads, 1,024 -> 1,024 in 125 and 78 against 66 us; tiles of 32
-// rows with shorter stages, 16 experts' 1,024 -> 2 x 512 in 203 against 186; and for two rows blocks of eight features, the experts' 37 against 20.
+// The widest form (64 x 64 outputs) is for many rows and features: 4,096 rows, 1,024 -> 4,096 in 931 us (1,535 in blocks of
+// 32 features, 1,357 in the tiles of 64 x 64 x 16); 64 rows, 1,024 -> 32,000 154 (227, 215); 2,048 rows, 512 -> 1,024 86
+// (127, 111).
+// Tried and slower: blocks of 64 features where they leave multiprocessors idle (408 rows, 1,024 -> 1,024: 78 against 66
+// us); tiles of 32 rows with shorter stages, 16 experts' 1,024 -> 2 x 512 in 203 against 186; for two rows blocks of eight
+// features, the experts' 37 against 20; a loop around the product for tiles longer than a stage (every call a tenth).
 template <typename T, int KC>
 __device__ __forceinline__ void stage_row(char* dst, const T* src, int k0, int K, int c, bool ok, int vec) {
   constexpr int PER = 16 / sizeof(T);
@@ -201,11 +205,18 @@ template <typename TA, typename TW>
 int launch(const GemmArgs& g, int m_tiles, cudaStream_t s) {
   if (m_tiles == 0) return NV_OK;
   if (m_tiles > 65535) return NV_ERR_BAD_SIZE;
-  // Two features a lane and shorter stages where there are tiles of 64 rows and enough of them for every
-  // multiprocessor; else blocks of 16 features (64 rows, 1,024 -> 1,024: 64 narrow blocks and not 32 wide ones).
-  const bool wide = g.M >= BM && (long long)((g.N + 31) / 32) * ((g.M + BM - 1) / BM) >= 148;
-  if (g.swiglu) return wide ? launch_form<TA, TW, true, 2, 64, 3>(g, m_tiles, s) : launch_form<TA, TW, true, 1, 128, 4>(g, m_tiles, s);
-  return wide ? launch_form<TA, TW, false, 2, 64, 3>(g, m_tiles, s) : launch_form<TA, TW, false, 1, 128, 4>(g, m_tiles, s);
+  // Wider blocks where there are enough of them for every multiprocessor (64 rows, 1,024 -> 1,024: 64 narrow blocks and not
+  // 32 wide ones), the widest where there are two for each.
+  constexpr int KC = sizeof(TA) == 2 && sizeof(TW) == 2 ? 64 : 32;
+  const int sms = num_multiprocessors();
+  const long long row_tiles = (g.M + BM - 1) / BM;
+  const bool wide = g.M > (g.tile_expert ? BM - 1 : BM / 2) && (long long)((g.N + 31) / 32) * row_tiles >= sms;
+  const bool widest = wide && (long long)((g.N + (g.swiglu ? 31 : 63)) / (g.swiglu ? 32 : 64)) * row_tiles >= 2 * sms;
+  if (g.swiglu)
+    return widest ? launch_form<TA, TW, true, 2, KC, 3>(g, m_tiles, s)
+         : wide ? launch_form<TA, TW, true, 2, 64, 3>(g, m_tiles, s) : launch_form<TA, TW, true, 1, 128, 4>(g, m_tiles, s);
+  return widest ? launch_form<TA, TW, false, 4, KC, 3>(g, m_tiles, s)
+       : wide ? launch_form<TA, TW, false, 2, 64, 3>(g, m_tiles, s) : launch_form<TA, TW, false, 1, 128, 4>(g, m_tiles, s);
 }
 
 }  // namespace

@@ -286,3 +286,21 @@ def test_plain_attention_forms_give_the_same_bits(Hq, Hkv, D, window, dtype):
     want = torch.einsum("htj,jhd->thd", s.masked_fill(~seen, -torch.inf).softmax(-1), v).reshape(n, -1)
     bound = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-5
     assert bool(((full.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(640, 2048 + 5, 68), (64, 20000, 33), (33, 20000, 36), (256, 4864, 128)])
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_gemm_plain_widest_form_gives_the_same_bits(M, N, K, ta, tw, swiglu):
+    """Blocks of 64 features (32 pairs), which many rows and features take: the bits of a call of few rows."""
+    o = ops()
+    a, w = rnd(M, K, seed=1, dtype=ta), rnd(2 * N if swiglu else N, K, seed=2, dtype=tw)
+    full = torch.empty(M, N, device=DEV)
+    o.gemm_plain(a, w, full, swiglu=swiglu)
+    z = a.double() @ w.double().T
+    want = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if swiglu else z
+    assert float((full.double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
+    for lo, rows in ((0, 1), (M - 9, 9), (max(0, M - 65), 32)):
+        few = torch.empty(rows, N, device=DEV)
+        o.gemm_plain(a[lo:lo + rows], w, few, swiglu=swiglu)
+        assert torch.equal(few, full[lo:lo + rows])
