@@ -370,6 +370,7 @@ def gemm_plain(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, tiles
         _i32(te, tr0, tr, nt)
         stride = w.stride(0)
         max_tiles = te.numel()
+        M = max(M, out.shape[0])         # (a tile has no more rows than there are outputs; the launcher sizes its stages by M)
     else:
         te = tr0 = tr = nt = None
         stride = 0

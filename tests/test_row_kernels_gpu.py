@@ -304,3 +304,16 @@ def test_gemm_plain_widest_form_gives_the_same_bits(M, N, K, ta, tw, swiglu):
         few = torch.empty(rows, N, device=DEV)
         o.gemm_plain(a[lo:lo + rows], w, few, swiglu=swiglu)
         assert torch.equal(few, full[lo:lo + rows])
+
+
+@pytest.mark.parametrize("M", [3, 12, 30])
+def test_grouped_plain_product_with_tiles_longer_than_its_row_count(M):
+    """The tile list says which rows there are; ``M`` below a tile's rows must not drop any."""
+    o, rows, N, K = ops(), 64, 40, 36
+    a, w = rnd(rows, K, seed=1), rnd(2, N, K, seed=2)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    tiles = tuple(torch.tensor(t, **i32) for t in ([1, 0], [0, 50], [50, 14], [2]))
+    out, want = torch.zeros(rows, N, device=DEV), torch.empty(rows, N, device=DEV)
+    o.gemm_plain(a, w, out, M=M, tiles=tiles)
+    o.gemm_plain(a, w, want, M=rows, tiles=tiles)
+    assert torch.equal(out, want)
