@@ -786,12 +786,13 @@ def moe_route_small(logits, K: int, renorm: bool, C: int, gate_logit, idx, score
 
 class StaticTiles:
     """The tiles of C experts E .. E + C - 1 that each take all T rows, in row order, their segments behind the
-    T * K routed pairs: what ``moe_route_small(static=True)`` leaves out of its list."""
+    T * K routed pairs: what ``moe_route_small(static=True)`` leaves out of its list.  ``hidden``, ``inter``: the experts' sizes,
+    as in ``grouped_token_tile``."""
 
-    def __init__(self, T: int, K: int, E: int, C: int, device):
-        # (4,523 rows of eight chunks of 2,560, width 3,584: 1,399 + 753 us in tiles of 128, 1,199 + 573 in tiles of 256; 2,048 rows of
-        # four of 1,408 108 + 59 against 114 + 50, 508 rows 53 + 25 against 53 + 29)
-        self.tile_m = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128 if T < 3072 else 256
+    def __init__(self, T: int, K: int, E: int, C: int, device, hidden: int = 0, inter: int = 0):
+        self.tile_m = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128
+        if T >= 3072 and tiles_of_256_pay(T * C, hidden, inter):
+            self.tile_m = 256
         experts, row0, rows = [], [], []
         for c in range(C):
             for r in range(0, T, self.tile_m):
@@ -1528,19 +1529,30 @@ def skinny_gemm(a, w, out, *, bias=None, swiglu=False, rows=None, err=None, act=
            f"skinny_gemm N={rows_w} K={K}", 0.0, float(w.element_size() * rows_w * K))
 
 
-def grouped_token_tile(TK: int, E: int, swiglu: bool = False) -> int:
+def tiles_of_256_pay(pairs: int, hidden: int, inter: int) -> bool:
+    """Whether the products of experts of ``inter`` x ``hidden`` over so many (row, expert) pairs take token tiles of 256
+    instead of 128.  Such tiles read the weights from L2 half as often but leave one accumulator set instead of two, so an
+    epilogue has no next tile beside it: K has to be long, and there have to be tiles for several rounds of all
+    multiprocessors.  Up and down product together, tiles of 256 against 128, rows an expert: experts of 2,560 x 3,584, 64 of
+    them 0.91 at 384 and 0.84 at 1,024, eight 0.96 and 0.86 (1.17 at 250); of 1,408 x 2,048, 60 of them 0.97 at 384 and 0.94 at
+    1,024, 16 1.06 at 512 and 0.96 at 1,024, eight 1.17 at 512; 16 of 512 x 1,024 1.36 at 512, 1.07 at 2,048; 128 of 768 x 2,048
+    1.02 at 448, 0.97 at 1,024; four chunks that take all of 3,100 rows, 1,408 x 2,048, 1.04, of 3,500 0.98."""
+    rounds = pairs / 256 * inter / 128 / num_sms()
+    return (hidden >= 3072 and inter >= 1024 and rounds >= 1.5) or (hidden >= 2048 and inter >= 1024 and rounds >= 4)
+
+
+def grouped_token_tile(TK: int, E: int, swiglu: bool = False, hidden: int = 0, inter: int = 0) -> int:
     """Token tile of the grouped tensor-core product for TK (row, expert) pairs over E experts: the most rows of
     one expert that a CTA takes at once.  The product's instruction is as wide as a tile's rows need (in steps
-    of 16) and so are its token loads (in boxes of 64 rows), so a short last tile of an expert is cheap.  Tiles
-    of 256 rows leave one accumulator set instead of two but read an expert's weights from L2 half as often: they win once
-    an expert has several hundred rows (64 experts of 2,560, width 3,584, 565 rows each: 1,341 + 709 us in tiles of 128, 1,181 +
-    581 in tiles of 256; at 136 rows each of 60 experts of 1,408 124 + 72 against 138 + 71).  ``swiglu`` lets the two products of an expert layer choose differently; they agree."""
+    of 16) and so are its token loads (in boxes of 64 rows), so a short last tile of an expert is cheap.
+    ``hidden``, ``inter``: the experts' sizes, without which there are no tiles of 256 (see ``tiles_of_256_pay``).
+    ``swiglu`` lets the two products of an expert layer choose differently; they agree."""
     avg = (TK + E - 1) // E
     if avg <= 12:
         return 16
     if avg <= 24:
         return 32
-    if avg >= 384:
+    if avg >= 384 and tiles_of_256_pay(TK, hidden, inter):
         return 256
     return 128 if avg >= 96 else 64
 

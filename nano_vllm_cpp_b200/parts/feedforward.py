@@ -262,7 +262,9 @@ class SparseMoeSwiGLU(FeedForward):
 
     def _alignment(self, TK, n_experts, device, fast):
         if fast:    # the down product's tile is the primary list, the SwiGLU product may want a wider one
-            tile_m, tile_m2 = ops.grouped_token_tile(TK, n_experts), ops.grouped_token_tile(TK, n_experts, swiglu=True)
+            sizes = dict(hidden=self.hidden, inter=self.inter)
+            tile_m = ops.grouped_token_tile(TK, n_experts, **sizes)
+            tile_m2 = ops.grouped_token_tile(TK, n_experts, swiglu=True, **sizes)
         else:
             tile_m, tile_m2 = ops.gemm_plain_tile_m(), 0
         key = (TK, n_experts, tile_m, tile_m2)
@@ -349,7 +351,7 @@ class SparseMoeSwiGLU(FeedForward):
             loose = [k for k in self._static if k not in self._static_kept]
             if len(loose) >= MAX_ALIGNMENTS:
                 self._static.pop(loose[0])
-            st = self._static[key] = ops.StaticTiles(T, K, self.E, C, dev)
+            st = self._static[key] = ops.StaticTiles(T, K, self.E, C, dev, self.hidden, self.inter)
         if torch.cuda.is_current_stream_capturing():       # a captured step names these buffers by address
             self._static_kept.add(key)
         act = torch.empty((T * KT, self.inter), dtype=ctx.act_dtype, device=dev)

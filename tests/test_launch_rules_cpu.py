@@ -11,3 +11,14 @@ from nano_vllm_cpp_b200.csrc import ops
     (544, 32, 0, 16, False), (1800, 200, 0, 16, False), (96, 32, 0, 8, False), (64, 64, 64, 16, False)])
 def test_memories_go_in_chunks_where_that_is_faster(rows, entries, singles, heads, chunks):
     assert ops.memory_chunks_pay(rows, entries, singles, heads) is chunks
+
+
+@pytest.mark.parametrize("experts,rows,hidden,inter,tile", [
+    (64, 384, 3584, 2560, 256), (72, 565, 3584, 2560, 256), (8, 384, 3584, 2560, 256), (60, 384, 2048, 1408, 256),
+    (64, 1024, 2048, 1408, 256), (16, 1024, 2048, 1408, 256), (8, 250, 3584, 2560, 128), (16, 512, 1024, 512, 128),
+    (16, 2048, 1024, 512, 128), (4, 1024, 1024, 512, 128), (16, 512, 2048, 1408, 128), (8, 512, 2048, 1408, 128),
+    (32, 512, 2048, 768, 128), (128, 448, 2048, 768, 128), (4, 512, 2048, 4096, 128), (64, 136, 2048, 1408, 128),
+    (64, 2000, 0, 0, 128)])
+def test_token_tiles_of_256_where_they_are_faster(experts, rows, hidden, inter, tile, monkeypatch):
+    monkeypatch.setattr(ops, "_num_sms", 148)
+    assert ops.grouped_token_tile(experts * rows, experts, hidden=hidden, inter=inter) == tile

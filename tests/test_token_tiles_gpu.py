@@ -1,0 +1,73 @@
+"""Token tiles of 256 rows in the grouped tensor-core products: segments that end inside, at and just behind a tile, by
+position and by counter, and the fixed list of experts that take every row.  Against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from nano_vllm_cpp_b200.csrc import ops as o
+    return o
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV).to(torch.bfloat16)
+
+
+def held(got, want, K, what):
+    """bfloat16 rounds by 2^-9 of the value (the up product's outputs); K / 16 partial sums are off by 2^-23 of the largest."""
+    if not got.numel():
+        return
+    bound = (2.0 ** -8 if got.dtype == torch.bfloat16 else 0.0) * want.abs() + K / 8 * 2.0 ** -23 * float(want.abs().max()) + 2e-6
+    assert bool(((got.double() - want).abs() <= bound).all()), what
+
+
+def pair(x, w):
+    z = x.double() @ w.double().T
+    return torch.nn.functional.silu(z[:, :z.shape[1] // 2]) * z[:, z.shape[1] // 2:]
+
+
+@pytest.mark.parametrize("sizes", [[1, 255, 257, 700, 0, 512, 385], [256], [2, 1300, 3]])
+@pytest.mark.parametrize("H,I", [(136, 72), (1032, 392)])
+@pytest.mark.parametrize("cap", [None, 0, 3])
+def test_grouped_products_in_tiles_of_256(sizes, H, I, cap):
+    """``cap``: None, tiles by position; else from a counter on at most so many CTAs (0: all)."""
+    o, E, TK = ops(), len(sizes), sum(sizes)
+    x, w1, w2 = rnd(TK, H, seed=1), rnd(E, 2 * I, H, seed=2, scale=0.05), rnd(E, H, I, seed=3, scale=0.05)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(sizes))
+    idx = idx[torch.randperm(TK, generator=torch.Generator().manual_seed(4))].to(torch.int32).to(DEV).view(TK, 1)
+    err, al = o.ErrorFlag(DEV), o.MoeAlignment(TK, E, 256, DEV)
+    o.moe_align(idx, 1, al, err)
+    act, y = torch.full((TK + 1, I), 7.0, dtype=torch.bfloat16, device=DEV), torch.full((TK + 1, H), 7.0, device=DEV)
+    count = torch.zeros(2, dtype=torch.int32, device=DEV)
+    kw = [{}, {}] if cap is None else [dict(counter=count[i:i + 1], max_ctas=cap) for i in (0, 1)]
+    o.gemm_fast_grouped(x, w1, act, al, a_rows=al.sorted_token, swiglu=True, err=err, **kw[0])
+    o.gemm_fast_grouped(act[:TK], w2, y, al, err=err, tiles_ready=True, **kw[1])
+    err.check("grouped")
+    assert count.tolist() == [0, 0] and bool((act[TK] == 7.0).all()) and bool((y[TK] == 7.0).all())
+    xs, at = x[al.sorted_token.long()], 0
+    for e, n in enumerate(sizes):
+        held(act[at:at + n], pair(xs[at:at + n], w1[e]), H, f"up {e}")
+        held(y[at:at + n], act[at:at + n].double() @ w2[e].double().T, I, f"down {e}")
+        at += n
+
+
+def test_fixed_list_in_tiles_of_256():
+    """Sizes for which the list itself chooses tiles of 256, and a row count that ends one row into a tile."""
+    o, T, K, E, C, H, I = ops(), 3073, 1, 2, 3, 3072, 1032
+    st = o.StaticTiles(T, K, E, C, DEV, H, I)
+    assert st.tile_m == 256 and st.max_tiles == 13 * C
+    x, w1, w2 = rnd(T, H, seed=1), rnd(E + C, 2 * I, H, seed=2, scale=0.02), rnd(E + C, H, I, seed=3, scale=0.02)
+    TK = T * (K + C)
+    err, al = o.ErrorFlag(DEV), o.MoeAlignment(TK, E + C, 128, DEV)
+    act, y = torch.full((TK, I), 7.0, dtype=torch.bfloat16, device=DEV), torch.full((TK, H), 7.0, device=DEV)
+    o.gemm_fast_grouped(x, w1, act, al, swiglu=True, err=err, tiles=st, tiles_ready=True, x_rows=st.x_rows, max_ctas=130)
+    o.gemm_fast_grouped(act, w2, y, al, err=err, tiles=st, tiles_ready=True, max_ctas=130)
+    err.check("fixed list")
+    assert bool((act[:T * K] == 7.0).all()) and bool((y[:T * K] == 7.0).all())           # the routed pairs' rows
+    for c in range(C):
+        r = slice(T * K + c * T, T * K + (c + 1) * T)
+        held(act[r], pair(x, w1[E + c]), H, f"up {c}")
+        held(y[r], act[r].double() @ w2[E + c].double().T, I, f"down {c}")
