@@ -1577,7 +1577,7 @@ def gemm_fast(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, err=No
     L = lib()
     n_tile = L.nv_tc_gemm_token_tile(M, (1 if swiglu else 0))
     if splits is None:
-        splits = L.nv_tc_gemm_splits(M, N, K, n_tile, num_sms())
+        splits = L.nv_tc_gemm_splits(M, N, K, n_tile, (1 if swiglu else 0), num_sms())
     scratch = None
     if splits > 1:
         scratch = torch.empty((splits, M, 2 * N if swiglu else N), dtype=torch.float32, device=a.device)

@@ -691,7 +691,7 @@ NV_API long long nv_tc_gemm_scratch_bytes(int M_tok, int N, int swiglu, int spli
 }
 
 // How many ways to split K so that a small grid still fills the GPU.  1 for large grids.
-NV_API int nv_tc_gemm_splits(int M_tok, int N, int K, int n_tile, int num_sms) {
+NV_API int nv_tc_gemm_splits(int M_tok, int N, int K, int n_tile, int swiglu, int num_sms) {
   int ctas = ((N + TILE_W - 1) / TILE_W) * ((M_tok + n_tile - 1) / n_tile);
   int k_steps = (K + BLOCK_K - 1) / BLOCK_K;
   if (ctas >= num_sms || k_steps < 8) return 1;
@@ -700,11 +700,13 @@ NV_API int nv_tc_gemm_splits(int M_tok, int N, int K, int n_tile, int num_sms) {
   int s = (M_tok <= 64 ? 2 * num_sms : num_sms) / ctas;
   if (s > k_steps / 4) s = k_steps / 4;
   if (s > 16) s = 16;
-  // With tiles of 128 tokens and more a k-step takes some 0.48 us and the partial sums are big: what the parts save of
-  // the chain of k-steps has to pay for writing and reading them and for the second kernel.  (Measured, float32 out: 1,000 rows,
-  // 2,048 x 2,048 in two parts 36 us, whole 22; 1,500 rows, 1,024 x 1,024 in three 31, whole 15; 512 rows, 1,024 x 4,096
-  // in nine 22, whole 32.)
-  if (M_tok >= 128 && s > 1 && 0.48 * k_steps * (s - 1) / s < 8.0 + 1.5e-6 * s * M_tok * N) return 1;
+  // With tiles of 128 tokens and more a k-step takes some 0.45 us and the partial sums are big: what the parts save of
+  // the chain of k-steps, and of the epilogue where it pairs two products, has to pay for writing and reading the sums and
+  // for the second kernel.  (Measured, whole and in parts: 1,000 rows, 2,048 x 2,048 22 and 36 us; 1,500 rows, 1,024 x 1,024
+  // 15 and 31; 512 rows, 1,024 x 4,096 32 and 22; 200 rows, 1,024 x 1,024 15 and 14, with SwiGLU 17 and 13.  Over 376
+  // products of 128 to 1,500 rows the rule is half a percent from the faster of both.)
+  const double saved = 0.45 * k_steps * (s - 1) / (s > 1 ? s : 1) + (swiglu ? 6.0 : 0.0);
+  if (M_tok >= 128 && s > 1 && saved < 6.0 + 2e-6 * s * M_tok * N * (swiglu ? 2 : 1)) return 1;
   return s < 1 ? 1 : s;
 }
 

@@ -22,3 +22,11 @@ def test_memories_go_in_chunks_where_that_is_faster(rows, entries, singles, head
 def test_token_tiles_of_256_where_they_are_faster(experts, rows, hidden, inter, tile, monkeypatch):
     monkeypatch.setattr(ops, "_num_sms", 148)
     assert ops.grouped_token_tile(experts * rows, experts, hidden=hidden, inter=inter) == tile
+
+
+@pytest.mark.parametrize("M,N,K,tile,swiglu,splits", [
+    (128, 1024, 1024, 128, 1, 4), (200, 1024, 1024, 128, 1, 4), (256, 1024, 1024, 128, 1, 4), (160, 2048, 1408, 128, 1, 4),
+    (200, 3072, 2048, 128, 1, 3), (128, 4096, 1024, 128, 1, 1), (128, 3584, 512, 128, 1, 1), (128, 1024, 1024, 128, 0, 1),
+    (1000, 2048, 2048, 256, 0, 1), (1500, 1024, 1024, 256, 0, 1), (512, 1024, 4096, 256, 0, 9), (128, 512, 3584, 128, 0, 14)])
+def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
+    assert ops.lib().nv_tc_gemm_splits(M, N, K, tile, swiglu, 148) == splits
