@@ -317,3 +317,52 @@ def test_grouped_plain_product_with_tiles_longer_than_its_row_count(M):
     o.gemm_plain(a, w, out, M=M, tiles=tiles)
     o.gemm_plain(a, w, want, M=rows, tiles=tiles)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("refused", [False, True])
+def test_portions_beside_single_rows(refused, monkeypatch):
+    """A step with both kinds: the portions' kernel on the second stream sees queries that the main stream has only just
+    written, and what follows on the main stream sees its result, also where the single rows' call is refused."""
+    from nano_vllm_cpp_b200.parts.attention import PagedAttention
+    o, Hq, Hkv, D, ends, rows = ops(), 4, 2, 64, [70, 33, 60], [1, 1, 40]
+    T, i32 = sum(rows), dict(dtype=torch.int32, device=DEV)
+    kc, vc, bt = paged(ends, Hkv, D, 3)
+    pos = [ends[e] - rows[e] + r for e in range(3) for r in range(rows[e])]
+    batch = types.SimpleNamespace(S=3, T=T, n_single=2, decode_only=False, max_context=70, max_single_context=70,
+                                  cu_rows=torch.tensor([0, 1, 2, T], **i32), entry_pos0=torch.tensor([69, 32, 20], **i32),
+                                  row_entry=torch.tensor([0, 1] + [2] * 40, **i32), positions=torch.tensor(pos, **i32),
+                                  single_rows=torch.tensor([0, 1], **i32))
+    final, qkv = rnd(T, (Hq + 2 * Hkv) * D, seed=9, dtype=torch.bfloat16), torch.zeros(T, (Hq + 2 * Hkv) * D, device=DEV).bfloat16()
+    att = torch.full((T, Hq * D), 7.0, dtype=torch.bfloat16, device=DEV)
+    part = types.SimpleNamespace(ctx=types.SimpleNamespace(fast_kernels=True, act_dtype=torch.bfloat16, err=o.ErrorFlag(DEV)),
+                                 scale=D ** -0.5, window=0, Hq=Hq, Hkv=Hkv, D=D)
+    prefill = o.attention_prefill
+
+    def slow(*a, **kw):
+        o.delay(20000)
+        prefill(*a, **kw)
+
+    def refuse(*a, **kw):
+        raise o.KernelError("refused")
+
+    monkeypatch.setattr(o, "attention_prefill", slow)
+    if refused:
+        monkeypatch.setattr(o, "attention_decode", refuse)
+    torch.cuda.synchronize()
+    o.delay(20000)
+    qkv.copy_(final)
+    try:
+        PagedAttention._attend(part, qkv, types.SimpleNamespace(k=kc, v=vc), bt, batch, att)
+        assert not refused
+    except o.KernelError:
+        assert refused
+    got = att.clone()                                  # (the main stream's next work)
+    part.ctx.err.check("attention")
+    for t in range(2 if refused else 0, T):
+        e, n = int(batch.row_entry[t]), pos[t] + 1
+        k, v = (c[bt[e].long().clamp(min=0)].transpose(1, 2).reshape(-1, Hkv, D)[:n].double().repeat_interleave(2, 1)
+                for c in (kc, vc))
+        s = torch.einsum("hd,nhd->hn", final[t, :Hq * D].double().view(Hq, D), k) * D ** -0.5
+        want = torch.einsum("hn,nhd->hd", s.softmax(-1), v)
+        # one bfloat16 term a weight and a bfloat16 result
+        assert bool(((got[t].double().view(Hq, D) - want).abs() <= 2.0 ** -8 * want.abs() + 8e-3).all())
