@@ -1279,6 +1279,9 @@ struct MaxState {
   const int* entry_slot;
   int S;
 };
+// FOUR: four elements a lane; MAX: with the blocks of the running maximum.  (Kernels apart: one that tested for both cost
+// a single row of 8 heads of 128 1 us of 8 more.)
+template <bool FOUR, bool MAX>
 __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restrict__ raw, int RW, int has_den,
                                                           float den_eps, const void* __restrict__ gate, int gate_dt,
                                                           long long gate_ld, int g0, int gate_act,
@@ -1286,10 +1289,8 @@ __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restric
                                                           void* __restrict__ out, int out_dt, int T, int H, int dv,
                                                           MaxState top) {
   const int lane = threadIdx.x & 31;
-  const bool four = out_dt == NV_DT_BF16 && gate_dt == NV_DT_F32 && dv % 4 == 0 && RW % 4 == 0 && gate_ld % 4 == 0 && g0 % 4 == 0 &&
-                    (((uintptr_t)raw | (uintptr_t)gate | (uintptr_t)w) & 15) == 0 && ((uintptr_t)out & 7) == 0;
   const unsigned row_blocks = (unsigned)(((long long)T * H + 7) / 8);
-  if (blockIdx.x >= row_blocks) {
+  if (MAX && blockIdx.x >= row_blocks) {
     const long long i = (long long)(blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
     if (i >= (long long)top.S * H) return;
     const int e = (int)(i / H), h = (int)(i % H), last = top.cu_rows[e + 1] - 1;
@@ -1306,14 +1307,16 @@ __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restric
   for (int i = lane; i < dv; i += 32) { const float o = x[i] * inv; ss = fmaf(o, o, ss); }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / (float)dv + eps);
-  if (four) {                          // (element by element: 65 us for 6,737 rows of 16 heads of 128)
+  if (FOUR) {                          // (element by element: 65 us for 6,737 rows of 16 heads of 128)
     for (int i = 4 * lane; i < dv; i += 128) {
-      const float4 v = *(const float4*)(x + i), g = *(const float4*)((const float*)gate + (size_t)t * gate_ld + g0 + h * dv + i);
+      const float4 v = *(const float4*)(x + i);
+      const float4 g = *(const float4*)((const float*)gate + (size_t)t * gate_ld + g0 + h * dv + i);
       const float4 wv = *(const float4*)(w + (w_per_head ? h * dv + i : i));
       auto one = [&](float a, float b, float c) { return a * inv * r * b * (gate_act == 0 ? sigmoidf_(c) : siluf_(c)); };
       const __nv_bfloat162 lo = __floats2bfloat162_rn(one(v.x, wv.x, g.x), one(v.y, wv.y, g.y));
       const __nv_bfloat162 hi = __floats2bfloat162_rn(one(v.z, wv.z, g.z), one(v.w, wv.w, g.w));
-      *(uint2*)((bf16*)out + (size_t)t * H * dv + (size_t)h * dv + i) = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+      bf16* to = (bf16*)out + (size_t)t * H * dv + (size_t)h * dv + i;
+      *(uint2*)to = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
     }
     return;
   }
@@ -1322,6 +1325,19 @@ __global__ void __launch_bounds__(256) head_finish_kernel(const float* __restric
     const float act = gate_act == 0 ? sigmoidf_(gv) : siluf_(gv);
     st_dt(out, out_dt, (size_t)t * H * dv + (size_t)h * dv + i, x[i] * inv * r * w[w_per_head ? h * dv + i : i] * act);
   }
+}
+
+int launch_head_finish(const float* raw, int RW, int has_den, float den_eps, const void* gate, int gate_dt, long long gate_ld,
+                       int g0, int gate_act, const float* w, int w_per_head, float eps, void* out, int out_dt, int T, int H,
+                       int dv, const MaxState& top, cudaStream_t s) {
+  const unsigned rows = (unsigned)(((long long)T * H + 7) / 8), max_blocks = (unsigned)(((long long)top.S * H + 255) / 256);
+  // (the matrix LSTM's rows are dv + 2 long: where dv is whole quads they are not, and go element by element)
+  const bool four = !top.m && out_dt == NV_DT_BF16 && gate_dt == NV_DT_F32 && dv % 4 == 0 && RW % 4 == 0 && gate_ld % 4 == 0 &&
+                    g0 % 4 == 0 && (((uintptr_t)raw | (uintptr_t)gate | (uintptr_t)w) & 15) == 0 && ((uintptr_t)out & 7) == 0;
+  auto* kernel = top.m ? head_finish_kernel<false, true> : four ? head_finish_kernel<true, false> : head_finish_kernel<false, false>;
+  kernel<<<rows + max_blocks, 256, 0, s>>>(raw, RW, has_den, den_eps, gate, gate_dt, gate_ld, g0, gate_act, w, w_per_head, eps, out,
+                                           out_dt, T, H, dv, top);
+  NV_RETURN_LAST();
 }
 
 // Before the scan with channel decays: decays[t, h dk + r] = exp(-exp(A_log[h]) softplus(pre[t, dec0 + h dk + r] +
@@ -1706,12 +1722,8 @@ NV_API int nv_mlstm_col_scan(const float* proj, long long ld, int q0, int k0, in
   rc = launch_col_scan<0>(a, num_entries, T, gate_buf, s);
   }
   if (rc) return rc;
-  const long long items = (long long)T * H;
-  const unsigned max_blocks = (unsigned)(((long long)num_entries * H + 255) / 256);
-  head_finish_kernel<<<(unsigned)((items + 7) / 8) + max_blocks, 256, 0, s>>>(
-      raw, dv + 2, 1, den_eps, proj, NV_DT_F32, ld, g0, 0, norm_w, norm_per_head, eps, out, out_dt, T, H, dv,
-      MaxState{m, m_stride, cu_rows, entry_slot, num_entries});
-  NV_RETURN_LAST();
+  return launch_head_finish(raw, dv + 2, 1, den_eps, proj, NV_DT_F32, ld, g0, 0, norm_w, norm_per_head, eps, out, out_dt, T, H,
+                            dv, MaxState{m, m_stride, cu_rows, entry_slot, num_entries}, s);
 }
 
 // Both delta rules in chunks; `dec` null: one decay per head, its pre-activation at column a0 of `proj`.
@@ -1753,10 +1765,7 @@ NV_API int nv_gated_delta_col_scan(const float* qkv, int C, int q0, int k0, int 
   rc = launch_col_scan<1>(a, num_entries, T, gate_buf, s);
   }
   if (rc) return rc;
-  const long long items = (long long)T * H;
-  head_finish_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(raw, dv, 0, 0.f, proj, proj_dt, ld, g0, 1, norm_w, 0,
-                                                                 eps, out, out_dt, T, H, dv, MaxState{});
-  NV_RETURN_LAST();
+  return launch_head_finish(raw, dv, 0, 0.f, proj, proj_dt, ld, g0, 1, norm_w, 0, eps, out, out_dt, T, H, dv, MaxState{}, s);
 }
 
 // The delta rule with a decay per head and key channel through col_scan_kernel.  `dec` [T, dec_ld] float32 holds the
@@ -1793,9 +1802,6 @@ NV_API int nv_channel_delta_scan(const float* qkv, int C, int q0, int k0, int v0
   rc = launch_col_scan_p<2, true>(a, num_entries, s);
   }
   if (rc) return rc;
-  const long long items = (long long)T * H;
-  head_finish_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(raw, dv, 0, 0.f, gsrc, gsrc_dt, gsrc_ld, g0,
-                                                                 gate_mode == 1 ? 0 : 1, norm_w, 0, eps, out, out_dt, T,
-                                                                 H, dv, MaxState{});
-  NV_RETURN_LAST();
+  return launch_head_finish(raw, dv, 0, 0.f, gsrc, gsrc_dt, gsrc_ld, g0, gate_mode == 1 ? 0 : 1, norm_w, 0, eps, out, out_dt, T,
+                            H, dv, MaxState{}, s);
 }
