@@ -488,6 +488,15 @@ def attention_prefill_tile_rows() -> int:
     return int(lib().nv_attention_prefill_tile_rows())
 
 
+def short_contexts_on_mma(entries: int, Hq: int, D: int, context: int) -> bool:
+    """Whether prompt attention with three terms a weight over so many entries of at most ``context`` keys is faster on the
+    mma.sync kernel: its blocks are cheaper to begin, which counts where there are more of them than multiprocessors and
+    each has a block of keys or two.  Measured, tcgen05 and mma.sync: 8 heads of 128 on 2, 64 fresh prompts of 16 tokens
+    35 and 30 us, of 64 45 and 42, of 128 65 and 73, eight of 16 7 and 11; 24 heads of 96 on 4, 64 of 16 98 and 73, 64 of 2
+    behind 200 170 and 168; 16 heads of 64 on 4, 64 of 2 34 and 31, of 32 39 and 41."""
+    return D <= 128 and context <= (64 if D > 64 else 16) and entries * Hq >= num_sms()
+
+
 def attention_prefill(qkv, k_cache, v_cache, block_table, cu_rows, entry_pos0, max_tiles: int, scale: float,
                       window: int, out, Hq: int, Hkv: int, D: int, err=None, min_rows: int = 1,
                       kernel: str = "auto", sink_score=None, weight_terms: int = 1, softcap: float = 0.0,

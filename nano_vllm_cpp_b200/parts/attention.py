@@ -304,7 +304,7 @@ class PagedAttention(Mixer):
         rounded term), the others to a tensor-core kernel (tcgen05, else mma.sync), where float32 weights enter the product
         with the values as three bfloat16 terms; each of them adds the sink to the softmax's
         denominator (1,500 rows, a sink, three terms: 8 heads of 128 on 2 199 us on mma.sync, 60 on tcgen05, 16 of 64 on 4 111
-        and 62; 64 rows 16 and 13).  ``q``: rows whose first Hq * P elements are the query heads."""
+        and 62; 64 rows 16 and 13; for many short contexts see ``short_contexts_on_mma``).  ``q``: rows whose first Hq * P elements are the query heads."""
         ctx, Hq, Hkv = self.ctx, self.Hq, self.Hkv
         scored = dict(softcap=self.softcap, gate=gate, chunk=self.chunk, slopes=self.slopes, bias_table=self.bias_table)
         single = batch.n_single if ops.attention_decode_usable(cache.k, P) else 0
@@ -317,6 +317,8 @@ class PagedAttention(Mixer):
             tiles = (batch.T - single) // ops.attention_prefill_tile_rows() + (batch.S - single)
             ops.attention_prefill(q, cache.k, cache.v, bt, batch.cu_rows, batch.entry_pos0, tiles, self.scale,
                                   self.window, att, Hq, Hkv, P, err=ctx.err, min_rows=2 if single else 1,
+                                  kernel="mma" if self.sink_score is not None and self.weight_terms == 3
+                                  and ops.short_contexts_on_mma(batch.S - single, Hq, P, batch.max_context) else "auto",
                                   sink_score=self.sink_score, weight_terms=self.weight_terms, **scored)
 
     def _forward_extended(self, proj, bt, batch, cache):

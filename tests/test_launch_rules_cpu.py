@@ -30,3 +30,11 @@ def test_token_tiles_of_256_where_they_are_faster(experts, rows, hidden, inter, 
     (1000, 2048, 2048, 256, 0, 1), (1500, 1024, 1024, 256, 0, 1), (512, 1024, 4096, 256, 0, 9), (128, 512, 3584, 128, 0, 14)])
 def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
     assert ops.lib().nv_tc_gemm_splits(M, N, K, tile, swiglu, 148) == splits
+
+
+@pytest.mark.parametrize("entries,heads,D,context,mma", [
+    (64, 8, 128, 16, True), (24, 8, 128, 64, True), (8, 24, 96, 8, True), (64, 16, 64, 2, True), (64, 16, 64, 32, False),
+    (64, 8, 128, 128, False), (8, 8, 128, 16, False), (1, 8, 128, 64, False), (64, 4, 256, 16, False), (24, 8, 128, 202, False)])
+def test_short_contexts_with_a_sink_take_the_faster_kernel(entries, heads, D, context, mma, monkeypatch):
+    monkeypatch.setattr(ops, "_num_sms", 148)
+    assert ops.short_contexts_on_mma(entries, heads, D, context) is mma
