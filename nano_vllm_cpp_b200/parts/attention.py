@@ -3,6 +3,7 @@ window and a position encoding applied to q and k before the cache write."""
 from __future__ import annotations
 
 import math
+from contextlib import nullcontext
 
 import torch
 
@@ -10,6 +11,9 @@ from ..csrc import ops
 from .base import Mixer, KVCacheSpec, TensorSpec, PartSpec
 from .linear import linear, side_stream
 from .registry import register_part, build_part
+
+
+BESIDE_MIN_ROWS = 512        # a step's rows from which its portions' attention runs beside its single rows' without a capture
 
 
 class PagedAttention(Mixer):
@@ -388,10 +392,13 @@ class PagedAttention(Mixer):
         single = batch.n_single if ops.attention_decode_usable(cache.k, self.D) else 0
         # Both kinds in one step: the portions' kernel, whose few tiles each go through their keys one block after the
         # other, runs on the second stream beside the single rows' stream of pages (64 rows of 200 to 2,048 tokens beside
-        # a portion of 512 behind 1,024: 108 + 53 us a layer one after the other; the step 3.93 -> 3.84 ms).  They write different rows of `att`.
-        main, side = torch.cuda.current_stream(qkv.device), None
-        if 0 < single < batch.S:
-            side, fork, join = side_stream(qkv.device), torch.cuda.Event(), torch.cuda.Event()
+        # a portion of 512 behind 1,024: 108 + 53 us a layer one after the other; the step 3.93 -> 3.84 ms).  They write
+        # different rows of `att`.  Short steps do so only inside a capture: launched one by one they wait for the host,
+        # which the events cost more than the GPU gains (4 rows beside a portion of 64, four layers: 1.42 ms, 1.62 with them).
+        side = None
+        if 0 < single < batch.S and (batch.T >= BESIDE_MIN_ROWS or torch.cuda.is_current_stream_capturing()):
+            main, side = torch.cuda.current_stream(qkv.device), side_stream(qkv.device)
+            fork, join = torch.cuda.Event(), torch.cuda.Event()
             fork.record(main)
             side.wait_event(fork)
         if single < batch.S:
@@ -400,7 +407,7 @@ class PagedAttention(Mixer):
             # an upper bound of the entries' tiles that depends on the step's totals only (CTAs without a tile leave
             # at once): a captured step serves every step with the same totals, however its rows are cut
             tiles = (batch.T - single) // tm + (batch.S - single)
-            with torch.cuda.stream(side if side is not None else main):
+            with torch.cuda.stream(side) if side is not None else nullcontext():
                 ops.attention_prefill(qkv, cache.k, cache.v, bt, batch.cu_rows, batch.entry_pos0, tiles, self.scale,
                                       self.window, att, self.Hq, self.Hkv, self.D, err=ctx.err, min_rows=min_rows)
         if side is not None:

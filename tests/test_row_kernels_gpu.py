@@ -323,7 +323,9 @@ def test_grouped_plain_product_with_tiles_longer_than_its_row_count(M):
 def test_portions_beside_single_rows(refused, monkeypatch):
     """A step with both kinds: the portions' kernel on the second stream sees queries that the main stream has only just
     written, and what follows on the main stream sees its result, also where the single rows' call is refused."""
-    from nano_vllm_cpp_b200.parts.attention import PagedAttention
+    from nano_vllm_cpp_b200.parts import attention
+    PagedAttention = attention.PagedAttention
+    monkeypatch.setattr(attention, "BESIDE_MIN_ROWS", 0)
     o, Hq, Hkv, D, ends, rows = ops(), 4, 2, 64, [70, 33, 60], [1, 1, 40]
     T, i32 = sum(rows), dict(dtype=torch.int32, device=DEV)
     kc, vc, bt = paged(ends, Hkv, D, 3)
