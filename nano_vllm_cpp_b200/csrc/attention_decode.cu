@@ -876,9 +876,9 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
       a.same_kv = 1;
     }
   }
-  // Calls with a sink keep what the lane-per-chunk kernel gives: weights with all their bits, a cap by tanhf, float32 queries as
-  // they are (the tensor-core form rounds queries to bfloat16) and any scale (it takes the largest raw score for the
-  // largest scaled one).
+  // Calls with a sink keep what the lane-per-chunk kernel gives: weights with all their bits, a cap by tanhf, float32
+  // queries as they are (the tensor-core form rounds queries to bfloat16) and any scale (it takes the largest raw score for
+  // the largest scaled one).
   const bool tc = cache_dt == NV_DT_BF16 && D >= 32 && D % 16 == 0 && page <= 256 && num_pages > 0 && tc_stages >= WARPS &&
                   !(has_sink && (q_dt == NV_DT_F32 || !(scale > 0.f)));
   if (tc) {

@@ -179,9 +179,8 @@ __device__ __forceinline__ float capped_log2(const ScoreMap& m, float s) {
 static inline int num_multiprocessors() {
   static const int n = [] {
     int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-      v = 148;
-    return v;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
   }();
   return n;
 }

@@ -1,6 +1,6 @@
 // Matrix memories over many rows, in chunks of eight: the delta rule (one decay per head, or per head and key channel)
-// and the matrix LSTM.  Included by seq_mix_ops.cu, whose row-by-row scan (col_scan_kernel) keeps the steps of a row or
-// two per entry and the float32 runs, whose sums do not depend on how a sequence is cut into steps.
+// and the matrix LSTM.  Included by seq_mix_ops.cu, whose row-by-row scan (col_scan_kernel) keeps the steps of many short
+// entries (memory_chunks_pay in ops.py) and the float32 runs, whose sums do not depend on how a sequence is cut into steps.
 //
 // What bounds the scan is that a row's product with the memory has to be known before the next row changes the memory:
 // a barrier, two shuffled sums and a hundred and sixty FMAs a lane for every row, one after the other (2,048 rows of one
@@ -16,11 +16,11 @@
 // chunk_scan_kernel walks a sequence's chunks with the memory in registers: four columns in sixteen lanes, eight rows of
 // each a lane at 128.  A 16-byte read of shared memory takes a warp four cycles of its multiprocessor's port however many
 // lanes read the same, so what matters is how many FMAs such a read feeds (16 here; with a column in eight lanes
-// and one column a lane the port was the kernel's time).  The eight sums of a column's chunk end, after eight shuffles, with lane i
-// holding row i's.  The matrix LSTM is the same without the first product and with weights exp(F_i - F_j + i_j - m_i) for
+// and one column a lane the port was the kernel's time).  The eight sums of a column's chunk end, after eight shuffles, with
+// lane i holding row i's.  The matrix LSTM is the same without the first product and with weights exp(F_i - F_j + i_j - m_i) for
 // the quotients (F the running sum of the log forget gates, m_i the running maximum).
-// Measured (heads of 128 x 128, preparation, gates and head norm included): 1,500 rows of one sequence, 8 heads: delta rule 576 ->
-// 281 us, matrix LSTM 531 -> 277; eight sequences of 200 to 2,048 rows, 16 heads, a decay per channel: 1,870 -> 734 us
+// Measured (heads of 128 x 128, preparation, gates and head norm included): 1,500 rows of one sequence, 8 heads: delta rule
+// 576 -> 281 us, matrix LSTM 531 -> 277; eight sequences of 200 to 2,048 rows, 16 heads, a decay per channel: 1,870 -> 734 us
 // (825 before two FMAs went into one instruction and the longest sequences first).  Against float64
 // the states are off by no more than row by row (tests/test_memory_chunks_gpu.py).
 
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
   const size_t rec_step = (size_t)a.H * REC;
   auto fetch = [&](int c) {
     if (c < chunks)
-      for (int i = tid; i < REC / 4; i += 32 * WARPS) cp_async16(ring + (c % MC_RING) * REC + 4 * i, rec + c * rec_step + 4 * i);
+      for (int i = tid; i < REC / 4; i += 32 * WARPS)
+        cp_async16(ring + (c % MC_RING) * REC + 4 * i, rec + c * rec_step + 4 * i);
     cp_async_commit();
   };
   for (int c = 0; c < MC_RING - 1; ++c) fetch(c);
@@ -255,7 +256,8 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
       const int r = 4 * (l + MC_LANES * p) + 2 * i;
 #pragma unroll
       for (int t = 0; t < CT; ++t)
-        S[p][i][t] = make_float2(col + t < ncols && r < dk ? *place(t, r) : 0.f, col + t < ncols && r + 1 < dk ? *place(t, r + 1) : 0.f);
+        S[p][i][t] = make_float2(col + t < ncols && r < dk ? *place(t, r) : 0.f,
+                                 col + t < ncols && r + 1 < dk ? *place(t, r + 1) : 0.f);
     }
   float m0 = LSTM ? a.m[(size_t)slot * a.m_stride + h] : 0.f;
   const float* vp = a.vsrc + (size_t)(row0 + row) * a.v_ld + a.v0 + (size_t)h * dv + col;
@@ -312,7 +314,10 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
     if (LSTM) {
       float f[MC_R], g[MC_R];
 #pragma unroll
-      for (int i = 0; i < MC_R; i += 4) { *(float4*)(f + i) = *(const float4*)(tri + i); *(float4*)(g + i) = *(const float4*)(tri + 8 + i); }
+      for (int i = 0; i < MC_R; i += 4) {
+        *(float4*)(f + i) = *(const float4*)(tri + i);
+        *(float4*)(g + i) = *(const float4*)(tri + 8 + i);
+      }
       float F = 0.f, mine = 0.f;                   // F: running sum of the log forget gates; this lane's row's
 #pragma unroll
       for (int j = 0; j < MC_R; ++j) { F += f[j]; f[j] = F; if (j <= row) mine = F; }
@@ -349,7 +354,7 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
       for (int j = 0; j < MC_R; ++j)
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
-          u[t][j] = __shfl_sync(0xffffffffu, beta * acc[t], j, MC_LANES);       // (what rows before j take off has been taken off)
+          u[t][j] = __shfl_sync(0xffffffffu, beta * acc[t], j, MC_LANES);       // (rows before j have taken theirs off)
           acc[t] = fmaf(-kkr[j], u[t][j], acc[t]);
           if (j <= row) o[t] = fmaf(qkr[j], u[t][j], o[t]);          // (0 times a later row's infinity would be NaN)
         }
@@ -417,7 +422,7 @@ int launch_chunks(const ChunkArgs& p, const ChunkScanArgs& a, int T, cudaStream_
   // Blocks of 32 columns share a record between four warps; where they would not give every multiprocessor one, blocks of
   // eight columns spread a few sequences further.
   const long long wide = (long long)S * a.H * ((a.dv + 31) / 32);
-  return wide >= 148 ? launch_chunk_scan<DK, LSTM, 4>(a, S, s) : launch_chunk_scan<DK, LSTM, 1>(a, S, s);
+  return wide >= num_multiprocessors() ? launch_chunk_scan<DK, LSTM, 4>(a, S, s) : launch_chunk_scan<DK, LSTM, 1>(a, S, s);
 }
 
 template <bool LSTM>

@@ -795,8 +795,8 @@ def moe_route_small(logits, K: int, renorm: bool, C: int, gate_logit, idx, score
 
 class StaticTiles:
     """The tiles of C experts E .. E + C - 1 that each take all T rows, in row order, their segments behind the
-    T * K routed pairs: what ``moe_route_small(static=True)`` leaves out of its list.  ``hidden``, ``inter``: the experts' sizes,
-    as in ``grouped_token_tile``."""
+    T * K routed pairs: what ``moe_route_small(static=True)`` leaves out of its list.  ``hidden``, ``inter``: the experts'
+    sizes, as in ``grouped_token_tile``."""
 
     def __init__(self, T: int, K: int, E: int, C: int, device, hidden: int = 0, inter: int = 0):
         self.tile_m = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128

@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(128) gemm_plain_kernel(GemmArgs g) {
 template <typename TA, typename TW, bool SWIGLU, int FT, int KC, int ST>
 int launch_form(const GemmArgs& g, int m_tiles, cudaStream_t s) {
   const dim3 grid((g.N + 16 * FT - 1) / (16 * FT), m_tiles);
-  const size_t smem = (size_t)ST * ((SWIGLU ? 2 : 1) * 16 * FT * (KC * sizeof(TW) + 16) + g.rows_alloc * (KC * sizeof(TA) + 16));
+  const size_t w_bytes = (SWIGLU ? 2 : 1) * 16 * FT * (KC * sizeof(TW) + 16), a_bytes = g.rows_alloc * (KC * sizeof(TA) + 16);
+  const size_t smem = ST * (w_bytes + a_bytes);
   auto* kernel = gemm_plain_kernel<TA, TW, SWIGLU, FT, KC, ST>;
   if (smem > 48 * 1024) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   NV_RETURN_IF(launch_dep(kernel, grid, dim3(128), smem, s, g));

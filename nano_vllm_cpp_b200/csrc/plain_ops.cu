@@ -403,13 +403,14 @@ __global__ void __launch_bounds__(256) rope_store_kernel(void* __restrict__ qkv,
 // A chunk's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
 // output element.  The heads of a block share the keys and values they read and run their chains side by side.  Keys come
 // in slices of 32 elements through NB buffers of shared memory (cp.async, whole sectors; a thread reads its own key's slice
-// 16 bytes at a time, rows 144 bytes apart, 80 for bfloat16 keys: no bank conflicts): two where many blocks hide each other's waits, four, so that a chunk's
-// keys are asked for at once, where a few rows leave multiprocessors idle.  Values are asked for 32 keys ahead, the first
-// before the scores.  The order of every sum is that of the element-by-element form, bit for bit.
-// Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 102 us element by element, 45 with keys in
-// slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.  bfloat16 caches (copied as they are
-// and widened from shared memory; element by element a slice was waited for 32 times over): one row at 4,096 keys 750 us
-// element by element from memory, 2,004 through slices copied so, 351 now.
+// 16 bytes at a time, rows 144 bytes apart, 80 for bfloat16 keys: no bank conflicts): two where many blocks hide each
+// other's waits, four, so that a chunk's keys are asked for at once, where a few rows leave multiprocessors idle.  Values
+// are asked for 32 keys ahead, the first before the scores.  The order of every sum is that of the element-by-element form,
+// bit for bit.
+// Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 102 us element by element, 45 with
+// keys in slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.  bfloat16 caches (copied
+// as they are and widened from shared memory; element by element a slice was waited for 32 times over): one row at 4,096
+// keys 750 us element by element from memory, 2,004 through slices copied so, 351 now.
 constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_AHEAD = 32;
 
 template <bool MAX, int HB>
@@ -610,12 +611,13 @@ int launch_plain_attention(const void* qkv, int dt, int q_stride, const TC* kc, 
                            int max_blocks, const int* row_entry, const int* positions, float scale, int window, void* out,
                            int out_dt, int T, int Hq, int Hkv, int D, int page, cudaStream_t s) {
   const dim3 grid(T, Hq / HB);
-  const bool few = (long long)T * (Hq / HB) <= 2 * num_multiprocessors();      // (four buffers leave a multiprocessor room for three blocks)
+  // (four buffers leave a multiprocessor room for three blocks)
+  const bool few = (long long)T * (Hq / HB) <= 2 * num_multiprocessors();
   const size_t smem = (few ? 4 : 2) * sizeof(KeySlice<TC>);
   auto* kernel = few ? paged_attention_plain_kernel<TC, HB, 4> : paged_attention_plain_kernel<TC, HB, 2>;
   if (few) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  NV_RETURN_IF(launch_dep(kernel, grid, dim3(ATT_THREADS), smem, s, qkv, dt, q_stride, kc, vc, block_table, max_blocks, row_entry,
-                          positions, scale, window, out, out_dt, Hq, Hkv, D, page));
+  NV_RETURN_IF(launch_dep(kernel, grid, dim3(ATT_THREADS), smem, s, qkv, dt, q_stride, kc, vc, block_table, max_blocks,
+                          row_entry, positions, scale, window, out, out_dt, Hq, Hkv, D, page));
   NV_RETURN_LAST();
 }
 
@@ -839,16 +841,14 @@ NV_API int nv_paged_attention_plain(const void* qkv, int dt, int q_stride, const
   if (D > 256 || D <= 0 || Hkv <= 0 || Hq % Hkv) return NV_ERR_UNSUPPORTED;
   if (T == 0) return NV_OK;
   auto go = [&](auto* k, auto* v) {
+    using TC = std::remove_cv_t<std::remove_pointer_t<decltype(k)>>;
     // (a few rows: a block per head, since there are multiprocessors for all of them; many: heads share what they read)
     const int group = (long long)T * Hq <= 4 * num_multiprocessors() ? 1 : Hq / Hkv;
-    if (group % 4 == 0)
-      return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 4>(
-          qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
-    if (group % 2 == 0)
-      return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 2>(
-          qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
-    return launch_plain_attention<std::remove_cv_t<std::remove_pointer_t<decltype(k)>>, 1>(
-        qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv, D, page, s);
+    auto* launch = group % 4 == 0   ? launch_plain_attention<TC, 4>
+                   : group % 2 == 0 ? launch_plain_attention<TC, 2>
+                                    : launch_plain_attention<TC, 1>;
+    return launch(qkv, dt, q_stride, k, v, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt, T, Hq, Hkv,
+                  D, page, s);
   };
   return cache_dt == NV_DT_F32 ? go((const float*)kc, (const float*)vc) : go((const bf16*)kc, (const bf16*)vc);
 }

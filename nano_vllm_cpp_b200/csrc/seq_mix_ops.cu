@@ -758,9 +758,9 @@ __global__ void __launch_bounds__(ATTG_THREADS) paged_attention_general_kernel(
 // q [T, H, D] float32 -> out [T, H, G * D]: out[t, h, c D + d] = sum over the heads g of kv head c of
 // mix[h, g] * q[t, g, d].  With it, sum_g mix[h, g] (q_g . k_kv(g)) is one product of the mixed query row with the
 // kv heads' keys side by side.  One block per row.
-// A thread keeps four elements of a kv head's REP query heads in registers and goes through the output heads, one
-// 16-byte read of weights per REP = 4 and sixteen FFMAs at a time (an element a thread, indices divided out and every operand read
-// from shared memory: 244 us for 6,737 rows of 16 heads of 128 on 4 kv heads; now 38 us, and 8 instead of 18 for eight rows).
+// A thread keeps four elements of a kv head's REP query heads in registers and goes through the output heads, REP weights
+// from shared memory and 4 REP FFMAs at a time (an element a thread, indices divided out and every operand read from shared
+// memory: 244 us for 6,737 rows of 16 heads of 128 on 4 kv heads; now 38 us, and 8 instead of 18 for eight rows).
 template <int REP>
 __global__ void __launch_bounds__(256) mix_query_heads_kernel(const float* __restrict__ q, const float* __restrict__ mix,
                                                               void* __restrict__ out, int out_dt, int H, int G, int D) {
@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(256) mix_query_heads_kernel(const float* __res
   const int t = blockIdx.x, quads = G * D / 4, rep = H / G;
   for (int i = threadIdx.x; i < H * H; i += blockDim.x) wm[i] = mix[i];
   __syncthreads();
-  const int per = blockDim.x / quads > 0 ? blockDim.x / quads : 1;        // threads that share out the output heads of four elements
+  const int per = blockDim.x / quads > 0 ? blockDim.x / quads : 1;      // threads that share out the heads of four elements
   for (int i = threadIdx.x; i < quads * per; i += blockDim.x) {
     const int at = i % quads, c = 4 * at / D, d = 4 * at % D;
     const float* src = q + (size_t)t * H * D + (size_t)c * rep * D + d;
@@ -911,7 +911,7 @@ __global__ void __launch_bounds__(HP_THREADS) head_project_kernel(const void* __
 __global__ void head_gate_kernel(const float* __restrict__ x, const float* __restrict__ gate, long long gate_ld, int gate0,
                                  void* __restrict__ out, int out_dt, long long total, int H, int N, int gate_each, int four) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (four) {                          // one gate per head, heads of whole quads: four elements a thread (65 -> 21 us for 6,737 x 2,048)
+  if (four) {                // one gate per head, heads of whole quads: four elements a thread (65 -> 21 us for 6,737 x 2,048)
     i *= 4;
     if (i >= total) return;
     const long long th = i / N;
@@ -1679,7 +1679,8 @@ NV_API int nv_head_gate(const float* x, const float* gate, long long gate_ld, in
   const long long total = (long long)T * H * N;
   const int four = !gate_each && out_dt == NV_DT_BF16 && N % 4 == 0 && (((uintptr_t)x & 15) | ((uintptr_t)out & 7)) == 0;
   const long long threads = four ? total / 4 : total;
-  head_gate_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(x, gate, gate_ld, gate0, out, out_dt, total, H, N, gate_each, four);
+  head_gate_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(x, gate, gate_ld, gate0, out, out_dt, total, H, N,
+                                                                    gate_each, four);
   NV_RETURN_LAST();
 }
 
@@ -1714,12 +1715,12 @@ NV_API int nv_mlstm_col_scan(const float* proj, long long ld, int q0, int k0, in
     a.raw = raw; a.RW = dv + 2; a.H = H; a.dk = dk; a.dv = dv;
     rc = launch_chunks_of<true>(p, a, T, s);
   } else {
-  ColArgs a = {};
-  a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.n = n; a.n_stride = n_stride;
-  a.m = m; a.m_stride = m_stride; a.qk = proj; a.qk_ld = ld; a.q0 = q0; a.k0 = k0; a.G = H; a.vsrc = proj; a.v_ld = ld;
-  a.v0 = v0; a.gates = proj; a.gates_dt = NV_DT_F32; a.gates_ld = ld; a.ga0 = i0; a.gb0 = f0; a.cap = cap;
-  a.q_scale = q_scale; a.raw = raw; a.RW = dv + 2; a.H = H; a.dk = dk; a.dv = dv;
-  rc = launch_col_scan<0>(a, num_entries, T, gate_buf, s);
+    ColArgs a = {};
+    a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.n = n; a.n_stride = n_stride;
+    a.m = m; a.m_stride = m_stride; a.qk = proj; a.qk_ld = ld; a.q0 = q0; a.k0 = k0; a.G = H; a.vsrc = proj; a.v_ld = ld;
+    a.v0 = v0; a.gates = proj; a.gates_dt = NV_DT_F32; a.gates_ld = ld; a.ga0 = i0; a.gb0 = f0; a.cap = cap;
+    a.q_scale = q_scale; a.raw = raw; a.RW = dv + 2; a.H = H; a.dk = dk; a.dv = dv;
+    rc = launch_col_scan<0>(a, num_entries, T, gate_buf, s);
   }
   if (rc) return rc;
   return launch_head_finish(raw, dv + 2, 1, den_eps, proj, NV_DT_F32, ld, g0, 0, norm_w, norm_per_head, eps, out, out_dt, T, H,
@@ -1757,12 +1758,12 @@ NV_API int nv_gated_delta_col_scan(const float* qkv, int C, int q0, int k0, int 
     rc = delta_chunks(qkv, C, q0, k0, v0, G, proj, proj_dt, ld, b0, a0, nullptr, 0, 0, A_log, dt_bias, cu_rows, entry_slot,
                       S, S_stride, H, dk, dv, raw, chunk_buf, num_entries, T, s);
   } else {
-  ColArgs a = {};
-  a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.qk = qkv; a.qk_ld = C; a.q0 = q0;
-  a.k0 = k0; a.G = G; a.vsrc = qkv; a.v_ld = C; a.v0 = v0; a.gates = proj; a.gates_dt = proj_dt; a.gates_ld = ld;
-  a.ga0 = b0; a.gb0 = a0; a.A_log = A_log; a.dt_bias = dt_bias; a.q_scale = 1.f; a.raw = raw; a.RW = dv; a.H = H;
-  a.dk = dk; a.dv = dv;
-  rc = launch_col_scan<1>(a, num_entries, T, gate_buf, s);
+    ColArgs a = {};
+    a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.qk = qkv; a.qk_ld = C; a.q0 = q0;
+    a.k0 = k0; a.G = G; a.vsrc = qkv; a.v_ld = C; a.v0 = v0; a.gates = proj; a.gates_dt = proj_dt; a.gates_ld = ld;
+    a.ga0 = b0; a.gb0 = a0; a.A_log = A_log; a.dt_bias = dt_bias; a.q_scale = 1.f; a.raw = raw; a.RW = dv; a.H = H;
+    a.dk = dk; a.dv = dv;
+    rc = launch_col_scan<1>(a, num_entries, T, gate_buf, s);
   }
   if (rc) return rc;
   return launch_head_finish(raw, dv, 0, 0.f, proj, proj_dt, ld, g0, 1, norm_w, 0, eps, out, out_dt, T, H, dv, MaxState{}, s);
@@ -1787,19 +1788,19 @@ NV_API int nv_channel_delta_scan(const float* qkv, int C, int q0, int k0, int v0
     rc = delta_chunks(qkv, C, q0, k0, v0, G, proj, proj_dt, ld, b0, 0, dec, dec_ld, dec0, A_log, dt_bias, cu_rows, entry_slot,
                       S, S_stride, H, dk, dv, raw, chunk_buf, num_entries, T, s);
   } else {
-  const long long n = (long long)T * H * dk;
-  channel_gates_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dec, dec_ld, dec0, proj, proj_dt, ld, b0, A_log,
-                                                                  dt_bias, H, dk, decays, gate_buf, n);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
-  ColArgs a = {};
-  a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.qk = qkv; a.qk_ld = C; a.q0 = q0;
-  a.k0 = k0; a.G = G; a.vsrc = qkv; a.v_ld = C; a.v0 = v0; a.gates = gate_buf; a.gates_dt = NV_DT_F32;
-  a.gates_ld = 2LL * H; a.ga0 = 0; a.gb0 = 1; a.A_log = A_log; a.dt_bias = dt_bias; a.q_scale = 1.f; a.raw = raw;
-  a.RW = dv; a.H = H; a.dk = dk; a.dv = dv; a.dec = decays; a.dec_ld = (long long)H * dk;
-  a.vec16 = (((uintptr_t)qkv & 15) == 0 && C % 4 == 0 && q0 % 4 == 0 && k0 % 4 == 0 && dk % 4 == 0 &&
-             ((uintptr_t)decays & 15) == 0) ? 1 : 0;
-  rc = launch_col_scan_p<2, true>(a, num_entries, s);
+    const long long n = (long long)T * H * dk;
+    channel_gates_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dec, dec_ld, dec0, proj, proj_dt, ld, b0, A_log,
+                                                                    dt_bias, H, dk, decays, gate_buf, n);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    ColArgs a = {};
+    a.cu_rows = cu_rows; a.entry_slot = entry_slot; a.S = S; a.S_stride = S_stride; a.qk = qkv; a.qk_ld = C; a.q0 = q0;
+    a.k0 = k0; a.G = G; a.vsrc = qkv; a.v_ld = C; a.v0 = v0; a.gates = gate_buf; a.gates_dt = NV_DT_F32;
+    a.gates_ld = 2LL * H; a.ga0 = 0; a.gb0 = 1; a.A_log = A_log; a.dt_bias = dt_bias; a.q_scale = 1.f; a.raw = raw;
+    a.RW = dv; a.H = H; a.dk = dk; a.dv = dv; a.dec = decays; a.dec_ld = (long long)H * dk;
+    a.vec16 = (((uintptr_t)qkv & 15) == 0 && C % 4 == 0 && q0 % 4 == 0 && k0 % 4 == 0 && dk % 4 == 0 &&
+               ((uintptr_t)decays & 15) == 0) ? 1 : 0;
+    rc = launch_col_scan_p<2, true>(a, num_entries, s);
   }
   if (rc) return rc;
   return launch_head_finish(raw, dv, 0, 0.f, gsrc, gsrc_dt, gsrc_ld, g0, gate_mode == 1 ? 0 : 1, norm_w, 0, eps, out, out_dt, T,
