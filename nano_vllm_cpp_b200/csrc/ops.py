@@ -71,11 +71,12 @@ def lib() -> ctypes.CDLL:
     if _lib is None:
         path = _build.library_path()
         try:
-            _lib = ctypes.CDLL(path)
-        except OSError as e:
+            loaded = ctypes.CDLL(path)
+            _declare(loaded)
+        except (OSError, AttributeError) as e:       # (AttributeError: a launcher of the sources is not in the library)
             raise KernelError(f"cannot load the CUDA library {path}: {e}") from None
-        _declare(_lib)
-        _lib.nv_set_dependent_launch(_early())
+        loaded.nv_set_dependent_launch(_early())
+        _lib = loaded                      # only now: without its types a launcher would be called with half of a pointer
     return _lib
 
 

@@ -38,3 +38,17 @@ def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
 def test_short_contexts_with_a_sink_take_the_faster_kernel(entries, heads, D, context, mma, monkeypatch):
     monkeypatch.setattr(ops, "_num_sms", 148)
     assert ops.short_contexts_on_mma(entries, heads, D, context) is mma
+
+
+def test_a_library_without_a_launcher_is_refused_at_every_call(monkeypatch):
+    """A library that is older than the sources: the first call says so, and so does every later one (a launcher whose types
+    were never declared would get its 64-bit addresses as 32-bit numbers)."""
+    class Old:
+        def __getattr__(self, name):
+            raise AttributeError(f"undefined symbol: {name}")
+
+    monkeypatch.setattr(ops, "_lib", None)
+    monkeypatch.setattr(ops.ctypes, "CDLL", lambda path: Old())
+    for _ in range(2):
+        with pytest.raises(ops.KernelError, match="undefined symbol"):
+            ops.lib()
