@@ -494,7 +494,8 @@ def short_contexts_on_mma(entries: int, Hq: int, D: int, context: int) -> bool:
     mma.sync kernel: its blocks are cheaper to begin, which counts where there are more of them than multiprocessors and
     each has a block of keys or two.  Measured, tcgen05 and mma.sync: 8 heads of 128 on 2, 64 fresh prompts of 16 tokens
     35 and 30 us, of 64 45 and 42, of 128 65 and 73, eight of 16 7 and 11; 24 heads of 96 on 4, 64 of 16 98 and 73, 64 of 2
-    behind 200 170 and 168; 16 heads of 64 on 4, 64 of 2 34 and 31, of 32 39 and 41."""
+    behind 200 170 and 168; 16 heads of 64 on 4, 64 of 2 34 and 31, of 32 39 and 41.  A captured step serves any contexts
+    and names the longest there may be: it takes the tcgen05 kernel, some microseconds a layer slower where they are short."""
     return D <= 128 and context <= (64 if D > 64 else 16) and entries * Hq >= num_sms()
 
 
