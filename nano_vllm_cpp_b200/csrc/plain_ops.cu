@@ -396,22 +396,24 @@ __global__ void __launch_bounds__(256) rope_store_kernel(void* __restrict__ qkv,
 }
 
 // --------------------------------------------------------------- paged attention (plain)
-// One block per row and HB query heads of one kv head.  Row t with position p sees keys [lo, p] where
-// lo = max(0, p + 1 - window) (window 0 = all).  Keys are taken in chunks of 128 from lo
-// upward with an online softmax; everything is fp32 (src/hip_ops.hip:473-551).
+// One block, or a cluster of eight, per row and HB query heads of one kv head.  Row t with position p sees keys [lo, p]
+// where lo = max(0, p + 1 - window) (window 0 = all).  Keys are taken in chunks of 128 from lo upward; a chunk has a softmax of
+// its own (its largest score, the sum of its weights, the weighted sum of its values, from zero), and the chunks are merged
+// in order; everything is fp32 (src/hip_ops.hip:473-551).
 //
 // A chunk's time is latency: the chain of D FFMAs of a score, the trees over 128 threads, the chain of 128 FFMAs of an
 // output element.  The heads of a block share the keys and values they read and run their chains side by side.  Keys come
 // in slices of 32 elements through NB buffers of shared memory (cp.async, whole sectors; a thread reads its own key's slice
 // 16 bytes at a time, rows 144 bytes apart, 80 for bfloat16 keys: no bank conflicts): two where many blocks hide each
 // other's waits, four, so that a chunk's keys are asked for at once, where a few rows leave multiprocessors idle.  Values
-// are asked for 32 keys ahead, the first before the scores.  The order of every sum is that of the element-by-element form,
-// bit for bit.
-// Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 102 us element by element, 45 with
-// keys in slices, 35 so; the 408 rows of their prompts 90 -> 69 us where four heads share a block.  bfloat16 caches (copied
+// are asked for 32 keys ahead, the first before the scores.  A handful of rows goes further: the blocks of a cluster (CL = 8)
+// take every eighth chunk, with values 64 keys ahead, and the first merges them out of distributed shared memory.  Which of
+// these a row takes changes no bit of it: the order of every sum depends on its position and the window alone.
+// Measured (float32, 8 heads of 128 on 2 kv heads): two decoded rows at 75 and 333 tokens 33 us in a
+// block a head, 16 in a cluster a head; the 408 rows of their prompts 90 -> 69 us where four heads share a block.  bfloat16 caches (copied
 // as they are and widened from shared memory; element by element a slice was waited for 32 times over): one row at 4,096
-// keys 750 us element by element from memory, 2,004 through slices copied so, 351 now.
-constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_AHEAD = 32;
+// keys 750 us element by element from memory, 2,004 through slices copied so, 351 in a block by itself.
+constexpr int ATT_THREADS = 128, ATT_SLICE = 32, ATT_CLUSTER = 8;
 
 template <bool MAX, int HB>
 __device__ __forceinline__ void chunk_trees(float (&v)[HB], float (*red)[ATT_THREADS], int tid) {
@@ -475,7 +477,7 @@ __device__ __forceinline__ void key_piece(const bf16* p, float (&v)[8]) {
   for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 
-template <typename TC, int HB, int NB>
+template <typename TC, int HB, int NB, int CL>
 __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     const void* __restrict__ qkv, int dt, int q_stride, const TC* __restrict__ kc, const TC* __restrict__ vc,
     const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_entry,
@@ -487,10 +489,11 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
   __shared__ int pslot[ATT_THREADS];   // element offset / D of each key of the chunk
   __shared__ float red[HB][ATT_THREADS];
   KeySlice<TC>* keys = (KeySlice<TC>*)att_keys;
-  constexpr int PER = KeySlice<TC>::PER;
+  float* kept = (float*)(att_keys + NB * sizeof(KeySlice<TC>));        // (cluster) this block's chunks: [chunk][HB][D + 2]
+  constexpr int PER = KeySlice<TC>::PER, AHEAD = CL > 1 ? 64 : 32;
   grid_dep_wait();
   grid_dep_launch();
-  const int t = blockIdx.x, h0 = blockIdx.y * HB, tid = threadIdx.x;
+  const int t = blockIdx.x / CL, rank = blockIdx.x % CL, h0 = blockIdx.y * HB, tid = threadIdx.x;
   const int kvh = h0 / (Hq / Hkv);
   const int n = positions[t] + 1;
   const int lo = window > 0 ? max(0, n - window) : 0;
@@ -501,7 +504,15 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
   float m[HB], l[HB], o[2][HB];
 #pragma unroll
   for (int b = 0; b < HB; ++b) { m[b] = -1e30f; l[b] = 0.f; o[0][b] = o[1][b] = 0.f; }
-  for (int c0 = lo; c0 < n; c0 += ATT_THREADS) {
+  // the chunks so far, (m, l, o), and one more: what both are worth beside the larger of the two maxima
+  auto merge = [&](int b, float cm, float cl, const float (&co)[2]) {
+    const float top = fmaxf(m[b], cm), w = expf(__fsub_rn(m[b], top)), cw = expf(__fsub_rn(cm, top));
+    m[b] = top;
+    l[b] = fmaf(l[b], w, __fmul_rn(cl, cw));
+#pragma unroll
+    for (int half = 0; half < 2; ++half) o[half][b] = fmaf(o[half][b], w, __fmul_rn(co[half], cw));
+  };
+  for (int c0 = lo + rank * ATT_THREADS; c0 < n; c0 += CL * ATT_THREADS) {
     const int j = c0 + tid, cnt = min(ATT_THREADS, n - c0);
     if (j < n) pslot[tid] = (bt[j / page] * Hkv + kvh) * page + j % page;
     __syncthreads();
@@ -509,9 +520,9 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
       if (sl < slices) stage_keys(keys[sl], kc, pslot, cnt, D, sl * ATT_SLICE, tid);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    uint32_t val[ATT_AHEAD];
+    uint32_t val[AHEAD];
 #pragma unroll
-    for (int i = 0; i < ATT_AHEAD; ++i) val[i] = tid < D && i < cnt ? raw_value(vc + (size_t)pslot[i] * D + tid) : 0u;
+    for (int i = 0; i < AHEAD; ++i) val[i] = tid < D && i < cnt ? raw_value(vc + (size_t)pslot[i] * D + tid) : 0u;
     float s[HB];
 #pragma unroll
     for (int b = 0; b < HB; ++b) s[b] = 0.f;
@@ -550,52 +561,92 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
       }
       __syncthreads();
     }
-    float top[HB], sum[HB];
+    float top[HB], sum[HB], co[HB][2];
 #pragma unroll
     for (int b = 0; b < HB; ++b) top[b] = s[b] = j < n ? __fmul_rn(s[b], scale) : -1e30f;
     chunk_trees<true, HB>(top, red, tid);
 #pragma unroll
     for (int b = 0; b < HB; ++b) {
-      const float m_new = fmaxf(m[b], top[b]);
-      // (every rounding is spelled out: the forms with one, two and four heads must not be contracted differently)
-      p[b][tid] = sum[b] = j < n ? expf(__fsub_rn(s[b], m_new)) : 0.f;
-      top[b] = expf(__fsub_rn(m[b], m_new));                 // what the sums so far are worth now
-      m[b] = m_new;
+      // (every rounding is spelled out: the forms must not be contracted differently)
+      top[b] = fmaxf(top[b], -1e30f);
+      p[b][tid] = sum[b] = j < n ? expf(__fsub_rn(s[b], top[b])) : 0.f;
+      co[b][0] = co[b][1] = 0.f;
     }
     chunk_trees<false, HB>(sum, red, tid);
-#pragma unroll
-    for (int b = 0; b < HB; ++b) {
-      l[b] = fmaf(l[b], top[b], sum[b]);
-      o[0][b] *= top[b];
-      o[1][b] *= top[b];
-    }
     for (int half = 0; half < halves; ++half) {
       const int d = tid + half * ATT_THREADS;
-      for (int i0 = 0; i0 < cnt; i0 += ATT_AHEAD) {
-        uint32_t now[ATT_AHEAD];
+      for (int i0 = 0; i0 < cnt; i0 += AHEAD) {
+        uint32_t now[AHEAD];
 #pragma unroll
-        for (int i = 0; i < ATT_AHEAD; ++i) now[i] = val[i];
-        const bool wrap = i0 + ATT_AHEAD >= cnt;             // the values after this half's are the next half's first
-        const int nd = wrap ? d + ATT_THREADS : d, ni = wrap ? 0 : i0 + ATT_AHEAD;
+        for (int i = 0; i < AHEAD; ++i) now[i] = val[i];
+        const bool wrap = i0 + AHEAD >= cnt;             // the values after this half's are the next half's first
+        const int nd = wrap ? d + ATT_THREADS : d, ni = wrap ? 0 : i0 + AHEAD;
         if (!wrap || half + 1 < halves) {
 #pragma unroll
-          for (int i = 0; i < ATT_AHEAD; ++i)
+          for (int i = 0; i < AHEAD; ++i)
             val[i] = nd < D && ni + i < cnt ? raw_value(vc + (size_t)pslot[ni + i] * D + nd) : 0u;
         }
-        const int k = min(ATT_AHEAD, cnt - i0);
+        const int k = min(AHEAD, cnt - i0);
 #pragma unroll
-        for (int i = 0; i < ATT_AHEAD; ++i)
+        for (int i = 0; i < AHEAD; ++i)
           if (i < k) {
 #pragma unroll
             for (int b = 0; b < HB; ++b) {
               const float w = p[b][i0 + i];
-              if (half == 0) o[0][b] = fmaf(w, wide_value<TC>(now[i]), o[0][b]);
-              else o[1][b] = fmaf(w, wide_value<TC>(now[i]), o[1][b]);
+              if (half == 0) co[b][0] = fmaf(w, wide_value<TC>(now[i]), co[b][0]);
+              else co[b][1] = fmaf(w, wide_value<TC>(now[i]), co[b][1]);
             }
           }
       }
     }
+    if (CL == 1) {
+#pragma unroll
+      for (int b = 0; b < HB; ++b) merge(b, top[b], sum[b], co[b]);
+    } else {
+#pragma unroll
+      for (int b = 0; b < HB; ++b) {
+        float* to = kept + ((c0 - lo) / (CL * ATT_THREADS) * HB + b) * (D + 2);
+        if (tid < D) to[tid] = co[b][0];
+        if (tid + ATT_THREADS < D) to[tid + ATT_THREADS] = co[b][1];
+        if (tid == 0) { to[D] = top[b]; to[D + 1] = sum[b]; }
+      }
+    }
     __syncthreads();
+  }
+  if (CL > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank == 0) {
+      auto there = [&](const float* at, int q) {
+        uint32_t a;
+        float v;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(q));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+        return v;
+      };
+      const int chunks = (n - lo + ATT_THREADS - 1) / ATT_THREADS;
+      for (int x = 0; x < chunks; x += CL) {
+        float cm[CL][HB], cl[CL][HB], co[CL][HB][2];
+#pragma unroll
+        for (int q = 0; q < CL; ++q)
+          if (x + q < chunks)
+#pragma unroll
+            for (int b = 0; b < HB; ++b) {
+              const float* from = kept + (x / CL * HB + b) * (D + 2);
+              cm[q][b] = there(from + D, q);
+              cl[q][b] = there(from + D + 1, q);
+              co[q][b][0] = tid < D ? there(from + tid, q) : 0.f;
+              co[q][b][1] = tid + ATT_THREADS < D ? there(from + tid + ATT_THREADS, q) : 0.f;
+            }
+#pragma unroll
+        for (int q = 0; q < CL; ++q)
+          if (x + q < chunks)
+#pragma unroll
+            for (int b = 0; b < HB; ++b) merge(b, cm[q][b], cl[q][b], co[q][b]);
+      }
+    }
+    // (nobody leaves while the first block still reads)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank != 0) return;
   }
 #pragma unroll
   for (int b = 0; b < HB; ++b) {
@@ -610,11 +661,37 @@ template <typename TC, int HB>
 int launch_plain_attention(const void* qkv, int dt, int q_stride, const TC* kc, const TC* vc, const int* block_table,
                            int max_blocks, const int* row_entry, const int* positions, float scale, int window, void* out,
                            int out_dt, int T, int Hq, int Hkv, int D, int page, cudaStream_t s) {
+  // A handful of rows: a cluster each, if the block tables reach beyond a chunk and what a block keeps of its chunks fits
+  // (two decoded rows of 8 heads: 33 us in blocks, 16 in clusters; blocks that fill the GPU by themselves stay alone).
+  const long long blocks = (long long)T * (Hq / HB);
+  const long long longest = window > 0 ? min((long long)window, (long long)max_blocks * page) : (long long)max_blocks * page;
+  const long long kept = (longest + ATT_CLUSTER * ATT_THREADS - 1) / (ATT_CLUSTER * ATT_THREADS) * HB * (D + 2) * 4;
+  if (ATT_CLUSTER * blocks <= 4 * num_multiprocessors() && longest > ATT_THREADS && kept <= 64 * 1024) {
+    const size_t smem = 4 * sizeof(KeySlice<TC>) + (size_t)kept;
+    auto* kernel = paged_attention_plain_kernel<TC, HB, 4, ATT_CLUSTER>;
+    NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * sizeof(KeySlice<TC>) + 64 * 1024)));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(T * ATT_CLUSTER, Hq / HB);
+    cfg.blockDim = dim3(ATT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = g_nv_dependent_launch ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ATT_CLUSTER;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    NV_RETURN_IF(cudaLaunchKernelEx(&cfg, kernel, qkv, dt, q_stride, kc, vc, block_table, max_blocks, row_entry, positions, scale,
+                                    window, out, out_dt, Hq, Hkv, D, page));
+    NV_RETURN_LAST();
+  }
   const dim3 grid(T, Hq / HB);
   // (four buffers leave a multiprocessor room for three blocks)
-  const bool few = (long long)T * (Hq / HB) <= 2 * num_multiprocessors();
+  const bool few = blocks <= 2 * num_multiprocessors();
   const size_t smem = (few ? 4 : 2) * sizeof(KeySlice<TC>);
-  auto* kernel = few ? paged_attention_plain_kernel<TC, HB, 4> : paged_attention_plain_kernel<TC, HB, 2>;
+  auto* kernel = few ? paged_attention_plain_kernel<TC, HB, 4, 1> : paged_attention_plain_kernel<TC, HB, 2, 1>;
   if (few) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   NV_RETURN_IF(launch_dep(kernel, grid, dim3(ATT_THREADS), smem, s, qkv, dt, q_stride, kc, vc, block_table, max_blocks,
                           row_entry, positions, scale, window, out, out_dt, Hq, Hkv, D, page));

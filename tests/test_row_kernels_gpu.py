@@ -288,6 +288,25 @@ def test_plain_attention_forms_give_the_same_bits(Hq, Hkv, D, window, dtype):
     assert bool(((full.double() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("n,window", [(1300, 0), (1300, 1100), (2600, 0)])
+def test_plain_attention_of_a_handful_of_rows_over_many_chunks(n, window):
+    """Rows whose chunks of keys a cluster shares out, eight and more of them: the bits of the rows beside many others."""
+    o, Hq, Hkv, D = ops(), 4, 2, 64
+    q = rnd(n, Hq * D, seed=1)
+    kc, vc, bt = paged([n], Hkv, D, 3)
+    pos, entry = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+
+    def run(a, b):
+        out = torch.empty(b - a, Hq * D, device=DEV)
+        o.paged_attention_plain(q[a:b].contiguous(), kc, vc, bt, entry[a:b].contiguous(), pos[a:b].contiguous(), D ** -0.5,
+                                window, out, Hq, Hkv, D)
+        return out
+
+    full = run(0, n)
+    for a, b in ((0, 3), (127, 130), (1023, 1027), (1150, 1153), (n - 1, n)):
+        assert torch.equal(run(a, b), full[a:b])
+
+
 @pytest.mark.parametrize("M,N,K", [(640, 2048 + 5, 68), (64, 20000, 33), (33, 20000, 36), (256, 4864, 128)])
 @pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("swiglu", [False, True])
