@@ -1597,8 +1597,24 @@ def gemm_fast(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, err=No
                         out.stride(0), _epilogue(swiglu, act), n_tile, splits,
                         _p(scratch), _p(None), _p(None), _p(None), _p(None), 0, 0,
                         _p(err.t if err is not None else _global_err().t), _early(), 0, 0,
-                        0, _p(None), 0, *_act_numbers(act), 0, 0, 0, _stream()), f"tc_gemm N={rows_w} K={K}", 2.0 * M * rows_w * K,
+                        0, _p(None), 0, *_act_numbers(act), 0, 0, 0, 1, _stream()), f"tc_gemm N={rows_w} K={K}", 2.0 * M * rows_w * K,
            w.element_size() * rows_w * K + a.element_size() * M * K + out.element_size() * M * N)
+
+
+def gemm_fast_segments(a, w, out, *, err=None, max_ctas: int = 0, tiles_ready=True) -> None:
+    """``out = sum_c a[c * T:(c + 1) * T] @ w[c].T`` on the tensor cores, one sum over all segments: ``a`` [C * T, K] and
+    ``w`` [C, N, K] bfloat16 (a matrix whose columns lie in C blocks of rows), ``out`` [T, N]."""
+    C, N, K = w.shape
+    T = out.shape[0]
+    _need(gemm_fast_usable(a, w, out) and a.shape == (C * T, K) and out.shape[1] == N, "segmented product: operands")
+    L = lib()
+    n_tile = L.nv_tc_gemm_token_tile(T, 0)
+    splits = L.nv_tc_gemm_splits(T, N, C * ((K + 63) // 64) * 64, n_tile, 0, num_sms())
+    scratch = torch.empty((splits, T, N), dtype=torch.float32, device=a.device) if splits > 1 else None
+    _check(L.nv_tc_gemm(_p(a), a.stride(0), T, _p(w), C * N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile,
+                        splits, _p(scratch), _p(None), _p(None), _p(None), _p(None), 0, 0,
+                        _p(err.t if err is not None else _global_err().t), (_early() if tiles_ready else 0), 0, 0, max_ctas,
+                        _p(None), 0, 0.0, 0.0, 0, 0, 0, C, _stream()), f"tc_gemm N={N} K={C * K}", 2.0 * T * N * C * K)
 
 
 def gemm_fast_grouped(a, w, out, align, *, a_rows=None, swiglu=False, err=None, tiles=None, tiles_ready=False,
@@ -1643,7 +1659,7 @@ def gemm_fast_grouped(a, w, out, align, *, a_rows=None, swiglu=False, err=None, 
                             _p(tl.tile_row0), _p(tl.tile_rows), _p(tl.num_tiles), tl.max_tiles,
                             rows_w, _p(err.t if err is not None else _global_err().t),
                             (_early() if tiles_ready else 0), x_sub, x_mod, max_ctas,
-                            _p(counter), align.TK, *_act_numbers(act), 0, 0, 0, _stream()),
+                            _p(counter), align.TK, *_act_numbers(act), 0, 0, 0, 1, _stream()),
            f"tc_gemm_grouped N={rows_w} K={K}")
 
 
@@ -1687,7 +1703,7 @@ def gemm_fast_heads(x, w, out, tiles: HeadTiles, x_step: int, o_step: int, err=N
                             0, tiles.tile_m, 1, _p(None), _p(tiles.tile_expert), _p(tiles.tile_row0),
                             _p(tiles.tile_rows), _p(tiles.num_tiles), tiles.max_tiles, N,
                             _p(err.t if err is not None else _global_err().t), 0, 0, 0, 0, _p(None), T, 0.0, 0.0,
-                            x_step, o_step, x.shape[1], _stream()),
+                            x_step, o_step, x.shape[1], 1, _stream()),
            f"tc_gemm_heads N={N} K={K}", 2.0 * T * H * N * K)
 
 

@@ -78,6 +78,9 @@ struct TcArgs {
   // own: a product per head of rows that hold their heads side by side.  (Columns that a k-step reads beyond the
   // head's own meet the zeros that the weight map fills in beyond K.)
   int x_col_step, o_col_step;
+  // Dense products whose K lies in segments (seg_steps k-steps each): segment c's columns of W's rows stand in rows
+  // c * w_seg_rows further down, those of X's in rows c * x_seg_rows.  Without segments seg_steps is beyond every k-step.
+  int seg_steps, w_seg_rows, x_seg_rows;
   // Tiles handed out by a counter instead of by position (nullptr: CTA b takes tiles b, b + grid, ...): a CTA that
   // starts late, because another kernel still holds its multiprocessor, then takes fewer tiles, and CTAs whose tiles
   // are short take more.  The counter must be 0 at launch; the CTA that draws the last number sets it back to 0.
@@ -357,22 +360,25 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int boxes = (n_act + a.x_box - 1) / a.x_box;
         const uint32_t bytes = a_bytes * (two ? 2 : 1) + (uint32_t)boxes * a.x_box * 128;
         const int wr = t.w_row_base + t.nb * a.w_per_cta;
+        int seg = (t.k_begin + k0) / a.seg_steps, in_seg = t.k_begin + k0 - seg * a.seg_steps;
         for (int k = k0; k < k1; ++k, s_ = (s_ + 1 == a.stages ? 0 : s_ + 1), ph_ ^= (s_ == 0)) {
+          if (in_seg == a.seg_steps) { in_seg = 0; ++seg; }
           const uint32_t st = smem0 + (uint32_t)s_ * stage_bytes, bar = full0 + (uint32_t)s_ * 8;
           if (weights) {
             mbar_wait(&empty_bar[s_], ph_ ^ 1, a.err, 0x7001);
             mbar_expect_tx_a(bar, bytes);
           }
-          const int kc = (t.k_begin + k) * BLOCK_K;
+          const int kc = in_seg++ * BLOCK_K;
           if (weights) {
-            tma_load_2d_a(st, &tm_w, bar, kc, wr);
+            const int row = wr + seg * a.w_seg_rows;
+            tma_load_2d_a(st, &tm_w, bar, kc, row);
             if (two)     // swiglu: the up rows of the same features; dual: the next 128 features
-              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, wr + (a.swiglu ? a.N : TILE_W));
+              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, row + (a.swiglu ? a.N : TILE_W));
           }
           if (tokens)
             for (int b = 0; b < boxes; ++b)
               tma_load_2d_a(st + a_bytes * (two ? 2 : 1) + (uint32_t)b * a.x_box * 128, &tm_x, bar, kc + t.x_col0,
-                            t.x_row0 + b * a.x_box);
+                            t.x_row0 + seg * a.x_seg_rows + b * a.x_box);
         }
       };
       auto advance = [&](int steps) {
@@ -715,7 +721,10 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
                       int splits, float* scratch, const int* tile_expert, const int* tile_row0,
                       const int* tile_rows, const int* num_tiles, int max_tiles, int rows_per_expert, int* err,
                       int early, int x_sub, int x_mod, int max_ctas, int* tile_counter, int m_out,
-                      float act_p0, float act_p1, int x_col_step, int o_col_step, int x_cols, cudaStream_t stream) {
+                      float act_p0, float act_p1, int x_col_step, int o_col_step, int x_cols, int segments,
+                      cudaStream_t stream) {
+  // segments > 1 (dense products): W is [segments, N, K] and X [segments, M_tok, K], and out = sum over the segments of
+  // X[s] W[s]^T, one sum of segments * K terms; `w_rows_total` is segments * N.
   // x_col_step / o_col_step (grouped products only): see TcArgs; x_cols: the columns that a row of X holds then (K is
   // the columns of one block).  Such a product does not split K, and its steps are 8 columns aligned.
   if (!dt_ok(out_dt) || (bias && !dt_ok(bias_dt))) return NV_ERR_BAD_DTYPE;
@@ -732,11 +741,14 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   if (x_mod < 0 || x_sub < 0 || (x_mod && !grouped)) return NV_ERR_BAD_SIZE;
   if (splits > 1 && !scratch) return NV_ERR_BAD_SIZE;
 
+  if (segments < 1 || (segments > 1 && (grouped || w_rows_total != segments * N || swiglu))) return NV_ERR_BAD_SIZE;
+  if ((long long)segments * M_tok > 0x7fffffff) return NV_ERR_BAD_SIZE;
+
   CUtensorMap tm_w, tm_x;
   int rc = get_map(W, w_rows_total, K, K, TILE_W, &tm_w);
   if (rc) return rc;
   const int x_box = n_tile < 64 ? n_tile : 64;
-  rc = get_map(X, M_tok, x_col_step ? x_cols : K, ldx, x_box, &tm_x);
+  rc = get_map(X, (long long)segments * M_tok, x_col_step ? x_cols : K, ldx, x_box, &tm_x);
   if (rc) return rc;
 
   TcArgs a;
@@ -744,7 +756,10 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   a.tile_rows = tile_rows; a.num_tiles = num_tiles; a.err = err; a.ldo = ldo; a.out_dt = out_dt; a.bias_dt = bias_dt;
   a.M_tok = M_tok; a.N = N; a.rows_per_expert = rows_per_expert;
   a.M_out = grouped && m_out > 0 ? m_out : M_tok;
-  a.k_steps_total = (K + BLOCK_K - 1) / BLOCK_K;
+  a.seg_steps = segments > 1 ? (K + BLOCK_K - 1) / BLOCK_K : 0x3fffffff;
+  a.w_seg_rows = N;
+  a.x_seg_rows = M_tok;
+  a.k_steps_total = segments * ((K + BLOCK_K - 1) / BLOCK_K);
   a.splits = splits < 1 ? 1 : splits;
   a.k_steps_per_split = (a.k_steps_total + a.splits - 1) / a.splits;
   a.n_tile = n_tile; a.swiglu = swiglu; a.act = act; a.act_p0 = act_p0; a.act_p1 = act_p1;
