@@ -23,6 +23,8 @@ static inline bool route_groups_ok(int E, int K, int groups, int keep) {
   return groups > 0 && E % groups == 0 && keep >= 1 && keep <= groups && K <= keep * (E / groups);
 }
 
+constexpr int ROUTE_KEYS = 4;      // scores a lane keeps in registers: up to 128 experts
+
 // One warp routes one row: p = softmax(logits) over all E in double, then K rounds of "largest
 // remaining, lowest index on a tie", optional renormalisation of the K weights in double
 // (src/hip_ops.hip:813-841); or the sigmoid rule of RouteRule.  `pr` is E + rule.groups doubles of scratch for this warp.
@@ -74,25 +76,57 @@ __device__ __forceinline__ void route_row(const float* __restrict__ r, int E, in
   }
   double wsum = 0.0;
   double mine = 0.0;  // lane k keeps the k-th weight (K <= 32)
-  for (int k = 0; k < K; ++k) {
-    double best = -1.0e300;                 // (a choice score may be negative; a taken expert is -infinity)
-    int bi = 0x7fffffff;
-    for (int e = lane; e < E; e += 32) {
-      double v = pr[e];
-      if (v > best) { best = v; bi = e; }
-    }
+  if (E <= 32 * ROUTE_KEYS) {
+    // Scores as 64-bit numbers of the same order, in registers: the largest of a warp is then three reductions of one
+    // instruction each (upper half, lower half, lowest index) instead of five rounds of three exchanges.
+    uint64_t key[ROUTE_KEYS];               // 0: not a number, taken, or -infinity
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+    for (int j = 0; j < ROUTE_KEYS; ++j) {
+      const int e = lane + 32 * j;
+      const double v = e < E ? pr[e] : -INFINITY;
+      const uint64_t u = (uint64_t)__double_as_longlong(v);
+      key[j] = v > -1.0e300 ? ((u >> 63) ? ~u : u | (1ull << 63)) : 0;
     }
-    if (bi >= E) { bi = 0; best = 0.0; }    // (no number among the scores: keep every index inside the arrays)
-    if (rule.mode == 1) best = (double)(1.f / (1.f + expf(-r[bi])));     // the weight is the score without the bias
-    if (lane == k) { mine = best; idx_row[k] = bi; }
-    wsum += best;
-    if (lane == 0) pr[bi] = -INFINITY;
-    __syncwarp();
+    for (int k = 0; k < K; ++k) {
+      uint64_t top = key[0];
+      int at = lane;
+#pragma unroll
+      for (int j = 1; j < ROUTE_KEYS; ++j)
+        if (key[j] > top) { top = key[j]; at = lane + 32 * j; }
+      const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(top >> 32));
+      const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(top >> 32) == hi ? (uint32_t)top : 0u);
+      const uint64_t all = (uint64_t)hi << 32 | lo;
+      int bi = (int)__reduce_min_sync(0xffffffffu, all && top == all ? (uint32_t)at : 0x7fffffffu);
+      double best = __longlong_as_double((long long)((all >> 63) ? all & ~(1ull << 63) : ~all));
+      if (bi >= E) { bi = 0; best = 0.0; }  // (no number among the scores: keep every index inside the arrays)
+      if (rule.mode == 1) best = (double)(1.f / (1.f + expf(-r[bi])));   // the weight is the score without the bias
+      if (lane == k) { mine = best; idx_row[k] = bi; }
+      wsum += best;
+#pragma unroll
+      for (int j = 0; j < ROUTE_KEYS; ++j)
+        if (bi == lane + 32 * j) key[j] = 0;
+    }
+  } else {
+    for (int k = 0; k < K; ++k) {
+      double best = -1.0e300;               // (a choice score may be negative; a taken expert is -infinity)
+      int bi = 0x7fffffff;
+      for (int e = lane; e < E; e += 32) {
+        double v = pr[e];
+        if (v > best) { best = v; bi = e; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+      }
+      if (bi >= E) { bi = 0; best = 0.0; }
+      if (rule.mode == 1) best = (double)(1.f / (1.f + expf(-r[bi])));
+      if (lane == k) { mine = best; idx_row[k] = bi; }
+      wsum += best;
+      if (lane == 0) pr[bi] = -INFINITY;
+      __syncwarp();
+    }
   }
   if (lane < K) {
     const float wk = (float)(renorm ? mine / wsum : mine);

@@ -819,6 +819,38 @@ class StaticTiles:
         self.x_rows = (T * K, T)
 
 
+def few_experts_usable(x, w1, w2, T: int, E: int, K: int, C: int, H: int, I: int, groups: int = 0) -> bool:
+    """Whether ``few_experts`` takes a layer (E routed experts of H x I, K a row, C that every row visits) of T rows."""
+    return bool(all(t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0 for t in (x, w1, w2))
+                and w1.is_contiguous() and w2.is_contiguous() and x.stride(0) % 8 == 0
+                and lib().nv_few_experts_usable(T, E, K, C, H, I, groups))
+
+
+def few_experts(x, w1, w2, act, y, logits, K: int, renorm: bool, C: int, gate_logit, idx, score, *, gated=True, fn=None,
+                rule=None) -> None:
+    """A whole mixture of experts for a handful of rows in two launches (few_experts.cu): routing (as ``router_topk``, into
+    ``idx`` and ``score`` [T, K + C]) and first product into ``act`` [T (K + C), I] bfloat16, second product into ``y``
+    [T (K + C), H]; pair (t, k) stands in row t (K + C) + k of both.  ``fn``: as ``act`` of ``gemm_plain``."""
+    _cuda_contig(act, y, idx, score, w1, w2)
+    T, E = logits.shape
+    H, I = x.shape[1], act.shape[1]
+    EC, KT = E + C, K + C
+    groups = rule[3][0] if rule is not None and len(rule) > 3 and rule[3] is not None else 0
+    _need(few_experts_usable(x, w1, w2, T, E, K, C, H, I, groups), "few experts: operands")
+    _need(logits.dtype == torch.float32 and logits.stride(1) == 1 and score.dtype == torch.float32
+          and (gate_logit is None or gate_logit.dtype == torch.float32), "few experts: float32 logits and scores")
+    _i32(idx)
+    _need(x.shape[0] == T and w1.shape == (EC, (2 if gated else 1) * I, H) and w2.shape == (EC, H, I) and act.shape == (T * KT, I)
+          and act.dtype == torch.bfloat16 and y.shape == (T * KT, H) and idx.shape == (T, KT) and score.shape == (T, KT),
+          "few experts: shapes")
+    mode, bias, wscale, n_groups, keep = _route_rule(rule, E)
+    gate_ld = gate_logit.stride(0) if gate_logit is not None else 0
+    for first, (a, w, out, epi) in ((1, (x, w1, act, _epilogue(gated, fn))), (0, (act, w2, y, 0))):
+        _check(lib().nv_few_experts(_p(a), a.stride(0), _p(w), _p(out), dt(out), _p(idx), _p(score), _p(logits), logits.stride(0),
+                                    _p(gate_logit), gate_ld, (1 if renorm else 0), T, E, K, C, out.shape[1], a.shape[1], first, epi,
+                                    *_act_numbers(fn), mode, _p(bias), wscale, n_groups, keep, _stream()), "few_experts")
+
+
 def moe_combine(y, pair_pos, score, shared, gate_logit, out) -> None:
     """``gate_logit``: [T] or a [T, 1] column slice of a wider float32 matrix."""
     _cuda_contig(y, pair_pos, score, shared, out)

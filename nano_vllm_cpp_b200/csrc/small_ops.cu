@@ -190,8 +190,12 @@ __global__ void rowdot_finish_kernel(const float* __restrict__ part, int ranges,
 }
 
 // Routing of a small batch in one launch: top-k of every row, the expert permutation, and the
-// expert-sorted copy of the (bfloat16) activations.  One block of 1024 threads; for batches whose
-// T * (K + C) pairs and rows fit one block's reach (the launcher checks).
+// expert-sorted copy of the (bfloat16) activations.  One block; for batches whose T * (K + C) pairs and rows fit one
+// block's reach (the launcher checks).  What bounds it is latency, trips to L2 above all, since the shared expert's product
+// fills the memory beside it: the choices stay in shared memory for the permutation (written to `idx` besides), and a block
+// has a warp per row, at least four (alone, of 60 experts four: one row 6.6 -> 5.2 us,
+// 64 rows 14.4 -> 12.5; of 64 eight: one row 8.3 -> 5.7, 44 rows 17.1 -> 13.0).
+constexpr int ROUTE_PAIRS = 1024;
 __global__ void __launch_bounds__(1024) moe_route_small_kernel(
     const float* __restrict__ logits, long long ld, int T, int E, int K, int renorm, int C,
     const float* __restrict__ gate_logit, long long gate_ld, int* __restrict__ idx, float* __restrict__ score,
@@ -201,30 +205,31 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(
     const bf16* __restrict__ x, bf16* __restrict__ x_sorted, int H, int n_static, int* __restrict__ zero,
     int n_zero, RouteRule rule) {
   extern __shared__ double rs_smem[];
+  __shared__ int idx_s[ROUTE_PAIRS];
   grid_dep_wait();
   grid_dep_launch();
-  if ((int)threadIdx.x < n_zero) zero[threadIdx.x] = 0;      // (tile counters of the products that follow)
+  for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;      // (tile counters of the products that follow)
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int KT = K + C;
-  for (int t = warp; t < T; t += 32)
-    route_row(logits + (size_t)t * ld, E, K, renorm, rs_smem + (size_t)warp * (E + rule.groups), lane, idx + (size_t)t * KT,
+  for (int t = warp; t < T; t += blockDim.x / 32)
+    route_row(logits + (size_t)t * ld, E, K, renorm, rs_smem + (size_t)warp * (E + rule.groups), lane, idx_s + t * KT,
               score + (size_t)t * KT, C, (C && gate_logit) ? gate_logit + (size_t)t * gate_ld : nullptr, rule);
-  __threadfence_block();
   __syncthreads();
+  for (int i = threadIdx.x; i < T * KT; i += blockDim.x) idx[i] = idx_s[i];
   int* al_s = (int*)(rs_smem + (size_t)32 * (E + rule.groups));
-  align_block(idx, T * KT, KT, E + C, tile_m, counts, offsets, sorted_token, pair_pos, tile_expert, tile_row0,
+  align_block(idx_s, T * KT, KT, E + C, tile_m, counts, offsets, sorted_token, pair_pos, tile_expert, tile_row0,
               tile_rows, num_tiles, err, al_s, 0, nullptr, nullptr, nullptr, nullptr, n_static);
   if (!x_sorted) return;
   __threadfence_block();
   __syncthreads();
   // flat copy of T*KT rows of H/8 16-byte chunks; four loads in flight per thread before the stores
   const int cpr = H / 8, total = T * KT * cpr;
-  for (int base = threadIdx.x; base < total; base += 4 * 1024) {
+  for (int base = threadIdx.x; base < total; base += 4 * blockDim.x) {
     uint4 v[4];
     int idx4[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      idx4[u] = base + u * 1024;
+      idx4[u] = base + u * blockDim.x;
       if (idx4[u] < total) {
         const int p = idx4[u] / cpr, c = idx4[u] - p * cpr;
         v[u] = *((const uint4*)(x + (size_t)sorted_token[p] * H) + c);
@@ -303,7 +308,7 @@ NV_API int nv_rowdot(const float* a, long long lda, const void* w, int w_dt, flo
 // Largest batch the fused routing kernel takes: rows and pairs one block can walk in a few microseconds.
 NV_API int nv_moe_route_small_usable(int T, int E, int K, int C, int H, int groups) {
   const size_t smem = (size_t)32 * (E + groups) * sizeof(double) + (size_t)4 * (E + C) * sizeof(int);
-  return T <= 64 && T * (K + C) <= 1024 && smem <= 48 * 1024 && H % 8 == 0 && K <= 32 && C <= 32;
+  return T <= 64 && T * (K + C) <= ROUTE_PAIRS && smem <= 48 * 1024 && H % 8 == 0 && K <= 32 && C <= 32;
 }
 
 NV_API int nv_moe_route_small(const float* logits, long long ld, int T, int E, int K, int renorm, int C,
@@ -318,7 +323,8 @@ NV_API int nv_moe_route_small(const float* logits, long long ld, int T, int E, i
   if (n_static != 0 && n_static != C) return NV_ERR_UNSUPPORTED;
   if (T == 0) return NV_OK;
   const size_t smem = (size_t)32 * (E + groups) * sizeof(double) + (size_t)4 * (E + C) * sizeof(int);
-  NV_RETURN_IF(launch_dep(moe_route_small_kernel, dim3(1), dim3(1024), smem, s, logits, ld, T, E, K, renorm, C,
+  const unsigned threads = x ? 1024 : 32 * (T < 4 ? 4 : T < 32 ? T : 32);
+  NV_RETURN_IF(launch_dep(moe_route_small_kernel, dim3(1), dim3(threads), smem, s, logits, ld, T, E, K, renorm, C,
                           gate_logit, gate_ld, idx, score, tile_m, counts, offsets, sorted_token, pair_pos, tile_expert,
                           tile_row0, tile_rows, num_tiles, err, (const bf16*)x, (bf16*)x_sorted, H, n_static, zero,
                           n_zero, RouteRule{mode, choice_bias, weight_scale, groups, keep}));

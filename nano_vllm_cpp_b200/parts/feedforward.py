@@ -19,6 +19,8 @@ SIDE_GRID_SHARE = 0.88
 # sum fewer tiles than there are multiprocessors, it is split again and the second kernel that adds the parts costs what was
 # gained (508 rows of the A2.7B sizes, eight layers: 2.61 -> 2.67 ms; 2,048 rows, 24 layers: 13.85 -> 13.62).
 ONE_SUM_MIN_ROWS = 1536
+# Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, go without a permutation.
+FEW_PAIRS = 16
 # Permutation buffers are kept per batch size; beyond this many sizes the oldest set is dropped.
 MAX_ALIGNMENTS = 16
 
@@ -176,6 +178,7 @@ class SparseMoeSwiGLU(FeedForward):
         self._captured = {}
         self._static = {}
         self._static_kept = set()
+        self._pair_rows = {}            # (rows of a step, device) -> the numbers of its pairs (a handful of small steps)
         self.router_and_gate = None
         self.last_alignment = None      # the permutation buffers of the latest forward (for statistics)
 
@@ -300,6 +303,10 @@ class SparseMoeSwiGLU(FeedForward):
             logits = small_linear(ctx, h32, self.router)
         fast = (ctx.fast_kernels and h.dtype == torch.bfloat16 and self.w_gate_up.dtype == torch.bfloat16
                 and self.w_down.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0)
+        if (fast and T * KT <= FEW_PAIRS and (C or not self.shared_inter)
+                and ops.few_experts_usable(h, self.w_gate_up, self.w_down, T, self.E, self.K, C, self.hidden, self.inter,
+                                           self.groups[0] if self.groups else 0)):
+            return self._forward_few(h, logits, gate_logit)
         many = fast and C and T >= 256
         # (with many rows the shared expert is one expert of the permutation, however many chunks its products have)
         V = 1 if many and T >= ONE_SUM_MIN_ROWS else C
@@ -344,6 +351,24 @@ class SparseMoeSwiGLU(FeedForward):
         # the combination (src/hip_ops.hip:873-892) is left to whoever takes the branch: the next norm sums it
         return RowMix(y, al.pair_pos[:T * KT].view(T, KT), score, shared, gate_logit if shared is not None else None)
 
+
+    def _forward_few(self, h, logits, gate_logit):
+        """A handful of pairs: no permutation, two launches (``ops.few_experts``)."""
+        ctx, T, KT, dev = self.ctx, h.shape[0], self.K + self.virtual, h.device
+        idx = torch.empty((T, KT), dtype=torch.int32, device=dev)
+        score = torch.empty((T, KT), dtype=torch.float32, device=dev)
+        act = torch.empty((T * KT, self.inter), dtype=ctx.act_dtype, device=dev)
+        y = torch.empty((T * KT, self.hidden), dtype=torch.float32, device=dev)
+        ops.few_experts(h, self.w_gate_up, self.w_down, act, y, logits, self.K, self.renorm, self.virtual, gate_logit, idx, score,
+                        gated=self.gated, fn=self.expert_act, rule=self.rule)
+        self.last_alignment = _Choices(idx, self.E + self.virtual)
+        key = (T, dev)
+        rows = self._pair_rows.get(key)                    # pair (t, k) stands in row t KT + k
+        if rows is None:
+            rows = torch.arange(T * KT, dtype=torch.int32, device=dev).view(T, KT)
+            if not torch.cuda.is_current_stream_capturing():      # (memory of a capture is the capture's)
+                self._pair_rows[key] = rows
+        return RowMix(y, rows, score, None, None)
 
     def _forward_beside(self, h, logits, gate_logit, idx, score, al, many=False):
         """The shared expert's chunks need no routing, so their two products run on a second stream beside the
@@ -407,6 +432,17 @@ class SparseMoeSwiGLU(FeedForward):
         ops.gemm_fast_grouped(act[:T * K], self.w_down, y, al, err=ctx.err, tiles_ready=True, counter=c1)
         main.wait_event(join)
         return RowMix(y, al.pair_pos[:T * (K + V)].view(T, K + V), score, None, None)
+
+
+class _Choices:
+    """What a step without a permutation has in its place for statistics: how many pairs chose each expert."""
+
+    def __init__(self, idx, experts):
+        self.idx, self.experts = idx, experts
+
+    @property
+    def counts(self):
+        return torch.bincount(self.idx.flatten(), minlength=self.experts)
 
 
 def _cat(ts):
