@@ -11,7 +11,9 @@
 // own only) and the rows there from the start.  The shared expert's units come first: the first of them is asked for before the
 // kernel in front has finished, and a seventeenth warp routes the rows meanwhile, in every block by itself, so that no
 // block waits for another.
-// Measured (@@FEW@@).
+// Measured inside a decode step of one row (60 experts of 1,408 x 2,048, four chosen, four chunks of the shared one): routing
+// and experts 38 -> 28 us a layer, the step 1.98 -> 1.71 ms.  With the pieces in registers, two rounds of them, instead of
+// the ring, and the rows read from L2 at every unit, 36 us: a unit's rows were waited for.
 #include "common.cuh"
 #include "moe_route.cuh"
 
@@ -210,9 +212,17 @@ __global__ void __launch_bounds__((FX_WARPS + 1) * 32, 1) few_experts_kernel(con
   };
   while (asked < a.stages - 1 && iu < shared_units) ask();        // (no choice of the routing is needed for these)
   grid_dep_wait();                                    // now the rows, and with them the rest
-  for (int i = threadIdx.x; i < x_rows * (a.K_in / 8); i += FX_THREADS) {
-    const int r = i / (a.K_in / 8);
-    xs[i] = *((const uint4*)(a.x + r * a.ldx) + (i - r * (a.K_in / 8)));
+  const int per = a.K_in / 8, x_all = x_rows * per;
+  for (int i0 = threadIdx.x; i0 < x_all; i0 += 4 * FX_THREADS) {
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = min(i0 + j * FX_THREADS, x_all - 1), r = i / per;
+      v[j] = *((const uint4*)(a.x + r * a.ldx) + (i - r * per));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j * FX_THREADS < x_all) xs[i0 + j * FX_THREADS] = v[j];
   }
   asm volatile("bar.sync 1, %0;" ::"n"(FX_THREADS) : "memory");
   while (asked < a.stages - 1) ask();

@@ -19,8 +19,13 @@ SIDE_GRID_SHARE = 0.88
 # sum fewer tiles than there are multiprocessors, it is split again and the second kernel that adds the parts costs what was
 # gained (508 rows of the A2.7B sizes, eight layers: 2.61 -> 2.67 ms; 2,048 rows, 24 layers: 13.85 -> 13.62).
 ONE_SUM_MIN_ROWS = 1536
-# Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, go without a permutation.
+# Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, go without a permutation, if the
+# experts are no larger than FEW_EXPERT_SIZE (hidden x inner).  Measured per pass of eight steps, with and without: A2.7B sizes
+# (eight pairs a row), eight layers, one row 5.07 and 5.83 ms, two 6.22 and 6.51, three 7.26 and 7.06, four 8.19 and 7.50
+# (pairs that share an expert each read it); experts of 3,584 x 2,560, sixteen pairs a row, one row 6.46 and 6.42: their
+# products are bound by memory either way.
 FEW_PAIRS = 16
+FEW_EXPERT_SIZE = 6 << 20
 # Permutation buffers are kept per batch size; beyond this many sizes the oldest set is dropped.
 MAX_ALIGNMENTS = 16
 
@@ -303,7 +308,7 @@ class SparseMoeSwiGLU(FeedForward):
             logits = small_linear(ctx, h32, self.router)
         fast = (ctx.fast_kernels and h.dtype == torch.bfloat16 and self.w_gate_up.dtype == torch.bfloat16
                 and self.w_down.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0)
-        if (fast and T * KT <= FEW_PAIRS and (C or not self.shared_inter)
+        if (fast and T * KT <= FEW_PAIRS and self.hidden * self.inter <= FEW_EXPERT_SIZE and (C or not self.shared_inter)
                 and ops.few_experts_usable(h, self.w_gate_up, self.w_down, T, self.E, self.K, C, self.hidden, self.inter,
                                            self.groups[0] if self.groups else 0)):
             return self._forward_few(h, logits, gate_logit)
