@@ -1633,6 +1633,28 @@ def gemm_fast(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, err=No
            w.element_size() * rows_w * K + a.element_size() * M * K + out.element_size() * M * N)
 
 
+def gemm_terms_usable(a, w, out) -> bool:
+    """Whether ``gemm_terms`` takes these operands: float32 rows, a bfloat16 matrix, float32 results."""
+    return bool(a.dtype == torch.float32 and a.stride(-1) == 1 and a.shape[1] % 8 == 0 and _tma_ok(w) and w.is_contiguous()
+                and w.dim() == 2 and out.dtype == torch.float32 and out.stride(-1) == 1)
+
+
+def gemm_terms(a, w, out, *, err=None) -> None:
+    """``out = a @ w.T`` for float32 ``a`` [T, K] and bfloat16 ``w`` [N, K] on the tensor cores: a value of ``a`` is the sum of
+    three bfloat16 terms, exactly, products of bfloat16 values are exact in float32, and the terms' products are added from the
+    smallest on, in one accumulator."""
+    T, K = a.shape
+    N = w.shape[0]
+    _need(gemm_terms_usable(a, w, out) and w.shape[1] == K and out.shape == (T, N), "product of terms: operands")
+    L = lib()
+    terms = torch.empty((3 * T, K), dtype=torch.bfloat16, device=a.device)
+    _check(L.nv_split_terms(_p(a), a.stride(0), _p(terms), T, K, _stream()), "split_terms")
+    n_tile = L.nv_tc_gemm_token_tile(T, 0)
+    _check(L.nv_tc_gemm(_p(terms), K, T, _p(w), N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile, 1, _p(None),
+                        _p(None), _p(None), _p(None), _p(None), 0, 0, _p(err.t if err is not None else _global_err().t), _early(),
+                        0, 0, 0, _p(None), 0, 0.0, 0.0, 0, 0, 0, -3, _stream()), f"tc_gemm N={N} K={3 * K}", 6.0 * T * N * K)
+
+
 def gemm_fast_segments(a, w, out, *, err=None, max_ctas: int = 0, tiles_ready=True) -> None:
     """``out = sum_c a[c * T:(c + 1) * T] @ w[c].T`` on the tensor cores, one sum over all segments: ``a`` [C * T, K] and
     ``w`` [C, N, K] bfloat16 (a matrix whose columns lie in C blocks of rows), ``out`` [T, N]."""

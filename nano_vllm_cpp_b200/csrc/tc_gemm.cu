@@ -589,6 +589,25 @@ __global__ void tc_gemm_finish_grouped_kernel(const float* __restrict__ partial,
   }
 }
 
+// A float32 value as three bfloat16 terms that add up to it exactly (eight bits each, cut off and not rounded, so that no
+// term is larger than the value; what is not finite is its first term): out[0] = the last bits, out[2] = the first, [3][T][K].
+__global__ void split_terms_kernel(const float* __restrict__ x, long long ldx, bf16* __restrict__ out, int T, int K) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const long long n = (long long)T * K, i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long t = i / K;
+  const float v = x[t * ldx + (i - t * K)];
+  const uint32_t u = __float_as_uint(v);
+  const bool number = v == v, finite = (u & 0x7f800000u) != 0x7f800000u;
+  const float hi = number ? __uint_as_float(u & 0xffff0000u) : v;
+  const float rest = finite ? v - hi : 0.f;
+  const float mid = __uint_as_float(__float_as_uint(rest) & 0xffff0000u);
+  out[i] = __float2bfloat16_rn(rest - mid);
+  out[n + i] = __float2bfloat16_rn(mid);
+  out[2 * n + i] = __float2bfloat16_rn(hi);
+}
+
 // out[r, :] = src[rows[r], :] for bf16 rows (the expert-sorted copy of the activations)
 __global__ void permute_rows_bf16_kernel(const bf16* __restrict__ src, const int* __restrict__ rows,
                                          bf16* __restrict__ dst, int H) {
@@ -724,7 +743,8 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
                       float act_p0, float act_p1, int x_col_step, int o_col_step, int x_cols, int segments,
                       cudaStream_t stream) {
   // segments > 1 (dense products): W is [segments, N, K] and X [segments, M_tok, K], and out = sum over the segments of
-  // X[s] W[s]^T, one sum of segments * K terms; `w_rows_total` is segments * N.
+  // X[s] W[s]^T, one sum of segments * K terms; `w_rows_total` is segments * N.  segments < -1: -segments of them over one
+  // W [N, K].
   // x_col_step / o_col_step (grouped products only): see TcArgs; x_cols: the columns that a row of X holds then (K is
   // the columns of one block).  Such a product does not split K, and its steps are 8 columns aligned.
   if (!dt_ok(out_dt) || (bias && !dt_ok(bias_dt))) return NV_ERR_BAD_DTYPE;
@@ -741,7 +761,9 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   if (x_mod < 0 || x_sub < 0 || (x_mod && !grouped)) return NV_ERR_BAD_SIZE;
   if (splits > 1 && !scratch) return NV_ERR_BAD_SIZE;
 
-  if (segments < 1 || (segments > 1 && (grouped || w_rows_total != segments * N || swiglu))) return NV_ERR_BAD_SIZE;
+  const bool one_w = segments < 0;
+  if (one_w) segments = -segments;
+  if (segments < 1 || (segments > 1 && (grouped || w_rows_total != (one_w ? 1 : segments) * N || swiglu))) return NV_ERR_BAD_SIZE;
   if ((long long)segments * M_tok > 0x7fffffff) return NV_ERR_BAD_SIZE;
 
   CUtensorMap tm_w, tm_x;
@@ -757,7 +779,7 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   a.M_tok = M_tok; a.N = N; a.rows_per_expert = rows_per_expert;
   a.M_out = grouped && m_out > 0 ? m_out : M_tok;
   a.seg_steps = segments > 1 ? (K + BLOCK_K - 1) / BLOCK_K : 0x3fffffff;
-  a.w_seg_rows = N;
+  a.w_seg_rows = one_w ? 0 : N;
   a.x_seg_rows = M_tok;
   a.k_steps_total = segments * ((K + BLOCK_K - 1) / BLOCK_K);
   a.splits = splits < 1 ? 1 : splits;
@@ -863,6 +885,14 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
                               out_dt, ldo, act_p0, act_p1));
     }
   }
+  NV_RETURN_LAST();
+}
+
+NV_API int nv_split_terms(const float* x, long long ldx, void* out, int T, int K, cudaStream_t stream) {
+  if (T <= 0 || K <= 0) return NV_OK;
+  const long long n = (long long)T * K;
+  if ((n + 255) / 256 > 0x7fffffff) return NV_ERR_BAD_SIZE;
+  NV_RETURN_IF(launch_dep(split_terms_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, x, ldx, (bf16*)out, T, K));
   NV_RETURN_LAST();
 }
 

@@ -1,6 +1,6 @@
 """Matrix products of the parts: picks the kernel for a product's types and sizes.
 
-float32 anywhere in the operands -> the plain FFMA kernel (true 32-bit, no tensor cores).
+float32 anywhere in the operands -> the plain FFMA kernel (true 32-bit, no tensor cores), but see TERMS_MIN_ROWS.
 bfloat16 x bfloat16 -> the tcgen05 kernel when its size rules hold, else the plain kernel.
 """
 from __future__ import annotations
@@ -14,6 +14,12 @@ from ..csrc import ops
 # 4.3 TB/s on a 622 MB output head, 2.5 against 3.5 TB/s on a 25 MB projection).
 SKINNY_ROWS = ops.SKINNY_MAX_ROWS
 SKINNY_MAX_BYTES = 128 << 20
+# float32 rows times a bfloat16 matrix with a short K (the second half of a low-rank projection), prompts of a bfloat16 run:
+# three bfloat16 terms on the tensor cores, from so many rows on and up to so long a K.  (6,737 rows, 64 -> 2,048:
+# 97 us in FFMAs, 4 + 22 so; relative error against float64 7.9e-8, 1.06e-7 in FFMAs.  The accumulator of the tensor cores loses more with every
+# step: at K = 128 1.26e-7 against 1.11e-7, at 512 4.8e-7 against 1.6e-7.)
+TERMS_MIN_ROWS = 256
+TERMS_MAX_K = 64
 
 
 def linear(ctx, a, w, out_dtype, *, bias=None, a_rows=None, swiglu=False, M=None, out=None, act=None):
@@ -39,6 +45,9 @@ def linear(ctx, a, w, out_dtype, *, bias=None, a_rows=None, swiglu=False, M=None
         return out
     if ctx.fast_kernels and ops.gemm_fast_usable(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu):
         ops.gemm_fast(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu, M=M, err=ctx.err, act=act)
+    elif (ctx.fast_kernels and ctx.act_dtype == torch.bfloat16 and M >= TERMS_MIN_ROWS and a.shape[-1] <= TERMS_MAX_K
+          and M == a.shape[0] and bias is None and a_rows is None and act is None and not swiglu and ops.gemm_terms_usable(a, w, out)):
+        ops.gemm_terms(a, w, out, err=ctx.err)
     else:
         ops.gemm_plain(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu, M=M, act=act)
     return out

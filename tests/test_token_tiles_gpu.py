@@ -83,3 +83,26 @@ def test_one_sum_over_segments(T, N, K, C):
     o.gemm_fast_segments(a, w, out, err=err)
     err.check("segments")
     held(out, sum(a[c * T:(c + 1) * T].double() @ w[c].double().T for c in range(C)), C * K, "segments")
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 16, 8), (256, 2048, 64), (300, 200, 64), (1500, 1024, 40)])
+def test_product_of_three_terms(T, N, K):
+    """float32 rows on the tensor cores: no further from float64 than a chain of FFMAs, and what is not finite stays so."""
+    o = ops()
+    a = torch.randn(T, 3 * K, generator=torch.Generator().manual_seed(1)).to(DEV)[:, K:2 * K]
+    a[0, 0] = 3e38
+    w = rnd(N, K, seed=2, scale=0.02)
+    out, plain, err = torch.empty(T, N, device=DEV), torch.empty(T, N, device=DEV), o.ErrorFlag(DEV)
+    o.gemm_terms(a, w, out, err=err)
+    err.check("terms")
+    o.gemm_plain(a, w, plain)
+    want = a.double() @ w.double().T
+    off = [float(((x.double() - want)[1:].norm() / want[1:].norm()) if T > 1 else 0.0) for x in (out, plain)]
+    assert off[0] <= max(1.1 * off[1], 1.5 * 2.0 ** -24) and bool(((out[0].double() - want[0]).abs() <= 2.0 ** -21 * want[0].abs().max()).all())
+    a[0, :4] = torch.tensor([float("inf"), -1.0, 0.0, 1e-41])
+    w[:, 0] = 1.0
+    o.gemm_terms(a, w, out, err=err)
+    assert bool((out[0] == float("inf")).all()) and bool(out[1:].isfinite().all())
+    a[0, 1] = float("nan")
+    o.gemm_terms(a, w, out, err=err)
+    assert bool(out[0].isnan().all()) and bool(out[1:].isfinite().all())
