@@ -80,12 +80,66 @@ struct DecArgs {
   float cap_in;           // MOD 2: scale / softcap
 };
 
+constexpr int MAX_SPLITS = 32;          // one lane each where they are added up
+constexpr int FEW_SPLITS = 8;
+
+// The splits of a head added up in their order: m and l of split s at part_ml[2 s], its elements at part_o[s D].  One load after
+// the other from the second-level cache was most of the time of this (eight rows of 16 heads of 256, 17 splits: 20 us).
+//
+// Up to eight splits: a thread asks for the weights and its element of every split at once and needs nobody else.
+__device__ __forceinline__ float few_splits_sum(const float* part_ml, const float* part_o, int splits, int D, bool has_sink, float sink,
+                                                float gate) {
+  float2 ml[FEW_SPLITS];
+  float v[FEW_SPLITS];
+#pragma unroll
+  for (int i = 0; i < FEW_SPLITS; ++i) {
+    ml[i] = i < splits ? __ldcg((const float2*)part_ml + i) : make_float2(-1e30f, 0.f);
+    v[i] = i < splits ? __ldcg(part_o + (size_t)i * D) : 0.f;
+  }
+  float mm = ml[0].x, ll = 0.f, o = 0.f;
+#pragma unroll
+  for (int i = 1; i < FEW_SPLITS; ++i) mm = fmaxf(mm, ml[i].x);
+#pragma unroll
+  for (int i = 0; i < FEW_SPLITS; ++i)
+    if (i < splits) {
+      const float sc = __expf(ml[i].x - mm);
+      ll = fmaf(ml[i].y, sc, ll);
+      o = fmaf(v[i], sc, o);
+    }
+  if (has_sink) ll += __expf(sink - mm);
+  return o * ((ll > 0.f ? 1.f / ll : 0.f) * gate);
+}
+// More: one warp works out what the splits weigh in the output, into w[splits] ...
+__device__ __forceinline__ void split_weights(const float* part_ml, int splits, int lane, bool has_sink, float sink, float gate,
+                                              float* w) {
+  const float2 ml = lane < splits ? __ldcg((const float2*)part_ml + lane) : make_float2(-1e30f, 0.f);
+  const float mm = warp_max(ml.x);
+  const float sc = lane < splits ? __expf(ml.x - mm) : 0.f;
+  float ll = warp_sum(ml.y * sc);
+  if (has_sink) ll += __expf(sink - mm);
+  if (lane < splits) w[lane] = sc * ((ll > 0.f ? 1.f / ll : 0.f) * gate);
+}
+// ... and a thread adds its element up, eight loads at a time.
+__device__ __forceinline__ float split_sum(const float* part_o, const float* w, int splits, int D) {
+  float o = 0.f;
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = s0 + i < splits ? __ldcg(part_o + (size_t)(s0 + i) * D) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (s0 + i < splits) o = fmaf(v[i], w[s0 + i], o);
+  }
+  return o;
+}
+
 // Called by every thread of a block once the block has written its split's partial results for the query heads
 // h0 .. h0 + nh - 1 of row r (batch row t): the block that arrives last for this (row, group of heads) adds the splits
 // up, in split order and with the arithmetic of attention_decode_merge_kernel, and writes the result; the others
 // leave.  That saves the merge kernel's launch, which stands between the attention and the output projection of
 // every layer.  The count goes back to zero for the next launch.
-__device__ __forceinline__ void merge_when_last(const DecArgs& a, int r, int t, int h0, int nh, int D) {
+// `w_s`: [nh][MAX_SPLITS] floats of shared memory that are free now (some of its own would cost a multiprocessor its third block).
+__device__ __forceinline__ void merge_when_last(const DecArgs& a, int r, int t, int h0, int nh, int D, float* w_s) {
   __shared__ int last_s;
   __threadfence();                      // this block's partial results are visible to every block ...
   __syncthreads();
@@ -98,19 +152,24 @@ __device__ __forceinline__ void merge_when_last(const DecArgs& a, int r, int t, 
   __syncthreads();
   if (!last_s) return;
   __threadfence();
+  if (a.splits <= FEW_SPLITS) {
+    for (int i = threadIdx.x; i < nh * D; i += blockDim.x) {
+      const int h = h0 + i / D, d = i % D;
+      const size_t pi = ((size_t)r * a.Hq + h) * a.splits;
+      st_dt(a.out, a.out_dt, ((size_t)t * a.Hq + h) * D + d,
+            few_splits_sum(a.part_ml + pi * 2, a.part_o + pi * D + d, a.splits, D, a.has_sink, a.sink, head_gate_of(a.gate, t, h)));
+    }
+    return;
+  }
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  for (int i = warp; i < nh; i += blockDim.x / 32)
+    split_weights(a.part_ml + ((size_t)r * a.Hq + h0 + i) * a.splits * 2, a.splits, lane, a.has_sink, a.sink,
+                  head_gate_of(a.gate, t, h0 + i), w_s + i * MAX_SPLITS);
+  __syncthreads();
   for (int i = threadIdx.x; i < nh * D; i += blockDim.x) {
     const int h = h0 + i / D, d = i % D;
-    const size_t pi = ((size_t)r * a.Hq + h) * a.splits;
-    float mm = -1e30f;
-    for (int s = 0; s < a.splits; ++s) mm = fmaxf(mm, __ldcg(a.part_ml + (pi + s) * 2));
-    float ll = 0.f, o = 0.f;
-    for (int s = 0; s < a.splits; ++s) {
-      const float sc = __expf(__ldcg(a.part_ml + (pi + s) * 2) - mm);
-      ll = fmaf(__ldcg(a.part_ml + (pi + s) * 2 + 1), sc, ll);
-      o = fmaf(__ldcg(a.part_o + (pi + s) * D + d), sc, o);
-    }
-    if (a.has_sink) ll += __expf(a.sink - mm);
-    st_dt(a.out, a.out_dt, ((size_t)t * a.Hq + h) * D + d, o * ((ll > 0.f ? 1.f / ll : 0.f) * head_gate_of(a.gate, t, h)));
+    st_dt(a.out, a.out_dt, ((size_t)t * a.Hq + h) * D + d,
+          split_sum(a.part_o + ((size_t)r * a.Hq + h) * a.splits * D + d, w_s + i / D * MAX_SPLITS, a.splits, D));
   }
 }
 
@@ -330,7 +389,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32) attention_decode_kernel(DecA
       }
     }
   }
-  if (a.splits > 1 && a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, D);
+  if (a.splits > 1 && a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, D, (float*)dec_smem);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -407,7 +466,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
       a.part_o[pi * a.D + i % a.D] = 0.f;
       if (i % a.D == 0) { a.part_ml[pi * 2] = -1e30f; a.part_ml[pi * 2 + 1] = 0.f; }
     }
-    if (a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, a.D);
+    if (a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, a.D, (float*)dec_smem);
     return;
   }
   const uint32_t box_bytes = (uint32_t)a.page * 128;           // one box: `page` keys x 64 elements
@@ -677,7 +736,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
       }
     }
   }
-  if (a.splits > 1 && a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, a.D);
+  if (a.splits > 1 && a.split_count) merge_when_last(a, r, t, kvh * G + g0, ng, a.D, (float*)dec_smem);
 }
 
 // Combines the splits of one (row, head) in split order.
@@ -689,17 +748,17 @@ __global__ void attention_decode_merge_kernel(const float* __restrict__ part_o, 
   const size_t pi = ((size_t)r * Hq + h) * splits;
   grid_dep_wait();
   grid_dep_launch();
-  float mm = -1e30f;
-  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, part_ml[(pi + s) * 2]);
-  float ll = 0.f;
-  for (int s = 0; s < splits; ++s) ll = fmaf(part_ml[(pi + s) * 2 + 1], __expf(part_ml[(pi + s) * 2] - mm), ll);
-  if (has_sink) ll += __expf(sink - mm);
-  const float inv = (ll > 0.f ? 1.f / ll : 0.f) * head_gate_of(gate, t, h);
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float o = 0.f;
-    for (int s = 0; s < splits; ++s) o = fmaf(part_o[(pi + s) * D + d], __expf(part_ml[(pi + s) * 2] - mm), o);
-    st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d, o * inv);
+  if (splits <= FEW_SPLITS) {
+    for (int d = threadIdx.x; d < D; d += blockDim.x)
+      st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d,
+            few_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
+    return;
   }
+  __shared__ float w_s[MAX_SPLITS];
+  if (threadIdx.x < 32) split_weights(part_ml + pi * 2, splits, threadIdx.x, has_sink, sink, head_gate_of(gate, t, h), w_s);
+  __syncthreads();
+  for (int d = threadIdx.x; d < D; d += blockDim.x)
+    st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d, split_sum(part_o + pi * D + d, w_s, splits, D));
 }
 
 template <typename TC, int CPL, int GB>
@@ -787,12 +846,15 @@ NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context
   const int G = Hq / Hkv;
   const long long slots = 3LL * num_sms;
   const long long blocks = (long long)rows * Hkv * ((G + 15) / 16);
-  int most = (max_context + 255) / 256;          // at least 256 keys per split
-  if (most > 32) most = 32;
+  // at least 256 keys per split; 128 while all splits run at once (one row of 2,064 keys, 16 heads: 18.6 and 16.4 us; with
+  // several waves of them 8 rows 39 and 49)
+  int most = (max_context + 127) / 128;
+  if (most > MAX_SPLITS) most = MAX_SPLITS;
   int best = 1;
   double best_score = -1.0;
   for (int s = 1; s <= most; ++s) {
     const long long ctas = blocks * s;
+    if (s > 1 && s > (max_context + 255) / 256 && ctas > slots) break;
     const long long waves = (ctas + slots - 1) / slots;
     const double score = (double)ctas / ((double)waves * (double)slots) - 0.001 * s;
     if (score > best_score + 1e-9) { best_score = score; best = s; }
@@ -828,7 +890,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   if (((uintptr_t)kc & 15) || ((uintptr_t)vc & 15)) return NV_ERR_UNSUPPORTED;
   if (R == 0) return NV_OK;
   if (splits < 1) splits = 1;
-  if (splits > 1 && !scratch) return NV_ERR_BAD_SIZE;
+  if (splits > MAX_SPLITS || (splits > 1 && !scratch)) return NV_ERR_BAD_SIZE;
   DecArgs a;
   a.qkv = qkv; a.kc = kc; a.vc = vc; a.block_table = block_table; a.row_entry = row_entry; a.positions = positions;
   a.rows = rows; a.out = out; a.scale = scale; a.q_dt = q_dt; a.out_dt = out_dt; a.q_stride = q_stride;
@@ -849,12 +911,13 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // the last blocks' sums lengthen the kernel's tail by more than the second kernel's launch costs (measured per
   // decode step: batch 1 507 -> 511 tokens/s, batch 8 2,209 -> 2,212, batch 64 6,252 -> 6,192).
   a.split_count = (split_count && (long long)R * Hq <= split_count_len && R * Hq <= 256) ? split_count : nullptr;
-  // ... and only while the last block's sum is short: a thread of it adds its outputs one after the other, each a chain
-  // of loads from the second-level cache, so with sixteen heads of 256 elements on one kv head (4,096 outputs for 160
-  // threads) that one block ran for 50 of the kernel's 64 us; the second kernel has a block per row and head.
+  // ... and only while the last block's sum is short: its 160 threads add the block's outputs up one after the other, each
+  // with loads from the second-level cache (one row of 4,096 keys, 28 heads of 128 on 4: 33 us so and 24 with the second kernel,
+  // which has a block per row and head; 8 rows of 512, 16 heads on 4: 20.5 and 17.4; one row of 2,064, 16 heads on 16: 18.6
+  // and 21.5).
   {
     const int heads_per_block = Hq / Hkv < 16 ? Hq / Hkv : 16;
-    if ((long long)heads_per_block * D > 1024) a.split_count = nullptr;
+    if ((long long)heads_per_block * D > 256) a.split_count = nullptr;
   }
   a.stages = stages;
   const size_t smem = (size_t)stages * 2 * page * D * esize;
