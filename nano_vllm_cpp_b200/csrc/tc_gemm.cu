@@ -360,9 +360,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int boxes = (n_act + a.x_box - 1) / a.x_box;
         const uint32_t bytes = a_bytes * (two ? 2 : 1) + (uint32_t)boxes * a.x_box * 128;
         const int wr = t.w_row_base + t.nb * a.w_per_cta;
-        int seg = (t.k_begin + k0) / a.seg_steps, in_seg = t.k_begin + k0 - seg * a.seg_steps;
+        int in_seg = t.k_begin + k0, wrow = wr, xrow = t.x_row0;
+        if (in_seg >= a.seg_steps) {               // (a division here at every product's tile cost decoding half a percent)
+          const int seg = in_seg / a.seg_steps;
+          in_seg -= seg * a.seg_steps;
+          wrow += seg * a.w_seg_rows;
+          xrow += seg * a.x_seg_rows;
+        }
         for (int k = k0; k < k1; ++k, s_ = (s_ + 1 == a.stages ? 0 : s_ + 1), ph_ ^= (s_ == 0)) {
-          if (in_seg == a.seg_steps) { in_seg = 0; ++seg; }
+          if (in_seg == a.seg_steps) { in_seg = 0; wrow += a.w_seg_rows; xrow += a.x_seg_rows; }
           const uint32_t st = smem0 + (uint32_t)s_ * stage_bytes, bar = full0 + (uint32_t)s_ * 8;
           if (weights) {
             mbar_wait(&empty_bar[s_], ph_ ^ 1, a.err, 0x7001);
@@ -370,15 +376,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           }
           const int kc = in_seg++ * BLOCK_K;
           if (weights) {
-            const int row = wr + seg * a.w_seg_rows;
-            tma_load_2d_a(st, &tm_w, bar, kc, row);
+            tma_load_2d_a(st, &tm_w, bar, kc, wrow);
             if (two)     // swiglu: the up rows of the same features; dual: the next 128 features
-              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, row + (a.swiglu ? a.N : TILE_W));
+              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, wrow + (a.swiglu ? a.N : TILE_W));
           }
           if (tokens)
             for (int b = 0; b < boxes; ++b)
               tma_load_2d_a(st + a_bytes * (two ? 2 : 1) + (uint32_t)b * a.x_box * 128, &tm_x, bar, kc + t.x_col0,
-                            t.x_row0 + seg * a.x_seg_rows + b * a.x_box);
+                            xrow + b * a.x_box);
         }
       };
       auto advance = [&](int steps) {
