@@ -13,7 +13,7 @@
 // so all eight products with the memory are independent, and what is left of the chain is eight steps of one FMA.  The
 // quotients D_i / D_j are products of the decays in between (no division, nothing overflows).  All sums are float32.
 // chunk_prepare_kernel makes D_i k_i, D_i q_i, k_j D_n / D_j and the two triangles once per chunk and head;
-// chunk_scan_kernel walks a sequence's chunks with the memory in registers: four columns in sixteen lanes, eight rows of
+// chunk_scan_kernel walks a sequence's chunks with the memory in registers: four (or two) columns in sixteen lanes, eight rows of
 // each a lane at 128.  A 16-byte read of shared memory takes a warp four cycles of its multiprocessor's port however many
 // lanes read the same, so what matters is how many FMAs such a read feeds (16 here; with a column in eight lanes
 // and one column a lane the port was the kernel's time).  The eight sums of a column's chunk end, after eight shuffles, with
@@ -205,11 +205,12 @@ __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b, float2 c) {
   d = *(float2*)&r;
 }
 
-constexpr int MC_CT = 4, MC_LANES = 16;                   // columns of a lane, lanes of a column
+constexpr int MC_LANES = 16;                              // lanes of a column
 
-template <int DK, bool LSTM, int WARPS>
+// CT: columns of a lane.
+template <int DK, bool LSTM, int WARPS, int CT>
 __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a) {
-  constexpr int REC = mc_record(DK, LSTM), NP = DK / 64, CT = MC_CT;      // a lane's rows: NP pieces of four, 64 apart
+  constexpr int REC = mc_record(DK, LSTM), NP = DK / 64;      // a lane's rows: NP pieces of four, 64 apart
   extern __shared__ __align__(16) float ring[];
   const int h = blockIdx.y, tid = threadIdx.x, l = tid % MC_LANES, row = l % MC_R, group = tid / MC_LANES;
   // Longest sequences first: a sequence is one walk however many blocks share its columns, so the last to begin should be
@@ -402,11 +403,11 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_scan_kernel(ChunkScanArgs a)
 
 // Ordinary launches: as programmatic dependents the scan's few blocks were placed while the preparation still ran, four
 // to a multiprocessor, and stayed there for the whole walk (1,500 rows of 8 heads: 790 instead of 340 us).
-template <int DK, bool LSTM, int WARPS>
+template <int DK, bool LSTM, int WARPS, int CT>
 int launch_chunk_scan(const ChunkScanArgs& a, int S, cudaStream_t s) {
-  const int ncols = LSTM ? a.dv + 1 : a.dv, per = 2 * WARPS * MC_CT;
+  const int ncols = LSTM ? a.dv + 1 : a.dv, per = 2 * WARPS * CT;
   const size_t smem = sizeof(float) * MC_RING * mc_record(DK, LSTM);
-  auto* kernel = chunk_scan_kernel<DK, LSTM, WARPS>;
+  auto* kernel = chunk_scan_kernel<DK, LSTM, WARPS, CT>;
   if (smem > 48 * 1024) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kernel<<<dim3((ncols + per - 1) / per, a.H, S), 32 * WARPS, smem, s>>>(a);
   NV_RETURN_LAST();
@@ -419,10 +420,16 @@ int launch_chunks(const ChunkArgs& p, const ChunkScanArgs& a, int T, cudaStream_
   chunk_prepare_kernel<DK, LSTM><<<dim3((unsigned)mc_records(T, S), a.H), DK, 0, s>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
-  // Blocks of 32 columns share a record between four warps; where they would not give every multiprocessor one, blocks of
-  // eight columns spread a few sequences further.
-  const long long wide = (long long)S * a.H * ((a.dv + 31) / 32);
-  return wide >= num_multiprocessors() ? launch_chunk_scan<DK, LSTM, 4>(a, S, s) : launch_chunk_scan<DK, LSTM, 1>(a, S, s);
+  // Blocks of 32 columns share a record between four warps of four columns a lane.  Where they would not give every
+  // multiprocessor one, a warp's instructions are the time of a chunk (1,130 of them, two cycles each, on one of four
+  // schedulers): two columns a lane halve them, at the price of reading the record twice as often, and four warps still share it
+  // (1,500 rows of one sequence, preparation and head norm included, 8 heads: delta rule 298 us with one warp of four columns a
+  // block, 263 so; matrix LSTM 309 and 272; 16 heads, a decay per channel, 328 and 280).  The LSTM's shorter chunks stay with the one
+  // warp where the halves are more than the multiprocessors (four sequences of 500, 8 heads: 152 and 155).
+  const int sms = num_multiprocessors();
+  const long long wide = (long long)S * a.H * ((a.dv + 31) / 32), half = (long long)S * a.H * ((a.dv + 15) / 16);
+  if (wide >= sms) return launch_chunk_scan<DK, LSTM, 4, 4>(a, S, s);
+  return LSTM && half > sms ? launch_chunk_scan<DK, LSTM, 1, 4>(a, S, s) : launch_chunk_scan<DK, LSTM, 4, 2>(a, S, s);
 }
 
 template <bool LSTM>
