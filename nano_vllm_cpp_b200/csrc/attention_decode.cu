@@ -848,13 +848,14 @@ NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context
   const long long blocks = (long long)rows * Hkv * ((G + 15) / 16);
   // at least 256 keys per split; 128 while all splits run at once (one row of 2,064 keys, 16 heads: 18.6 and 16.4 us; with
   // several waves of them 8 rows 39 and 49)
-  int most = (max_context + 127) / 128;
+  const int usual = (max_context + 255) / 256;
+  int most = max_context / 128 > usual ? max_context / 128 : usual;
   if (most > MAX_SPLITS) most = MAX_SPLITS;
   int best = 1;
   double best_score = -1.0;
   for (int s = 1; s <= most; ++s) {
     const long long ctas = blocks * s;
-    if (s > 1 && s > (max_context + 255) / 256 && ctas > slots) break;
+    if (s > usual && ctas > slots) break;
     const long long waves = (ctas + slots - 1) / slots;
     const double score = (double)ctas / ((double)waves * (double)slots) - 0.001 * s;
     if (score > best_score + 1e-9) { best_score = score; best = s; }

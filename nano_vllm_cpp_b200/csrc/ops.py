@@ -1649,7 +1649,7 @@ def gemm_terms(a, w, out, *, err=None) -> None:
     L = lib()
     terms = torch.empty((3 * T, K), dtype=torch.bfloat16, device=a.device)
     _check(L.nv_split_terms(_p(a), a.stride(0), _p(terms), T, K, _stream()), "split_terms")
-    n_tile = L.nv_tc_gemm_token_tile(T, 0)
+    n_tile = 256
     _check(L.nv_tc_gemm(_p(terms), K, T, _p(w), N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile, 1, _p(None),
                         _p(None), _p(None), _p(None), _p(None), 0, 0, _p(err.t if err is not None else _global_err().t), _early(),
                         0, 0, 0, _p(None), 0, 0.0, 0.0, 0, 0, 0, -3, _stream()), f"tc_gemm N={N} K={3 * K}", 6.0 * T * N * K)
@@ -1662,7 +1662,7 @@ def gemm_fast_segments(a, w, out, *, err=None, max_ctas: int = 0, tiles_ready=Tr
     T = out.shape[0]
     _need(gemm_fast_usable(a, w, out) and a.shape == (C * T, K) and out.shape[1] == N, "segmented product: operands")
     L = lib()
-    n_tile = L.nv_tc_gemm_token_tile(T, 0)
+    n_tile = 256                       # (the kernel of the big tiles knows segments, the others do not)
     splits = L.nv_tc_gemm_splits(T, N, C * ((K + 63) // 64) * 64, n_tile, 0, num_sms())
     scratch = torch.empty((splits, T, N), dtype=torch.float32, device=a.device) if splits > 1 else None
     _check(L.nv_tc_gemm(_p(a), a.stride(0), T, _p(w), C * N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile,

@@ -360,21 +360,22 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int boxes = (n_act + a.x_box - 1) / a.x_box;
         const uint32_t bytes = a_bytes * (two ? 2 : 1) + (uint32_t)boxes * a.x_box * 128;
         const int wr = t.w_row_base + t.nb * a.w_per_cta;
+        // (segments are for the big tiles only: what they add to a k-step cost the small tiles of decoding half a percent)
         int in_seg = t.k_begin + k0, wrow = wr, xrow = t.x_row0;
-        if (in_seg >= a.seg_steps) {               // (a division here at every product's tile cost decoding half a percent)
+        if (MODE == 2 && in_seg >= a.seg_steps) {
           const int seg = in_seg / a.seg_steps;
           in_seg -= seg * a.seg_steps;
           wrow += seg * a.w_seg_rows;
           xrow += seg * a.x_seg_rows;
         }
         for (int k = k0; k < k1; ++k, s_ = (s_ + 1 == a.stages ? 0 : s_ + 1), ph_ ^= (s_ == 0)) {
-          if (in_seg == a.seg_steps) { in_seg = 0; wrow += a.w_seg_rows; xrow += a.x_seg_rows; }
+          if (MODE == 2 && in_seg == a.seg_steps) { in_seg = 0; wrow += a.w_seg_rows; xrow += a.x_seg_rows; }
           const uint32_t st = smem0 + (uint32_t)s_ * stage_bytes, bar = full0 + (uint32_t)s_ * 8;
           if (weights) {
             mbar_wait(&empty_bar[s_], ph_ ^ 1, a.err, 0x7001);
             mbar_expect_tx_a(bar, bytes);
           }
-          const int kc = in_seg++ * BLOCK_K;
+          const int kc = MODE == 2 ? in_seg++ * BLOCK_K : (t.k_begin + k) * BLOCK_K;
           if (weights) {
             tma_load_2d_a(st, &tm_w, bar, kc, wrow);
             if (two)     // swiglu: the up rows of the same features; dual: the next 128 features
@@ -856,6 +857,7 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
     }
   }
   const int mode = n_tile < 32 ? 0 : ((!pair && n_tile >= 128) ? 2 : 1);
+  if (segments > 1 && mode != 2) return NV_ERR_UNSUPPORTED;      // (token tiles of 256 are such)
   const auto kernel = mode == 0 ? tc_gemm_kernel<0> : (mode == 1 ? tc_gemm_kernel<1> : tc_gemm_kernel<2>);
   const unsigned threads = mode == 2 ? WIDE_THREADS : NUM_THREADS;
   cudaError_t e;

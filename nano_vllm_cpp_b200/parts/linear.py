@@ -15,8 +15,8 @@ from ..csrc import ops
 SKINNY_ROWS = ops.SKINNY_MAX_ROWS
 SKINNY_MAX_BYTES = 128 << 20
 # float32 rows times a bfloat16 matrix with a short K (the second half of a low-rank projection), prompts of a bfloat16 run:
-# three bfloat16 terms on the tensor cores, from so many rows on and up to so long a K.  (6,737 rows, 64 -> 2,048:
-# 97 us in FFMAs, 4 + 22 so; relative error against float64 7.9e-8, 1.06e-7 in FFMAs.  The accumulator of the tensor cores loses more with every
+# three bfloat16 terms on the tensor cores, from so many rows on and up to so long a K.  (6,737 rows, 64 -> 2,048: 97 us in
+# FFMAs, 4 + 22 so; relative error against float64 7.9e-8, 1.06e-7 in FFMAs.  The tensor cores' accumulator loses more with every
 # step: at K = 128 1.26e-7 against 1.11e-7, at 512 4.8e-7 against 1.6e-7.)
 TERMS_MIN_ROWS = 256
 TERMS_MAX_K = 64
