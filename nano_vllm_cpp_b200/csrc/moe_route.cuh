@@ -178,7 +178,7 @@ __device__ __forceinline__ void spread_tail_tiles(int* __restrict__ tile_expert,
 // counts and offsets per expert, the pairs sorted by expert (sorted_token = source row of each sorted
 // position, pair_pos = sorted position of each pair) and the list of tiles (expert, first row, rows)
 // of at most tile_m rows — and a second list cut by tile_m2, for a product that prefers another tile
-// (t2 == nullptr: none).  One block of 1024 threads; `al_s` is 4 * E ints of shared memory.  The
+// (t2 == nullptr: none).  One block of whole warps; `al_s` is 4 * E ints of shared memory.  The
 // order of pairs inside an expert's segment comes from atomics and may differ from run to run; it
 // decides only where a pair's row sits, never a sum's order.
 // The last `n_static` experts are ones that every row visits (a shared expert's chunks): their pairs sit in row

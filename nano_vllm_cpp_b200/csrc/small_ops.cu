@@ -324,6 +324,9 @@ NV_API int nv_moe_route_small(const float* logits, long long ld, int T, int E, i
   if (T == 0) return NV_OK;
   const size_t smem = (size_t)32 * (E + groups) * sizeof(double) + (size_t)4 * (E + C) * sizeof(int);
   const unsigned threads = x ? 1024 : 32 * (T < 4 ? 4 : T < 32 ? T : 32);
+  // (beyond 44 KB the choices' 4 KB of static shared memory take a block over the 48 KB that need no leave)
+  if (smem + sizeof(int) * ROUTE_PAIRS > 48 * 1024)
+    NV_RETURN_IF(cudaFuncSetAttribute(moe_route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024));
   NV_RETURN_IF(launch_dep(moe_route_small_kernel, dim3(1), dim3(threads), smem, s, logits, ld, T, E, K, renorm, C,
                           gate_logit, gate_ld, idx, score, tile_m, counts, offsets, sorted_token, pair_pos, tile_expert,
                           tile_row0, tile_rows, num_tiles, err, (const bf16*)x, (bf16*)x_sorted, H, n_static, zero,
