@@ -80,7 +80,7 @@ struct DecArgs {
   float cap_in;           // MOD 2: scale / softcap
 };
 
-constexpr int MAX_SPLITS = 32;          // one lane each where they are added up
+constexpr int MAX_SPLITS = 32;          // of the library's own choice: one lane each where they are added up
 constexpr int FEW_SPLITS = 8;
 
 // The splits of a head added up in their order: m and l of split s at part_ml[2 s], its elements at part_o[s D].  One load after
@@ -131,6 +131,19 @@ __device__ __forceinline__ float split_sum(const float* part_o, const float* w, 
       if (s0 + i < splits) o = fmaf(v[i], w[s0 + i], o);
   }
   return o;
+}
+// A caller's choice of more splits than a warp has lanes: one after the other.
+__device__ __forceinline__ float many_splits_sum(const float* part_ml, const float* part_o, int splits, int D, bool has_sink, float sink,
+                                                 float gate) {
+  float mm = -1e30f, ll = 0.f, o = 0.f;
+  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, __ldcg(part_ml + s * 2));
+  for (int s = 0; s < splits; ++s) {
+    const float sc = __expf(__ldcg(part_ml + s * 2) - mm);
+    ll = fmaf(__ldcg(part_ml + s * 2 + 1), sc, ll);
+    o = fmaf(__ldcg(part_o + (size_t)s * D), sc, o);
+  }
+  if (has_sink) ll += __expf(sink - mm);
+  return o * ((ll > 0.f ? 1.f / ll : 0.f) * gate);
 }
 
 // Called by every thread of a block once the block has written its split's partial results for the query heads
@@ -754,6 +767,12 @@ __global__ void attention_decode_merge_kernel(const float* __restrict__ part_o, 
             few_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
     return;
   }
+  if (splits > MAX_SPLITS) {
+    for (int d = threadIdx.x; d < D; d += blockDim.x)
+      st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d,
+            many_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
+    return;
+  }
   __shared__ float w_s[MAX_SPLITS];
   if (threadIdx.x < 32) split_weights(part_ml + pi * 2, splits, threadIdx.x, has_sink, sink, head_gate_of(gate, t, h), w_s);
   __syncthreads();
@@ -891,7 +910,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   if (((uintptr_t)kc & 15) || ((uintptr_t)vc & 15)) return NV_ERR_UNSUPPORTED;
   if (R == 0) return NV_OK;
   if (splits < 1) splits = 1;
-  if (splits > MAX_SPLITS || (splits > 1 && !scratch)) return NV_ERR_BAD_SIZE;
+  if (splits > 1 && !scratch) return NV_ERR_BAD_SIZE;
   DecArgs a;
   a.qkv = qkv; a.kc = kc; a.vc = vc; a.block_table = block_table; a.row_entry = row_entry; a.positions = positions;
   a.rows = rows; a.out = out; a.scale = scale; a.q_dt = q_dt; a.out_dt = out_dt; a.q_stride = q_stride;
@@ -918,7 +937,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // and 21.5).
   {
     const int heads_per_block = Hq / Hkv < 16 ? Hq / Hkv : 16;
-    if ((long long)heads_per_block * D > 256) a.split_count = nullptr;
+    if ((long long)heads_per_block * D > 256 || splits > MAX_SPLITS) a.split_count = nullptr;
   }
   a.stages = stages;
   const size_t smem = (size_t)stages * 2 * page * D * esize;

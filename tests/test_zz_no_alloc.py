@@ -94,3 +94,26 @@ def test_no_alloc_decode_attention_matches_the_ordinary_entry_point():
     assert _call(lib, "nv_attention_decode_noalloc", qkv[:2], kc, vc, bt, ent, pos, out[:2], Hq, Hkv, 20, page, splits) == -4
     assert _call(lib, "nv_attention_decode_noalloc", qkv[:2], kc, vc, bt, ent, pos, out[:2], Hq, 0, D, page, splits) == -4
     assert _call(lib, "nv_attention_decode_noalloc", qkv[:2], kc, vc, bt, ent, pos, out[:2], -Hq, -Hkv, D, page, splits) == -4
+
+
+@pytest.mark.parametrize("splits", [8, 9, 31, 32, 33, 100, 1024])
+@pytest.mark.parametrize("D", [64, 40])
+def test_any_number_of_splits(splits, D):
+    """A caller chooses the splits (more of them than pages, too): both entry points against float64.  The weights are
+    rounded to bfloat16 before their product with the values (2^-9 of each, in the form for heads of 64; the form for 40 keeps
+    float32), the result to bfloat16 (2^-9 of it)."""
+    from nano_vllm_cpp_b200.csrc import ops
+    lib = ops.lib()
+    Hq, Hkv, page, lens = 8, 2, 16, [1900]
+    qkv, kc, vc, bt, ent, pos = _setup(lens, Hq, Hkv, D, page, seed=splits)
+    pages = bt[0].long()
+    k, v = (c[pages].double().transpose(1, 2).reshape(-1, Hkv, D)[:lens[0]].repeat_interleave(Hq // Hkv, dim=1) for c in (kc, vc))
+    p = torch.softmax(torch.einsum("hd,nhd->hn", qkv[0, :Hq * D].double().view(Hq, D), k) / math.sqrt(D), dim=1)
+    want, size = (torch.einsum("hn,nhd->hd", p, x).reshape(-1) for x in (v, v.abs()))
+    lib.nv_attention_decode_noalloc_max_rows.restype = c_int
+    assert lib.nv_attention_decode_noalloc_max_rows(c_int(Hq), c_int(D), c_int(splits)) >= 1
+    scratch = torch.empty(Hq * splits * (D + 2), dtype=torch.float32, device=DEV)
+    for name, room in (("nv_attention_decode_noalloc", None), ("nv_attention_decode", scratch)):
+        out = torch.full((1, Hq * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        assert _call(lib, name, qkv, kc, vc, bt, ent, pos, out, Hq, Hkv, D, page, splits, room) == 0
+        assert bool(((out[0].double() - want).abs() <= 2.0 ** -8 * size + 2.0 ** -8 * want.abs() + 1e-5).all()), name
