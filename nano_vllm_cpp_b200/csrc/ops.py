@@ -348,9 +348,12 @@ def _act_numbers(act):
     return (float(act[1]), float(act[2]) if len(act) > 2 else 0.0) if isinstance(act, tuple) else (0.0, 0.0)
 
 
-def gemm_plain(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, tiles=None, act=None) -> None:
+def gemm_plain(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, tiles=None, act=None, w_ready=False) -> None:
     """out[m, :] = a[a_rows[m] or m, :] @ w.T (+ bias), or silu(gate) * up with ``swiglu``, or with ``act``
     (gelu_erf, gelu_tanh, silu) that function of every value.
+
+    ``w_ready``: ``w`` was complete before the kernel that precedes this product on the stream started (a layer's weights);
+    the product may then read it before that kernel has ended.
 
     ``tiles`` = (tile_expert, tile_row0, tile_rows, num_tiles) selects the grouped form, where w is
     [E, rows, K]."""
@@ -383,7 +386,7 @@ def gemm_plain(a, w, out, *, bias=None, a_rows=None, swiglu=False, M=None, tiles
                                _p(bias), (dt(bias) if bias is not None else 0),
                                _p(out), dt(out), out.stride(0),
                                M, N, K, _epilogue(swiglu, act),
-                               _p(te), _p(tr0), _p(tr), _p(nt), max_tiles, *_act_numbers(act), _stream()), "gemm_plain")
+                               _p(te), _p(tr0), _p(tr), _p(nt), max_tiles, *_act_numbers(act), (1 if w_ready else 0), _stream()), "gemm_plain")
 
 
 def rowdot(a, w, out, wide: bool = False) -> None:

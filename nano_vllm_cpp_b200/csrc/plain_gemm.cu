@@ -55,6 +55,7 @@ struct GemmArgs {
   float act_p0, act_p1;     // its two numbers (xIELU)
   int a_vec, w_vec;         // rows of A / W start on 16 bytes: copied in pieces of 16, else element by element
   int rows_alloc;           // rows of A that a stage has room for, and the rows of a dense tile
+  int early;                // W may be read before the kernel in front has finished: that kernel does not write it
 };
 
 __device__ __forceinline__ void copy16(void* dst, const void* src, int bytes) {      // the rest of the 16 is zeroed
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(128, (SWIGLU ? 2 : 1) * FT >= 4 ? 4 : 5) gemm_
 // ------------------------------------------------------------------ a handful of rows
 // What bounds it: the stream of W, and for one product the way from the launch to the first sums.  A block makes up to 16
 // rows x 16 rows of W (8 pairs); its eight warps take a range of K each, so the chain of an output is K / 8 FFMAs, through
-// rings of their own that no other warp waits for.  A dense product asks for its first stages of W before the kernel in
+// rings of their own that no other warp waits for.  A dense product of weights asks for its first stages of W before the kernel in
 // front of it has finished.  Measured (float32, two rows, cold weights, the launch included): 1,024 -> 1,536 14.4 us with one
 // chain over K and 16 features a block, 9.2 so; 2,048 -> 2,048 22.6 and 12.3; eight pairs of 16 experts, SwiGLU 1,024 -> 512
 // 20.5 and 16.4.  In a chain of decode steps (two rows, four layers of width 1,024 with experts of 512) a product of rows took
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(256) gemm_few_kernel(GemmArgs g) {
   int row0 = 0, rows_here = g.M;
   const TW* W = (const TW*)g.W;
   const int col0 = blockIdx.x * (SWIGLU ? 8 : 16);
-  const bool early = !g.tile_expert && !g.a_rows && g.w_vec;
+  const bool early = g.early && !g.tile_expert && !g.a_rows && g.w_vec;
   if (early) {
     constexpr int WROW = FEW_STEP * sizeof(TW) + 16, AROW = FEW_STEP * sizeof(TA) + 16, WCH = FEW_STEP * sizeof(TW) / 16;
     const int c = threadIdx.x / 32, lane = threadIdx.x % 32, L = class_len(g.K), k_end = min(g.K, (c + 1) * L);
@@ -472,7 +473,8 @@ NV_API int nv_gemm_plain(const void* A, int a_dt, long long lda, const int* a_ro
                          void* out, int out_dt, long long ldo,
                          int M, int N, int K, int swiglu,
                          const int* tile_expert, const int* tile_row0, const int* tile_rows,
-                         const int* num_tiles, int max_tiles, float act_p0, float act_p1, cudaStream_t stream) {
+                         const int* num_tiles, int max_tiles, float act_p0, float act_p1, int early, cudaStream_t stream) {
+  // early: the kernel in front on the stream does not write W (a layer's weights), which may then be read before it has ended
   if (!dt_ok(a_dt) || !dt_ok(w_dt) || !dt_ok(out_dt) || (bias && !dt_ok(bias_dt))) return NV_ERR_BAD_DTYPE;
   if (M < 0 || N <= 0 || K <= 0 || swiglu < 0 || swiglu > NV_EPI_LAST) return NV_ERR_BAD_SIZE;
   const int act = epi_unary(swiglu);
@@ -484,7 +486,7 @@ NV_API int nv_gemm_plain(const void* A, int a_dt, long long lda, const int* a_ro
   g.A = A; g.W = W; g.bias = bias; g.out = out; g.a_rows = a_rows;
   g.tile_expert = tile_expert; g.tile_row0 = tile_row0; g.tile_rows = tile_rows; g.num_tiles = num_tiles;
   g.lda = lda; g.ldo = ldo; g.w_expert_stride = w_expert_stride;
-  g.M = M; g.N = N; g.K = K; g.bias_dt = bias_dt; g.out_dt = out_dt; g.swiglu = swiglu;
+  g.M = M; g.N = N; g.K = K; g.bias_dt = bias_dt; g.out_dt = out_dt; g.swiglu = swiglu; g.early = early;
   const size_t ea = a_dt == NV_DT_F32 ? 4 : 2, ew = w_dt == NV_DT_F32 ? 4 : 2;
   g.a_vec = (uintptr_t)A % 16 == 0 && lda * ea % 16 == 0;
   g.w_vec = (uintptr_t)W % 16 == 0 && K * ew % 16 == 0 && w_expert_stride * ew % 16 == 0;

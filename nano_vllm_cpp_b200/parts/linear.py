@@ -23,7 +23,8 @@ TERMS_MAX_K = 64
 
 
 def linear(ctx, a, w, out_dtype, *, bias=None, a_rows=None, swiglu=False, M=None, out=None, act=None):
-    """``out = a[a_rows] @ w.T (+ bias)``; with ``swiglu`` w is [2N, K] (gate rows, then up rows)
+    """``out = a[a_rows] @ w.T (+ bias)`` for weights ``w`` (no kernel of the step writes them: they are read ahead of it);
+    with ``swiglu`` w is [2N, K] (gate rows, then up rows)
     and ``out = silu(a @ gate.T) * (a @ up.T)``; with ``act`` (gelu_erf, gelu_tanh, silu, relu2) every value of the
     result passes that function in the product's epilogue, on the float32 sum; ``swiglu`` with
     ``act=("glu_clamped", limit, slope)`` pairs the rows as ``g sigmoid(slope g) (u + 1)`` with ``g = min(gate, limit)``
@@ -49,7 +50,7 @@ def linear(ctx, a, w, out_dtype, *, bias=None, a_rows=None, swiglu=False, M=None
           and M == a.shape[0] and bias is None and a_rows is None and act is None and not swiglu and ops.gemm_terms_usable(a, w, out)):
         ops.gemm_terms(a, w, out, err=ctx.err)
     else:
-        ops.gemm_plain(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu, M=M, act=act)
+        ops.gemm_plain(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu, M=M, act=act, w_ready=True)
     return out
 
 

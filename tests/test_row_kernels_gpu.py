@@ -387,3 +387,18 @@ def test_portions_beside_single_rows(refused, monkeypatch):
         want = torch.einsum("hn,nhd->hd", s.softmax(-1), v)
         # one bfloat16 term a weight and a bfloat16 result
         assert bool(((got[t].double().view(Hq, D) - want).abs() <= 2.0 ** -8 * want.abs() + 8e-3).all())
+
+
+def test_product_with_a_matrix_of_the_kernel_in_front():
+    """A handful of rows times a matrix that the kernel right before wrote: read only once that kernel has ended."""
+    o, N, K = ops(), 512, 1024
+    x, a = rnd(N, K, seed=1), rnd(2, K, seed=2)
+    w, out = torch.zeros(N, K, device=DEV), torch.empty(6, 2, N, device=DEV)
+    eyes = [s * torch.eye(K, device=DEV) for s in (1.0, 2.0, 4.0, 8.0, 16.0, 32.0)]       # (powers of two change no rounding)
+    for i, eye in enumerate(eyes):
+        o.gemm_plain(x, eye, w)
+        o.gemm_plain(a, w, out[i])
+    first = torch.empty(2, N, device=DEV)
+    o.gemm_plain(a, x, first, w_ready=True)
+    for i in range(len(eyes)):
+        assert torch.equal(out[i], first * 2.0 ** i)
