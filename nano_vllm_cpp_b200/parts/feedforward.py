@@ -183,7 +183,7 @@ class SparseMoeSwiGLU(FeedForward):
         self._captured = {}
         self._static = {}
         self._static_kept = set()
-        self._pair_rows = {}            # (rows of a step, device) -> the numbers of its pairs (a handful of small steps)
+        self.pair_rows = None           # the numbers of a small step's pairs (set at load)
         self.router_and_gate = None
         self.last_alignment = None      # the permutation buffers of the latest forward (for statistics)
 
@@ -233,6 +233,8 @@ class SparseMoeSwiGLU(FeedForward):
         EC = E + self.virtual
         # every expert's [gate; up] rows and down matrix in one block each, indexed by expert
         self.w_gate_up = torch.empty((EC, G * I, H), dtype=first.dtype, device=first.device)
+        # (with the weights, so that it is there for whichever stream a step runs on)
+        self.pair_rows = torch.arange(FEW_PAIRS, dtype=torch.int32, device=first.device)
         self.w_down = torch.empty((EC, H, I), dtype=first.dtype, device=first.device)
         if stacked:
             self.w_gate_up[:E].copy_(first)
@@ -367,12 +369,7 @@ class SparseMoeSwiGLU(FeedForward):
         ops.few_experts(h, self.w_gate_up, self.w_down, act, y, logits, self.K, self.renorm, self.virtual, gate_logit, idx, score,
                         gated=self.gated, fn=self.expert_act, rule=self.rule)
         self.last_alignment = _Choices(idx, self.E + self.virtual)
-        key = (T, dev)
-        rows = self._pair_rows.get(key)                    # pair (t, k) stands in row t KT + k
-        if rows is None:
-            rows = torch.arange(T * KT, dtype=torch.int32, device=dev).view(T, KT)
-            if not torch.cuda.is_current_stream_capturing():      # (memory of a capture is the capture's)
-                self._pair_rows[key] = rows
+        rows = self.pair_rows[:T * KT].view(T, KT)         # pair (t, k) stands in row t KT + k
         return RowMix(y, rows, score, None, None)
 
     def _forward_beside(self, h, logits, gate_logit, idx, score, al, many=False):

@@ -51,3 +51,26 @@ def test_what_few_experts_leaves_to_the_others():
     x, w1, w2 = (torch.zeros(*s, dtype=torch.bfloat16, device=DEV) for s in ((9, 64), (2, 64, 64), (2, 64, 32)))
     assert not o.few_experts_usable(x, w1, w2, 9, 2, 1, 0, 64, 32)                     # nine rows
     assert not o.few_experts_usable(x[:1].float(), w1, w2, 1, 2, 1, 0, 64, 32)
+
+
+def test_first_small_steps_on_two_streams():
+    """A layer's first step of a handful of rows waits on one stream; a step on another stream needs nothing of it."""
+    from test_parts_gpu import DictFetch, ctx_for, rand_tensors
+    from nano_vllm_cpp_b200.parts import PartSpec, build_part
+    H, I = 64, 32
+    part = build_part("feed_forward", PartSpec("sparse_moe_swiglu", dict(hidden_size=H, num_experts=6, top_k=2, intermediate_size=I,
+                                                                          shared_intermediate_size=2 * I)))
+    part.load(DictFetch(rand_tensors(part.tensor_specs(), 1), torch.bfloat16), ctx_for(torch.bfloat16))
+    h = rnd(2, H, seed=7).to(torch.bfloat16)
+    h32 = h.float()
+    torch.cuda.synchronize()
+    held, free = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(held):
+        torch.cuda._sleep(200_000_000)
+        late = part.forward(h, h32, None).sum()
+    with torch.cuda.stream(free):
+        got = part.forward(h, h32, None).sum()
+    free.synchronize()
+    got = got.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(got, late) and torch.equal(got, part.forward(h, h32, None).sum())
