@@ -1644,8 +1644,8 @@ def gemm_terms_usable(a, w, out) -> bool:
 
 def gemm_terms(a, w, out, *, err=None) -> None:
     """``out = a @ w.T`` for float32 ``a`` [T, K] and bfloat16 ``w`` [N, K] on the tensor cores: a value of ``a`` is the sum of
-    three bfloat16 terms, exactly, products of bfloat16 values are exact in float32, and the terms' products are added from the
-    smallest on, in one accumulator."""
+    three bfloat16 terms, to within 2^-132, products of bfloat16 values are exact in float32, and the terms' products are
+    added from the smallest on, in one accumulator.  Infinities and NaN of either operand come out as in ``gemm_plain``."""
     T, K = a.shape
     N = w.shape[0]
     _need(gemm_terms_usable(a, w, out) and w.shape[1] == K and out.shape == (T, N), "product of terms: operands")

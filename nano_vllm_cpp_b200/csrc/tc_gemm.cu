@@ -596,7 +596,10 @@ __global__ void tc_gemm_finish_grouped_kernel(const float* __restrict__ partial,
 }
 
 // A float32 value as three bfloat16 terms that add up to it exactly (eight bits each, cut off and not rounded, so that no
-// term is larger than the value; what is not finite is its first term): out[0] = the last bits, out[2] = the first, [3][T][K].
+// term is larger than the value): out[0] = the last bits, out[2] = the first, [3][T][K].  No term of a value other than zero
+// is zero, so that its product with an infinite weight is infinite as the value's own is: a term without bits is the
+// smallest number of the value's sign (2^-133, nothing beside any value that a float32 sum can hold exactly), and an infinite
+// value is infinite in every term.
 __global__ void split_terms_kernel(const float* __restrict__ x, long long ldx, bf16* __restrict__ out, int T, int K) {
   grid_dep_wait();
   grid_dep_launch();
@@ -605,13 +608,18 @@ __global__ void split_terms_kernel(const float* __restrict__ x, long long ldx, b
   const long long t = i / K;
   const float v = x[t * ldx + (i - t * K)];
   const uint32_t u = __float_as_uint(v);
-  const bool number = v == v, finite = (u & 0x7f800000u) != 0x7f800000u;
-  const float hi = number ? __uint_as_float(u & 0xffff0000u) : v;
-  const float rest = finite ? v - hi : 0.f;
-  const float mid = __uint_as_float(__float_as_uint(rest) & 0xffff0000u);
-  out[i] = __float2bfloat16_rn(rest - mid);
-  out[n + i] = __float2bfloat16_rn(mid);
-  out[2 * n + i] = __float2bfloat16_rn(hi);
+  const bool finite = (u & 0x7f800000u) != 0x7f800000u;
+  const float hi = v == v ? __uint_as_float(u & 0xffff0000u) : v;      // (a NaN's upper half alone may be an infinity)
+  const float rest = finite ? v - hi : v;
+  const float mid = finite ? __uint_as_float(__float_as_uint(rest) & 0xffff0000u) : v;
+  auto put = [&](long long at, float f) {
+    uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(f));
+    if (v != 0.f && !(b & 0x7fff)) b = (uint16_t)(u >> 16 & 0x8000u) | 1;
+    out[at] = __ushort_as_bfloat16(b);
+  };
+  put(i, finite ? rest - mid : v);
+  put(n + i, mid);
+  put(2 * n + i, hi);
 }
 
 // out[r, :] = src[rows[r], :] for bf16 rows (the expert-sorted copy of the activations)

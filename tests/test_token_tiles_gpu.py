@@ -106,3 +106,30 @@ def test_product_of_three_terms(T, N, K):
     a[0, 1] = float("nan")
     o.gemm_terms(a, w, out, err=err)
     assert bool(out[0].isnan().all()) and bool(out[1:].isfinite().all())
+
+
+@pytest.mark.parametrize("K", [8, 40, 64])
+def test_product_of_three_terms_with_infinite_weights(K):
+    """Values whose lower terms have no bits (whole numbers, powers of two), tiny ones, zero and infinite ones, times weights of
+    which some are infinite or NaN: infinities and NaN stand where the chain of FFMAs has them; other columns are as without."""
+    o, T, N = ops(), 300, 136
+    g = torch.Generator().manual_seed(K)
+    a = torch.randint(-3, 4, (T, K), generator=g).float()
+    a[a == 0] = 1.5
+    a[100:200] = torch.randn(100, K, generator=g)
+    a[200:] *= 2.0 ** -100
+    a[7, 0], a[8, 1], a[9, 2], a[10, 3] = 0.0, float("inf"), float("-inf"), float("nan")
+    w = torch.randn(N, K, generator=g) * 0.02
+    w[3, 0], w[4, 1], w[5, 2], w[6, 3] = float("inf"), float("-inf"), float("nan"), 0.0
+    w[7, :2] = torch.tensor([float("inf"), float("-inf")])
+    a, w = a.to(DEV), w.to(DEV).to(torch.bfloat16)
+    out, plain = torch.empty(T, N, device=DEV), torch.empty(T, N, device=DEV)
+    o.gemm_terms(a, w, out)
+    o.gemm_plain(a, w, plain)
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isposinf(), plain.isposinf())
+    assert torch.equal(out.isneginf(), plain.isneginf()) and bool(plain.isposinf().any()) and bool(plain.isneginf().any())
+    fine = plain.isfinite()
+    want = (a.double() @ w.double().T)[fine]
+    size = (a.double().abs() @ w.double().abs().T)[fine]
+    # exact products, K of them with three terms each added in float32 (cut off), of values no larger than their sum of sizes
+    assert bool(((out[fine].double() - want).abs() <= 3 * K * 2.0 ** -23 * size).all())
