@@ -1652,26 +1652,10 @@ def gemm_terms(a, w, out, *, err=None) -> None:
     L = lib()
     terms = torch.empty((3 * T, K), dtype=torch.bfloat16, device=a.device)
     _check(L.nv_split_terms(_p(a), a.stride(0), _p(terms), T, K, _stream()), "split_terms")
-    n_tile = 256
+    n_tile = 256                       # (the kernel of the big tiles knows segments, the others do not)
     _check(L.nv_tc_gemm(_p(terms), K, T, _p(w), N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile, 1, _p(None),
                         _p(None), _p(None), _p(None), _p(None), 0, 0, _p(err.t if err is not None else _global_err().t), _early(),
-                        0, 0, 0, _p(None), 0, 0.0, 0.0, 0, 0, 0, -3, _stream()), f"tc_gemm N={N} K={3 * K}", 6.0 * T * N * K)
-
-
-def gemm_fast_segments(a, w, out, *, err=None, max_ctas: int = 0, tiles_ready=True) -> None:
-    """``out = sum_c a[c * T:(c + 1) * T] @ w[c].T`` on the tensor cores, one sum over all segments: ``a`` [C * T, K] and
-    ``w`` [C, N, K] bfloat16 (a matrix whose columns lie in C blocks of rows), ``out`` [T, N]."""
-    C, N, K = w.shape
-    T = out.shape[0]
-    _need(gemm_fast_usable(a, w, out) and a.shape == (C * T, K) and out.shape[1] == N, "segmented product: operands")
-    L = lib()
-    n_tile = 256                       # (the kernel of the big tiles knows segments, the others do not)
-    splits = L.nv_tc_gemm_splits(T, N, C * ((K + 63) // 64) * 64, n_tile, 0, num_sms())
-    scratch = torch.empty((splits, T, N), dtype=torch.float32, device=a.device) if splits > 1 else None
-    _check(L.nv_tc_gemm(_p(a), a.stride(0), T, _p(w), C * N, N, K, _p(None), 0, _p(out), dt(out), out.stride(0), 0, n_tile,
-                        splits, _p(scratch), _p(None), _p(None), _p(None), _p(None), 0, 0,
-                        _p(err.t if err is not None else _global_err().t), (_early() if tiles_ready else 0), 0, 0, max_ctas,
-                        _p(None), 0, 0.0, 0.0, 0, 0, 0, C, _stream()), f"tc_gemm N={N} K={C * K}", 2.0 * T * N * C * K)
+                        0, 0, 0, _p(None), 0, 0.0, 0.0, 0, 0, 0, 3, _stream()), f"tc_gemm N={N} K={3 * K}", 6.0 * T * N * K)
 
 
 def gemm_fast_grouped(a, w, out, align, *, a_rows=None, swiglu=False, err=None, tiles=None, tiles_ready=False,

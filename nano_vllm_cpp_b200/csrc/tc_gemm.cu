@@ -78,9 +78,9 @@ struct TcArgs {
   // own: a product per head of rows that hold their heads side by side.  (Columns that a k-step reads beyond the
   // head's own meet the zeros that the weight map fills in beyond K.)
   int x_col_step, o_col_step;
-  // Dense products whose K lies in segments (seg_steps k-steps each): segment c's columns of W's rows stand in rows
-  // c * w_seg_rows further down, those of X's in rows c * x_seg_rows.  Without segments seg_steps is beyond every k-step.
-  int seg_steps, w_seg_rows, x_seg_rows;
+  // Dense products over several X with one W, one sum of all (seg_steps k-steps each): segment c's rows of X stand
+  // c * x_seg_rows further down.  Without segments seg_steps is beyond every k-step.
+  int seg_steps, x_seg_rows;
   // Tiles handed out by a counter instead of by position (nullptr: CTA b takes tiles b, b + grid, ...): a CTA that
   // starts late, because another kernel still holds its multiprocessor, then takes fewer tiles, and CTAs whose tiles
   // are short take more.  The counter must be 0 at launch; the CTA that draws the last number sets it back to 0.
@@ -361,15 +361,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const uint32_t bytes = a_bytes * (two ? 2 : 1) + (uint32_t)boxes * a.x_box * 128;
         const int wr = t.w_row_base + t.nb * a.w_per_cta;
         // (segments are for the big tiles only: what they add to a k-step cost the small tiles of decoding half a percent)
-        int in_seg = t.k_begin + k0, wrow = wr, xrow = t.x_row0;
+        int in_seg = t.k_begin + k0, xrow = t.x_row0;
         if (MODE == 2 && in_seg >= a.seg_steps) {
           const int seg = in_seg / a.seg_steps;
           in_seg -= seg * a.seg_steps;
-          wrow += seg * a.w_seg_rows;
           xrow += seg * a.x_seg_rows;
         }
         for (int k = k0; k < k1; ++k, s_ = (s_ + 1 == a.stages ? 0 : s_ + 1), ph_ ^= (s_ == 0)) {
-          if (MODE == 2 && in_seg == a.seg_steps) { in_seg = 0; wrow += a.w_seg_rows; xrow += a.x_seg_rows; }
+          if (MODE == 2 && in_seg == a.seg_steps) { in_seg = 0; xrow += a.x_seg_rows; }
           const uint32_t st = smem0 + (uint32_t)s_ * stage_bytes, bar = full0 + (uint32_t)s_ * 8;
           if (weights) {
             mbar_wait(&empty_bar[s_], ph_ ^ 1, a.err, 0x7001);
@@ -377,9 +376,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           }
           const int kc = MODE == 2 ? in_seg++ * BLOCK_K : (t.k_begin + k) * BLOCK_K;
           if (weights) {
-            tma_load_2d_a(st, &tm_w, bar, kc, wrow);
+            tma_load_2d_a(st, &tm_w, bar, kc, wr);
             if (two)     // swiglu: the up rows of the same features; dual: the next 128 features
-              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, wrow + (a.swiglu ? a.N : TILE_W));
+              tma_load_2d_a(st + a_bytes, &tm_w, bar, kc, wr + (a.swiglu ? a.N : TILE_W));
           }
           if (tokens)
             for (int b = 0; b < boxes; ++b)
@@ -756,9 +755,8 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
                       int early, int x_sub, int x_mod, int max_ctas, int* tile_counter, int m_out,
                       float act_p0, float act_p1, int x_col_step, int o_col_step, int x_cols, int segments,
                       cudaStream_t stream) {
-  // segments > 1 (dense products): W is [segments, N, K] and X [segments, M_tok, K], and out = sum over the segments of
-  // X[s] W[s]^T, one sum of segments * K terms; `w_rows_total` is segments * N.  segments < -1: -segments of them over one
-  // W [N, K].
+  // segments > 1 (dense products): X is [segments, M_tok, K], and out = sum over the segments of X[s] W^T, one sum of
+  // segments * K terms.
   // x_col_step / o_col_step (grouped products only): see TcArgs; x_cols: the columns that a row of X holds then (K is
   // the columns of one block).  Such a product does not split K, and its steps are 8 columns aligned.
   if (!dt_ok(out_dt) || (bias && !dt_ok(bias_dt))) return NV_ERR_BAD_DTYPE;
@@ -775,9 +773,7 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   if (x_mod < 0 || x_sub < 0 || (x_mod && !grouped)) return NV_ERR_BAD_SIZE;
   if (splits > 1 && !scratch) return NV_ERR_BAD_SIZE;
 
-  const bool one_w = segments < 0;
-  if (one_w) segments = -segments;
-  if (segments < 1 || (segments > 1 && (grouped || w_rows_total != (one_w ? 1 : segments) * N || swiglu))) return NV_ERR_BAD_SIZE;
+  if (segments < 1 || (segments > 1 && (grouped || w_rows_total != N || swiglu))) return NV_ERR_BAD_SIZE;
   if ((long long)segments * M_tok > 0x7fffffff) return NV_ERR_BAD_SIZE;
 
   CUtensorMap tm_w, tm_x;
@@ -793,7 +789,6 @@ NV_API int nv_tc_gemm(const void* X, long long ldx, int M_tok, const void* W, in
   a.M_tok = M_tok; a.N = N; a.rows_per_expert = rows_per_expert;
   a.M_out = grouped && m_out > 0 ? m_out : M_tok;
   a.seg_steps = segments > 1 ? (K + BLOCK_K - 1) / BLOCK_K : 0x3fffffff;
-  a.w_seg_rows = one_w ? 0 : N;
   a.x_seg_rows = M_tok;
   a.k_steps_total = segments * ((K + BLOCK_K - 1) / BLOCK_K);
   a.splits = splits < 1 ? 1 : splits;

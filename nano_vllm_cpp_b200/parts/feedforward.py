@@ -15,10 +15,6 @@ SIDE_MAX_ROWS = 64
 # copy) on a second stream with their grid capped to this share of the multiprocessors, which leaves the chain's
 # kernels room; the routed experts' products follow on the first stream.
 SIDE_GRID_SHARE = 0.88
-# Steps of so many rows and more take the shared expert's second product as one sum over its chunks.  Fewer rows give that
-# sum fewer tiles than there are multiprocessors, it is split again and the second kernel that adds the parts costs what was
-# gained (508 rows of the A2.7B sizes, eight layers: 2.61 -> 2.67 ms; 2,048 rows, 24 layers: 13.85 -> 13.62).
-ONE_SUM_MIN_ROWS = 1536
 # Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, go without a permutation, if the
 # experts are no larger than FEW_EXPERT_SIZE (hidden x inner).  Measured per pass of eight steps, with and without: A2.7B sizes
 # (eight pairs a row), eight layers, one row 5.07 and 5.83 ms, two 6.22 and 6.51, three 7.26 and 7.06, four 8.19 and 7.50
@@ -274,22 +270,21 @@ class SparseMoeSwiGLU(FeedForward):
         else:
             self.virtual = 0
 
-    def _alignment(self, TK, n_experts, device, fast, TK_listed, n_listed):
-        """Buffers for ``TK_listed`` pairs over ``n_listed`` experts; the tiles follow the products' pairs and experts."""
+    def _alignment(self, TK, n_experts, device, fast):
         if fast:    # the down product's tile is the primary list, the SwiGLU product may want a wider one
             sizes = dict(hidden=self.hidden, inter=self.inter)
             tile_m = ops.grouped_token_tile(TK, n_experts, **sizes)
             tile_m2 = ops.grouped_token_tile(TK, n_experts, swiglu=True, **sizes)
         else:
             tile_m, tile_m2 = ops.gemm_plain_tile_m(), 0
-        key = (TK_listed, n_listed, tile_m, tile_m2)
+        key = (TK, n_experts, tile_m, tile_m2)
         if key in self._captured:
             return self._captured[key]
         al = self._align.pop(key, None)
         if al is None:
             if len(self._align) >= MAX_ALIGNMENTS:
                 self._align.pop(next(iter(self._align)))
-            al = ops.MoeAlignment(TK_listed, n_listed, tile_m, device, tile_m2)
+            al = ops.MoeAlignment(TK, n_experts, tile_m, device, tile_m2)
         if torch.cuda.is_current_stream_capturing():     # a captured step names these buffers by address: kept for good
             self._captured[key] = al
         else:
@@ -314,18 +309,15 @@ class SparseMoeSwiGLU(FeedForward):
                 and ops.few_experts_usable(h, self.w_gate_up, self.w_down, T, self.E, self.K, C, self.hidden, self.inter,
                                            self.groups[0] if self.groups else 0)):
             return self._forward_few(h, logits, gate_logit)
-        many = fast and C and T >= 256
-        # (with many rows the shared expert is one expert of the permutation, however many chunks its products have)
-        V = 1 if many and T >= ONE_SUM_MIN_ROWS else C
-        idx = torch.empty((T, self.K + V), dtype=torch.int32, device=dev)
-        score = torch.empty((T, self.K + V), dtype=torch.float32, device=dev)
-        al = self._alignment(T * KT, self.E + C, dev, fast, T * (self.K + V), self.E + V)
+        idx = torch.empty((T, KT), dtype=torch.int32, device=dev)
+        score = torch.empty((T, KT), dtype=torch.float32, device=dev)
+        al = self._alignment(T * KT, self.E + C, dev, fast)
         groups = self.groups[0] if self.groups else 0
         x_sorted = None
         if (fast and C and T <= SIDE_MAX_ROWS and al.secondary is None
                 and ops.moe_route_small_usable(T, self.E, self.K, C, self.hidden, groups)):
             return self._forward_beside(h, logits, gate_logit, idx, score, al)
-        if many:
+        if fast and C and T >= 256 and al.secondary is None:
             return self._forward_beside(h, logits, gate_logit, idx, score, al, many=True)
         # (the products' CTAs take their tiles from a counter, as in _forward_beside, unless a handful of pairs split K)
         c0 = c1 = zero = None
@@ -377,15 +369,9 @@ class SparseMoeSwiGLU(FeedForward):
         routing and the row copy, which keep few multiprocessors busy; the routed experts' products follow on the
         first stream and write the other rows of the same two buffers.  Few rows (decoding): one launch routes.
         ``many`` rows (a prompt): the routing is three kernels that take a tenth of the layer's time, and the side
-        products leave them some multiprocessors.
-
-        Many rows: the chunks' second products are one sum over all chunks (``gemm_fast_segments``), a row of the result for
-        every row of the batch, and the permutation knows the shared expert as one more expert that all rows visit.  The
-        chunks' own float32 rows, C of them where there is now one, were written and read back by the norm behind them
-        (2,048 rows of 2,048, four chunks: 100 MB a layer less; the norm 36 -> 31 us; 4,523 rows of 3,584, eight chunks: three
-        layers 14.18 -> 13.75 ms)."""
+        products leave them some multiprocessors."""
         ctx, T, K, C, dev = self.ctx, h.shape[0], self.K, self.virtual, h.device
-        V = idx.shape[1] - K                               # experts that all rows visit, as the permutation knows them
+        KT = K + C
         key = (T, dev)
         st = self._static.get(key)
         if st is None:
@@ -395,8 +381,8 @@ class SparseMoeSwiGLU(FeedForward):
             st = self._static[key] = ops.StaticTiles(T, K, self.E, C, dev, self.hidden, self.inter)
         if torch.cuda.is_current_stream_capturing():       # a captured step names these buffers by address
             self._static_kept.add(key)
-        act = torch.empty((T * (K + C), self.inter), dtype=ctx.act_dtype, device=dev)
-        y = torch.empty((T * (K + V), self.hidden), dtype=torch.float32, device=dev)
+        act = torch.empty((T * KT, self.inter), dtype=ctx.act_dtype, device=dev)
+        y = torch.empty((T * KT, self.hidden), dtype=torch.float32, device=dev)
         main, side = torch.cuda.current_stream(dev), side_stream(dev)
         fork, join = torch.cuda.Event(), torch.cuda.Event()
         fork.record(main)
@@ -405,10 +391,7 @@ class SparseMoeSwiGLU(FeedForward):
         with torch.cuda.stream(side):
             ops.gemm_fast_grouped(h, self.w_gate_up, act, al, swiglu=self.gated, err=ctx.err, tiles=st, tiles_ready=True,
                                   x_rows=st.x_rows, max_ctas=cap, act=self.expert_act)
-            if V == C:
-                ops.gemm_fast_grouped(act, self.w_down, y, al, err=ctx.err, tiles=st, tiles_ready=True, max_ctas=cap)
-            else:
-                ops.gemm_fast_segments(act[T * K:], self.w_down[self.E:], y[T * K:], err=ctx.err, max_ctas=cap)
+            ops.gemm_fast_grouped(act, self.w_down, y, al, err=ctx.err, tiles=st, tiles_ready=True, max_ctas=cap)
             join.record(side)
         # The routed products' CTAs take their tiles from a counter: a prompt's start while the side products still hold
         # most multiprocessors, so the ones that start early do more of the work; a decode step's tiles are one to
@@ -422,8 +405,8 @@ class SparseMoeSwiGLU(FeedForward):
                 self._counters = torch.zeros(2, dtype=torch.int32, device=dev)
             c0, c1 = self._counters[0:1], self._counters[1:2]
         if many:
-            ops.router_topk(logits, K, self.renorm, idx, score, V, gate_logit, rule=self.rule)
-            ops.moe_align(idx, K + V, al, ctx.err, static_last=V, zero=self._counters)
+            ops.router_topk(logits, K, self.renorm, idx, score, C, gate_logit, rule=self.rule)
+            ops.moe_align(idx, KT, al, ctx.err, static_last=C, zero=self._counters)
         else:
             ops.moe_route_small(logits, K, self.renorm, C, gate_logit, idx, score, al, ctx.err, x=None, static=True,
                                 zero=self._counters if c0 is not None else None, rule=self.rule)
@@ -431,9 +414,9 @@ class SparseMoeSwiGLU(FeedForward):
         x_sorted = ops.permute_rows(h, al.sorted_token, T * K)
         ops.gemm_fast_grouped(x_sorted, self.w_gate_up, act, al, swiglu=self.gated, err=ctx.err, tiles_ready=True,
                               counter=c0, act=self.expert_act)
-        ops.gemm_fast_grouped(act[:T * K], self.w_down, y, al, err=ctx.err, tiles_ready=True, counter=c1)
+        ops.gemm_fast_grouped(act, self.w_down, y, al, err=ctx.err, tiles_ready=True, counter=c1)
         main.wait_event(join)
-        return RowMix(y, al.pair_pos[:T * (K + V)].view(T, K + V), score, None, None)
+        return RowMix(y, al.pair_pos[:T * KT].view(T, KT), score, None, None)
 
 
 class _Choices:

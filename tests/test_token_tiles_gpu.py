@@ -73,18 +73,6 @@ def test_fixed_list_in_tiles_of_256():
         held(y[r], act[r].double() @ w2[E + c].double().T, I, f"down {c}")
 
 
-@pytest.mark.parametrize("T,N,K,C", [(1, 136, 72, 2), (130, 264, 200, 3), (300, 520, 1408, 4), (2048, 2048, 136, 5)])
-def test_one_sum_over_segments(T, N, K, C):
-    """A matrix whose columns lie in C blocks: the last k-step of a block is ragged, K is split where that pays."""
-    o = ops()
-    a, w = rnd(C * T, K, seed=5), rnd(C, N, K, seed=6)
-    out = torch.full((T, N), float("nan"), device=DEV)
-    err = o.ErrorFlag(DEV)
-    o.gemm_fast_segments(a, w, out, err=err)
-    err.check("segments")
-    held(out, sum(a[c * T:(c + 1) * T].double() @ w[c].double().T for c in range(C)), C * K, "segments")
-
-
 @pytest.mark.parametrize("T,N,K", [(1, 16, 8), (256, 2048, 64), (300, 200, 64), (1500, 1024, 40)])
 def test_product_of_three_terms(T, N, K):
     """float32 rows on the tensor cores: no further from float64 than a chain of FFMAs, and what is not finite stays so."""
