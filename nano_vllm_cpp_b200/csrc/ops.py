@@ -829,6 +829,22 @@ def few_experts_usable(x, w1, w2, T: int, E: int, K: int, C: int, H: int, I: int
                 and lib().nv_few_experts_usable(T, E, K, C, H, I, groups))
 
 
+def few_experts_pay(T: int, K: int, hidden: int, inter: int) -> bool:
+    """Whether ``few_experts`` is the faster way for T rows that choose K experts of ``inter`` x ``hidden`` each (at most 16 pairs
+    with those of a shared expert's chunks).  It saves launches and the permutation, some 10 us a layer, but reads an expert
+    once for every pair, at a lower rate than the grouped products: what counts is the pairs that are routed, and how much
+    they read.  Measured per layer, graphs of 2 to 16 layers, with it against without, by rows x experts a row (millions of
+    elements that the pairs' matrices of one kind hold): 1 x 4 of 60 (12, and four chunks) 34 and 49 us, 2 x 4 (23, and four
+    chunks) 49 and 56, of 32 (42) 56.2 and 59.3, (50) 71 and 69, (74) 87 and 74; 1 x 8 of 64 (23) 40 and 45, of 32 (42) 55 and
+    60; 1 x 12 (19) 38.6 and 39.2, 1 x 16 (8) 26 and 29, 2 x 5 (5) 22 and 26, 2 x 8 of 128 (25) 52 and 45; 3 x 2 of 8 (18) 35 and 36,
+    of 16 (31) 48 and 47; 4 x 1 of 16 (25) 45 and 47; 4 x 2 of 16 (8) 26 and 28, (17) 36.0 and 35.7, of 8 (24) 41.3 and 40.3; 3 x 4 of
+    64 (19) 42 and 38; 6 x 2 of 8 (35) 57 and 44; 8 x 2 of 8 (8) 34 and 27, of four (47) 67 and 43; 8 x 1 of 64 (4) 29.6 and 28.2."""
+    routed, read = T * K, T * K * hidden * inter
+    if T > 4 or (T > 2 and routed > 8):
+        return False
+    return read <= (44_000_000 if T <= 2 and routed <= 8 else 26_000_000 if routed <= 6 else 16_000_000)
+
+
 def few_experts(x, w1, w2, act, y, logits, K: int, renorm: bool, C: int, gate_logit, idx, score, *, gated=True, fn=None,
                 rule=None) -> None:
     """A whole mixture of experts for a handful of rows in two launches (few_experts.cu): routing (as ``router_topk``, into

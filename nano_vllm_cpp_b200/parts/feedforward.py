@@ -15,13 +15,9 @@ SIDE_MAX_ROWS = 64
 # copy) on a second stream with their grid capped to this share of the multiprocessors, which leaves the chain's
 # kernels room; the routed experts' products follow on the first stream.
 SIDE_GRID_SHARE = 0.88
-# Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, go without a permutation, if the
-# experts are no larger than FEW_EXPERT_SIZE (hidden x inner).  Measured per pass of eight steps, with and without: A2.7B sizes
-# (eight pairs a row), eight layers, one row 5.07 and 5.83 ms, two 6.22 and 6.51, three 7.26 and 7.06, four 8.19 and 7.50
-# (pairs that share an expert each read it); experts of 3,584 x 2,560, sixteen pairs a row, one row 6.46 and 6.42: their
-# products are bound by memory either way.
+# Steps of so many (row, expert) pairs, those of the shared expert's chunks among them, may go without a permutation
+# (``ops.few_experts_pay``).
 FEW_PAIRS = 16
-FEW_EXPERT_SIZE = 6 << 20
 # Permutation buffers are kept per batch size; beyond this many sizes the oldest set is dropped.
 MAX_ALIGNMENTS = 16
 
@@ -305,7 +301,7 @@ class SparseMoeSwiGLU(FeedForward):
             logits = small_linear(ctx, h32, self.router)
         fast = (ctx.fast_kernels and h.dtype == torch.bfloat16 and self.w_gate_up.dtype == torch.bfloat16
                 and self.w_down.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0)
-        if (fast and T * KT <= FEW_PAIRS and self.hidden * self.inter <= FEW_EXPERT_SIZE and (C or not self.shared_inter)
+        if (fast and T * KT <= FEW_PAIRS and ops.few_experts_pay(T, self.K, self.hidden, self.inter) and (C or not self.shared_inter)
                 and ops.few_experts_usable(h, self.w_gate_up, self.w_down, T, self.E, self.K, C, self.hidden, self.inter,
                                            self.groups[0] if self.groups else 0)):
             return self._forward_few(h, logits, gate_logit)

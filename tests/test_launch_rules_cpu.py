@@ -32,6 +32,16 @@ def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
     assert ops.lib().nv_tc_gemm_splits(M, N, K, tile, swiglu, 148) == splits
 
 
+@pytest.mark.parametrize("rows,chosen,hidden,inter,few", [
+    (1, 4, 2048, 1408, True), (2, 4, 2048, 1408, True), (2, 4, 2560, 2048, True), (1, 8, 2048, 1408, True), (1, 8, 2560, 2048, True),
+    (1, 16, 1024, 512, True), (2, 5, 1024, 512, True), (3, 2, 2048, 1408, True), (4, 1, 4096, 1536, True), (4, 2, 1024, 1024, True),
+    (4, 1, 1024, 512, True), (2, 2, 4096, 2048, True), (2, 4, 4096, 1536, False), (2, 4, 3584, 2560, False), (1, 8, 3584, 2560, False),
+    (2, 8, 2048, 768, False), (3, 2, 2560, 2048, False), (3, 4, 2048, 768, False), (4, 2, 2048, 1408, False), (4, 2, 2048, 1024, False),
+    (6, 2, 2048, 1408, False), (8, 2, 2048, 1408, False), (8, 2, 1024, 512, False), (8, 1, 1024, 512, False)])
+def test_a_handful_of_pairs_goes_without_a_permutation_where_that_is_faster(rows, chosen, hidden, inter, few):
+    assert ops.few_experts_pay(rows, chosen, hidden, inter) is few
+
+
 @pytest.mark.parametrize("entries,heads,D,context,mma", [
     (64, 8, 128, 16, True), (24, 8, 128, 64, True), (8, 24, 96, 8, True), (64, 16, 64, 2, True), (64, 16, 64, 32, False),
     (64, 8, 128, 128, False), (8, 8, 128, 16, False), (1, 8, 128, 64, False), (64, 4, 256, 16, False), (24, 8, 128, 202, False)])
