@@ -858,17 +858,16 @@ NV_API int nv_attention_decode_usable(int D, int page, int cache_dt) {
   return decode_stages(page, D, cache_dt == NV_DT_BF16 ? 2 : 4) > 0;
 }
 
-// Number of splits for this many rows.  Blocks are short and all alike, so what counts is how full the last
-// wave of resident blocks is: the split count whose blocks fill whole waves best wins, with a small price per
-// split for its start-up and the merge.  Three blocks of the kernel live on a multiprocessor.
-NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context, int num_sms) {
+namespace {
+// Blocks are short and all alike, so what counts is how full the last wave of resident blocks is: the split count whose blocks
+// fill whole waves best wins, with a small price per split for its start-up and the merge.  Three blocks of the kernel live on
+// a multiprocessor.  A split has at least 256 keys, or at least `one_wave_keys` while all splits run at once.
+int choose_splits(int rows, int Hq, int Hkv, int max_context, int num_sms, int one_wave_keys) {
   const int G = Hq / Hkv;
   const long long slots = 3LL * num_sms;
   const long long blocks = (long long)rows * Hkv * ((G + 15) / 16);
-  // at least 256 keys per split; 128 while all splits run at once (one row of 2,064 keys, 16 heads: 18.6 and 16.4 us; with
-  // several waves of them 8 rows 39 and 49)
   const int usual = (max_context + 255) / 256;
-  int most = max_context / 128 > usual ? max_context / 128 : usual;
+  int most = max_context / one_wave_keys > usual ? max_context / one_wave_keys : usual;
   if (most > MAX_SPLITS) most = MAX_SPLITS;
   int best = 1;
   double best_score = -1.0;
@@ -880,6 +879,19 @@ NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context
     if (score > best_score + 1e-9) { best_score = score; best = s; }
   }
   return best;
+}
+}  // namespace
+
+// Number of splits for this many rows, whatever the heads' size.
+NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context, int num_sms) {
+  return choose_splits(rows, Hq, Hkv, max_context, num_sms, 256);
+}
+
+// The same for heads of D elements: up to 128, splits of 128 keys pay while all of them run at once (one row of 2,064 keys, 16
+// heads: 18.6 and 16.4 us; with several waves of them 8 rows 39 and 49).  Of larger heads one block lives on a multiprocessor,
+// and more blocks are more waves (one kv head of 256 with 16 heads: 64 rows of 500 keys in three splits 36.5 us, in two 24.3).
+NV_API int nv_attention_decode_splits_of(int rows, int Hq, int Hkv, int D, int max_context, int num_sms) {
+  return choose_splits(rows, Hq, Hkv, max_context, num_sms, D <= 128 ? 128 : 256);
 }
 
 // The kernel is launched as a programmatic dependent of the kernel before it on the stream and reads the index

@@ -428,7 +428,7 @@ def attention_decode(qkv, k_cache, v_cache, block_table, row_entry, positions, s
     page = k_cache.shape[2]
     L = lib()
     seen = min([max_context] + [n for n in (window, chunk) if n > 0])        # the most keys a row reads
-    splits = L.nv_attention_decode_splits(R, Hq, Hkv, seen, num_sms())
+    splits = L.nv_attention_decode_splits_of(R, Hq, Hkv, D, seen, num_sms())
     scratch = counts = None
     if splits > 1:
         scratch = torch.empty(R * Hq * splits * (D + 2), dtype=torch.float32, device=qkv.device)

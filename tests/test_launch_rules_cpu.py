@@ -32,6 +32,14 @@ def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
     assert ops.lib().nv_tc_gemm_splits(M, N, K, tile, swiglu, 148) == splits
 
 
+@pytest.mark.parametrize("rows,Hq,Hkv,D,context,splits", [
+    (1, 16, 16, 128, 2064, 16), (1, 28, 4, 128, 4096, 32), (8, 16, 16, 128, 2048, 3), (8, 16, 4, 128, 512, 4), (2, 8, 8, 64, 200, 1),
+    (64, 16, 1, 256, 500, 2), (32, 16, 1, 256, 1000, 4), (12, 16, 1, 256, 2048, 8), (16, 16, 1, 256, 4096, 16), (1, 8, 8, 192, 2048, 8)])
+def test_decode_splits_by_the_heads_size(rows, Hq, Hkv, D, context, splits):
+    assert ops.lib().nv_attention_decode_splits_of(rows, Hq, Hkv, D, context, 148) == splits
+    assert ops.lib().nv_attention_decode_splits(rows, Hq, Hkv, context, 148) <= (context + 255) // 256
+
+
 @pytest.mark.parametrize("rows,chosen,hidden,inter,few", [
     (1, 4, 2048, 1408, True), (2, 4, 2048, 1408, True), (2, 4, 2560, 2048, True), (1, 8, 2048, 1408, True), (1, 8, 2560, 2048, True),
     (1, 16, 1024, 512, True), (2, 5, 1024, 512, True), (3, 2, 2048, 1408, True), (4, 1, 4096, 1536, True), (4, 2, 1024, 1024, True),
