@@ -203,21 +203,30 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // ran 7 % slower with every kernel a dependent), and a launch latency is nothing beside such a kernel's time.
 constexpr unsigned NV_DEP_MAX_BLOCKS = 2048;
 extern int g_nv_dependent_launch;
+// launch_dep_clusters: the same in clusters of `cluster` neighbours in x.
 template <typename... Exp, typename... Act>
-static inline cudaError_t launch_dep(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                     Act&&... args) {
+static inline cudaError_t launch_dep_clusters(unsigned cluster, void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem,
+                                              cudaStream_t stream, Act&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   const unsigned long long blocks = (unsigned long long)grid.x * grid.y * grid.z;
   attr[0].val.programmaticStreamSerializationAllowed = (g_nv_dependent_launch && blocks <= NV_DEP_MAX_BLOCKS) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Exp>(args)...);
+}
+template <typename... Exp, typename... Act>
+static inline cudaError_t launch_dep(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                     Act&&... args) {
+  return launch_dep_clusters(1, kernel, grid, block, smem, stream, std::forward<Act>(args)...);
 }
 #define NV_RETURN_IF(e)                            \
   do {                                             \

@@ -398,25 +398,7 @@ int launch_tiles(const GemmArgs& g, int m_tiles, cudaStream_t s) {
   auto* kernel = gemm_plain_kernel<TA, TW, SWIGLU, FT, CL>;
   if (smem > 48 * 1024) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const dim3 grid((g.N + 16 * FT - 1) / (16 * FT) * CL, m_tiles);
-  if (CL == 1) {
-    NV_RETURN_IF(launch_dep(kernel, grid, dim3(128), smem, s, g));
-    NV_RETURN_LAST();
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed =
-      (g_nv_dependent_launch && (unsigned long long)grid.x * grid.y <= NV_DEP_MAX_BLOCKS) ? 1 : 0;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = CL;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  NV_RETURN_IF(cudaLaunchKernelEx(&cfg, kernel, g));
+  NV_RETURN_IF(launch_dep_clusters(CL, kernel, grid, dim3(128), smem, s, g));
   NV_RETURN_LAST();
 }
 

@@ -664,31 +664,22 @@ template <typename TC, int HB>
 int launch_plain_attention(const void* qkv, int dt, int q_stride, const TC* kc, const TC* vc, const int* block_table,
                            int max_blocks, const int* row_entry, const int* positions, float scale, int window, void* out,
                            int out_dt, int T, int Hq, int Hkv, int D, int page, cudaStream_t s) {
-  // A handful of rows: a cluster each, if the block tables reach beyond a chunk and what a block keeps of its chunks fits
-  // (two decoded rows of 8 heads: 33 us in blocks, 16 in clusters; blocks that fill the GPU by themselves stay alone).
   const long long blocks = (long long)T * (Hq / HB);
-  const long long longest = window > 0 ? min((long long)window, (long long)max_blocks * page) : (long long)max_blocks * page;
-  const long long kept = (longest + ATT_CLUSTER * ATT_THREADS - 1) / (ATT_CLUSTER * ATT_THREADS) * HB * (D + 2) * 4;
-  if (ATT_CLUSTER * blocks <= 4 * num_multiprocessors() && longest > ATT_THREADS && kept <= 64 * 1024) {
-    const size_t smem = 4 * sizeof(KeySlice<TC>) + (size_t)kept;
-    auto* kernel = paged_attention_plain_kernel<TC, HB, 4, ATT_CLUSTER>;
-    NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * sizeof(KeySlice<TC>) + 64 * 1024)));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(T * ATT_CLUSTER, Hq / HB);
-    cfg.blockDim = dim3(ATT_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = g_nv_dependent_launch ? 1 : 0;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = ATT_CLUSTER;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    NV_RETURN_IF(cudaLaunchKernelEx(&cfg, kernel, qkv, dt, q_stride, kc, vc, block_table, max_blocks, row_entry, positions, scale,
-                                    window, out, out_dt, Hq, Hkv, D, page));
-    NV_RETURN_LAST();
+  // A handful of rows: a cluster each, if the block tables reach beyond a chunk and what a block keeps of its chunks fits
+  // (two decoded rows of 8 heads: 33 us in blocks, 16 in clusters; blocks that fill the GPU by themselves stay alone, and so do
+  // those of several heads, of which there are always more than multiprocessors).
+  if constexpr (HB == 1) {
+    const long long longest = window > 0 ? min((long long)window, (long long)max_blocks * page) : (long long)max_blocks * page;
+    const long long kept = (longest + ATT_CLUSTER * ATT_THREADS - 1) / (ATT_CLUSTER * ATT_THREADS) * (D + 2) * 4;
+    if (ATT_CLUSTER * blocks <= 4 * num_multiprocessors() && longest > ATT_THREADS && kept <= 64 * 1024) {
+      const size_t ring = 4 * sizeof(KeySlice<TC>);
+      auto* kernel = paged_attention_plain_kernel<TC, HB, 4, ATT_CLUSTER>;
+      NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ring + 64 * 1024)));
+      NV_RETURN_IF(launch_dep_clusters(ATT_CLUSTER, kernel, dim3(T * ATT_CLUSTER, Hq), dim3(ATT_THREADS), ring + (size_t)kept, s, qkv,
+                                       dt, q_stride, kc, vc, block_table, max_blocks, row_entry, positions, scale, window, out, out_dt,
+                                       Hq, Hkv, D, page));
+      NV_RETURN_LAST();
+    }
   }
   const dim3 grid(T, Hq / HB);
   // (four buffers leave a multiprocessor room for three blocks)
