@@ -402,3 +402,26 @@ def test_product_with_a_matrix_of_the_kernel_in_front():
     o.gemm_plain(a, x, first, w_ready=True)
     for i in range(len(eyes)):
         assert torch.equal(out[i], first * 2.0 ** i)
+
+
+# One case for every rule of the plain product's choice on 148 multiprocessors: narrow blocks of a cluster in one wave, wide
+# ones up to three and a half a multiprocessor, narrow ones up to three and a half waves, wide ones again, whole K; then a K
+# that ends inside a range and ones that leave ranges empty.
+@pytest.mark.parametrize("M,N,K,swiglu", [(40, 96, 512, False), (320, 1024, 1000, False), (400, 1000, 1000, False), (512, 512, 640, True),
+                                          (600, 1000, 516, False), (1400, 1000, 544, False), (640, 1024, 513, True),
+                                          (1500, 1536, 520, False), (65, 40, 700, True), (50, 100, 300, False), (700, 512, 256, False)])
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_every_form_of_the_plain_product_gives_the_same_bits(M, N, K, swiglu, ta, tw):
+    """A row's bits beside many others are those of the row in a call of two; and the bound of a chain of K / 8 FFMAs and eight
+    sums for each of them."""
+    o = ops()
+    a, w = rnd(M, K, seed=1, dtype=ta), (rnd((2 if swiglu else 1) * N, K, seed=2) * 0.05).to(tw)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    o.gemm_plain(a, w, out, swiglu=swiglu)
+    for r in (0, 31, min(M - 2, 62), M // 2, M - 2):
+        two = torch.empty(2, N, device=DEV)
+        o.gemm_plain(a[r:r + 2], w, two, swiglu=swiglu)
+        assert torch.equal(two, out[r:r + 2])
+    if not swiglu:
+        want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+        assert bool(((out.double() - want).abs() <= (K // 8 + 32 + 8) * 2.0 ** -24 * size).all())
