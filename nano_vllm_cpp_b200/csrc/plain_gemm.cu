@@ -394,7 +394,10 @@ __global__ void __launch_bounds__(256) gemm_few_kernel(GemmArgs g) {
 
 template <typename TA, typename TW, bool SWIGLU, int FT, int CL>
 int launch_tiles(const GemmArgs& g, int m_tiles, cudaStream_t s) {
-  const size_t smem = ST * ((size_t)(SWIGLU ? 32 : 16) * FT * (STEP * sizeof(TW) + 16) + g.rows_alloc * (STEP * sizeof(TA) + 16));
+  size_t smem = ST * ((size_t)(SWIGLU ? 32 : 16) * FT * (STEP * sizeof(TW) + 16) + g.rows_alloc * (STEP * sizeof(TA) + 16));
+  // (a cluster's blocks put two sums of 128 threads x (rows / 8) x FW outputs where the ring was)
+  const size_t sums = (size_t)2 * ((g.rows_alloc + 7) / 8) * (SWIGLU ? 2 * FT : FT) * 128 * sizeof(float);
+  if (CL > 1 && sums > smem) smem = sums;
   auto* kernel = gemm_plain_kernel<TA, TW, SWIGLU, FT, CL>;
   if (smem > 48 * 1024) NV_RETURN_IF(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const dim3 grid((g.N + 16 * FT - 1) / (16 * FT) * CL, m_tiles);
@@ -416,32 +419,44 @@ template <typename TA, typename TW>
 int launch(GemmArgs g, int max_tiles, cudaStream_t s) {
   const bool grouped = g.tile_expert != nullptr;
   const int sms = num_multiprocessors();
-  const bool few = g.M <= FEW_ROWS;
   g.rows_alloc = g.M <= 2 ? 2 : g.M <= 4 ? 4 : g.M <= 8 ? 8 : g.M <= 16 ? 16 : g.M <= 32 ? 32 : BM;
   const long long m_tiles = grouped ? max_tiles : (g.M + BM - 1) / BM;
   if (m_tiles == 0) return NV_OK;
   if (m_tiles > 65535) return NV_ERR_BAD_SIZE;
-  // (with a short K most of the eight warps of the few-row kernel have no range: eight rows, 64 -> 2,048, 6.1 us against 3.9)
-  if (few && g.K >= 256) return g.swiglu ? launch_few<TA, TW, true>(g, m_tiles, s) : launch_few<TA, TW, false>(g, m_tiles, s);
-  // Which blocks, by their number (measured, us; WHOLE_WIDE, SPLIT_WIDE, WHOLE_NARROW, SPLIT_NARROW): a product that would
-  // leave multiprocessors with a block or two shares K among a cluster, in narrow blocks (32 rows, 1,024 -> 1,024: 49, 22,
-  // 33, 14; 408 rows, 1,024 -> 1,536: 94, 82, 78, 68), or in wide ones where these fill one wave of three a multiprocessor
-  // (408 rows, 1,024 -> 1,024: 92, 49, 66, 59).  Many blocks take whole K and are wide (1,500 rows, 1,024 -> 1,536: 156, 174,
-  // 174, 203).  With a short K a block is mostly its epilogue, and narrow ones are spread better (6,737 rows, 64 -> 2,048:
-  // 118, 306, 92, 278).
+  // Which blocks: by their number, every form measured at 1 to 3,000 rows, 64 to 32,000 features and K of 64 to 4,096 (us below:
+  // WHOLE_WIDE, SPLIT_WIDE, WHOLE_NARROW, SPLIT_NARROW, float32, K = 1,024 unless said).  Five narrow blocks live on a multiprocessor
+  // and four wide ones.  A grouped product is taken for its list's most tiles.
   const long long wide = (g.N + (g.swiglu ? 31 : 63)) / (g.swiglu ? 32 : 64) * m_tiles;
   const long long narrow = (g.N + (g.swiglu ? 15 : 31)) / (g.swiglu ? 16 : 32) * m_tiles;
-  if constexpr (sizeof(TA) == 4) {                 // (the shapes of float32 rows: the float32 path and gates)
-    if (g.K >= 512) {
-      if (4 * wide >= 2 * sms && 4 * wide <= 3 * sms + sms / 8)
-        return g.swiglu ? launch_tiles<TA, TW, true, 2, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 4, 4>(g, m_tiles, s);
-      if (2 * narrow <= 7 * sms)
-        return g.swiglu ? launch_tiles<TA, TW, true, 1, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 4>(g, m_tiles, s);
-    }
+  // Up to 16 rows: the kernel of a handful of rows, whose eight warps want a K for each of them (eight rows, 128 -> 1,024: 2.5, 3.5
+  // in tiles; nine rows, 64 -> 2,048: 4.1 and 3.0), but float32 rows from nine on only where there are few blocks (16 rows -> 8,000:
+  // 36, SPLIT_WIDE 20; -> 32,000: 123, WHOLE_WIDE 62; -> 1,024: 9 either way).
+  if (g.M <= FEW_ROWS && (g.K >= 128 || g.M <= 4) && (sizeof(TA) == 2 || g.M <= 8 || narrow < sms))
+    return g.swiglu ? launch_few<TA, TW, true>(g, m_tiles, s) : launch_few<TA, TW, false>(g, m_tiles, s);
+  // Narrow blocks that share K among a cluster, while they run in one wave (192 rows, 1,536: 68, 42, 43, 30; 320 rows, 1,024, 640
+  // blocks: 68, 43, 58, 30; 50 rows, 256 -> 512: 27, 13, 15, 7).  Beyond that wide ones while they are three and a half a
+  // multiprocessor: the fourth costs what a wave costs (408 rows, 1,024: 69, 43, 59, 46; 512 rows, 512 blocks: 68, 44, 59, 50; 576
+  // rows, 576 blocks: 69, 57, 59, 54).  Then narrow ones, which leave less of a last wave (640 rows, 1,024: 91, 64, 74, 57; 896 rows:
+  // 93, 79, 104, 76), until those are three and a half waves; from there wide ones again up to three and a quarter whole blocks a
+  // multiprocessor (1,500 rows, 1,024: 145, 114, 121, 120; 640 rows, 2,048 -> 2,048: 277, 180, 202, 195), after which whole K fills
+  // the multiprocessors as well and needs no exchange (1,500 rows, 1,536: 148, 162, 168, 174).
+  const bool one_wave = 4 * narrow <= 5 * sms;
+  if (g.K >= 512) {
+    if (!one_wave && (8 * wide <= 7 * sms || (2 * narrow > 7 * sms && 4 * wide <= 13 * sms)))
+      return g.swiglu ? launch_tiles<TA, TW, true, 2, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 4, 4>(g, m_tiles, s);
+    if (2 * narrow <= 7 * sms)
+      return g.swiglu ? launch_tiles<TA, TW, true, 1, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 4>(g, m_tiles, s);
+    if (narrow >= 4 * sms)
+      return g.swiglu ? launch_tiles<TA, TW, true, 2, 1>(g, m_tiles, s) : launch_tiles<TA, TW, false, 4, 1>(g, m_tiles, s);
+  } else {
+    if ((g.K >= 256 && one_wave) || (g.K >= 128 && 4 * narrow <= sms))
+      return g.swiglu ? launch_tiles<TA, TW, true, 1, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 4>(g, m_tiles, s);
+    // With a short K a block is mostly its epilogue: blocks of 16 features while there are no more than two a multiprocessor (64
+    // rows, 64 -> 2,048: 6, narrow 8; 200 rows, 128 -> 1,024, bfloat16: 8, narrow 11 and split 12), else narrow ones (6,737 rows, 64 ->
+    // 2,048: 118, 306, 92, 278).
+    if (!g.swiglu && narrow <= sms) return launch_tiles<TA, TW, false, 1, 1>(g, m_tiles, s);
   }
-  if (g.K < 512 || narrow < 4 * sms)
-    return g.swiglu ? launch_tiles<TA, TW, true, 1, 1>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 1>(g, m_tiles, s);
-  return g.swiglu ? launch_tiles<TA, TW, true, 2, 1>(g, m_tiles, s) : launch_tiles<TA, TW, false, 4, 1>(g, m_tiles, s);
+  return g.swiglu ? launch_tiles<TA, TW, true, 1, 1>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 1>(g, m_tiles, s);
 }
 
 }  // namespace

@@ -409,7 +409,9 @@ def test_product_with_a_matrix_of_the_kernel_in_front():
 # that ends inside a range and ones that leave ranges empty.
 @pytest.mark.parametrize("M,N,K,swiglu", [(40, 96, 512, False), (320, 1024, 1000, False), (400, 1000, 1000, False), (512, 512, 640, True),
                                           (600, 1000, 516, False), (1400, 1000, 544, False), (640, 1024, 513, True),
-                                          (1500, 1536, 520, False), (65, 40, 700, True), (50, 100, 300, False), (700, 512, 256, False)])
+                                          (1500, 1536, 520, False), (65, 40, 700, True), (50, 100, 300, False), (700, 512, 256, False),
+                                          (200, 1000, 128, False), (50, 40, 33, True), (64, 2048, 64, False), (300, 1000, 100, False),
+                                          (12, 8000, 256, False), (16, 32000, 512, False), (9, 4100, 36, False)])
 @pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
 def test_every_form_of_the_plain_product_gives_the_same_bits(M, N, K, swiglu, ta, tw):
     """A row's bits beside many others are those of the row in a call of two; and the bound of a chain of K / 8 FFMAs and eight
@@ -418,7 +420,7 @@ def test_every_form_of_the_plain_product_gives_the_same_bits(M, N, K, swiglu, ta
     a, w = rnd(M, K, seed=1, dtype=ta), (rnd((2 if swiglu else 1) * N, K, seed=2) * 0.05).to(tw)
     out = torch.full((M, N), float("nan"), device=DEV)
     o.gemm_plain(a, w, out, swiglu=swiglu)
-    for r in (0, 31, min(M - 2, 62), M // 2, M - 2):
+    for r in (0, min(M - 2, 31), min(M - 2, 62), M // 2, M - 2):
         two = torch.empty(2, N, device=DEV)
         o.gemm_plain(a[r:r + 2], w, two, swiglu=swiglu)
         assert torch.equal(two, out[r:r + 2])
