@@ -15,10 +15,13 @@ from ..csrc import ops
 SKINNY_ROWS = ops.SKINNY_MAX_ROWS
 SKINNY_MAX_BYTES = 128 << 20
 # float32 rows times a bfloat16 matrix with a short K (the second half of a low-rank projection), prompts of a bfloat16 run:
-# three bfloat16 terms on the tensor cores, from so many rows on and up to so long a K.  (6,737 rows, 64 -> 2,048: 97 us in
-# FFMAs, 4 + 22 so; relative error against float64 7.9e-8, 1.06e-7 in FFMAs.  The tensor cores' accumulator loses more with every
-# step: at K = 128 1.26e-7 against 1.11e-7, at 512 4.8e-7 against 1.6e-7.)
+# three bfloat16 terms on the tensor cores, from so many rows on and between these lengths of K.  (6,737 rows, 64 -> 2,048: 97 us in
+# FFMAs, 4 + 22 so.)  Relative error against float64, terms, FFMAs in ranges of 32 and in one chain over K: rows and weights of both
+# signs, K = 16 5.0e-8, 7.4e-8, 7.4e-8, K = 64 7.9e-8, 1.06e-7, 1.44e-7; all positive, K = 8 5.1e-8, 4.7e-8, 4.7e-8, K = 16 5.1e-8,
+# 6.2e-8, 6.2e-8, K = 64 9.4e-8, 7.0e-8, 1.21e-7.  The tensor cores' accumulator loses more with every step: at K = 128 1.26e-7 against
+# 1.11e-7, at 512 4.8e-7 against 1.6e-7.
 TERMS_MIN_ROWS = 256
+TERMS_MIN_K = 16
 TERMS_MAX_K = 64
 
 
@@ -46,7 +49,7 @@ def linear(ctx, a, w, out_dtype, *, bias=None, a_rows=None, swiglu=False, M=None
         return out
     if ctx.fast_kernels and ops.gemm_fast_usable(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu):
         ops.gemm_fast(a, w, out, bias=bias, a_rows=a_rows, swiglu=swiglu, M=M, err=ctx.err, act=act)
-    elif (ctx.fast_kernels and ctx.act_dtype == torch.bfloat16 and M >= TERMS_MIN_ROWS and a.shape[-1] <= TERMS_MAX_K
+    elif (ctx.fast_kernels and ctx.act_dtype == torch.bfloat16 and M >= TERMS_MIN_ROWS and TERMS_MIN_K <= a.shape[-1] <= TERMS_MAX_K
           and M == a.shape[0] and bias is None and a_rows is None and act is None and not swiglu and ops.gemm_terms_usable(a, w, out)):
         ops.gemm_terms(a, w, out, err=ctx.err)
     else:

@@ -121,3 +121,13 @@ def test_product_of_three_terms_with_infinite_weights(K):
     size = (a.double().abs() @ w.double().abs().T)[fine]
     # exact products, K of them with three terms each added in float32 (cut off), of values no larger than their sum of sizes
     assert bool(((out[fine].double() - want).abs() <= 3 * K * 2.0 ** -23 * size).all())
+
+
+def test_a_very_short_k_stays_with_the_chain():
+    """Eight terms of one sign are closer to float64 as one chain of FFMAs."""
+    from test_parts_gpu import ctx_for
+    from nano_vllm_cpp_b200.parts.linear import linear
+    o, a, w = ops(), torch.rand(300, 8, generator=torch.Generator().manual_seed(1)).to(DEV), rnd(256, 8, seed=2).abs()
+    out = torch.empty(300, 256, device=DEV)
+    o.gemm_plain(a, w, out)
+    assert torch.equal(linear(ctx_for(torch.bfloat16), a, w, torch.float32), out)
