@@ -412,8 +412,9 @@ __global__ void __launch_bounds__((WARPS + 1) * 32) attention_decode_kernel(DecA
 // The lane-per-chunk kernel above spends a few hundred instructions per key and page, and on this
 // GPU the instruction issue rate, not memory, then bounds it at about half of the memory speed.
 // Here a warp takes a whole page: S = Q K^T and O += P V are m16n8k16 bf16 MMAs whose 16 rows are
-// the query heads that share the kv head (rows beyond them are zero), about ninety instructions per
-// page.  Pages arrive by tiled TMA copies (boxes of `page` keys x 64 elements, 128-byte swizzle) so
+// the query heads that share the kv head (rows beyond them are zero): some four hundred instructions a
+// page of 16 keys of 128 elements (16 rows of 16 heads, two splits, 512 to 2,048 keys; what a block starts and merges
+// with is 880 more for each of its warps).  Pages arrive by tiled TMA copies (boxes of `page` keys x 64 elements, 128-byte swizzle) so
 // that ldmatrix reads them without bank conflicts; the ring, the split over keys and the merges are
 // those of the kernel above.
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {

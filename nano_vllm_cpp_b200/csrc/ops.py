@@ -1079,11 +1079,13 @@ def channel_scan_usable(dk: int, dv: int) -> bool:
 
 def memory_chunks_pay(T: int, S: int, n_single: int, H: int) -> bool:
     """Whether a step of T rows in S entries, ``n_single`` of them of one row, takes its memories in chunks of eight rows
-    (memory_chunks.cuh).  Chunks halve the time of the longest entry's chain, 0.36 us a row row by row; they cost every entry a
-    record of eight rows and a state read by fewer blocks, which counts where entries fill the GPU.  Measured, row by row
-    against chunks, 16 heads of 128 x 128: one entry of 40 rows 30 and 30 us, of 256 116 and 71; 64 rows beside a portion of
-    40 73 and 130, of 128 126 and 134, of 512 361 and 196; 8 entries of 40 58 and 58, 32 of 17 87 and 110; 2 heads, 64 rows
-    beside 128: 69 and 54.  Over 546 such points the rule is on average within a percent of the faster of both."""
+    (memory_chunks.cuh).  Chunks take less than half the time of the longest entry's chain, 0.36 us a row row by row; they cost
+    every entry a record of eight rows and a state read by fewer blocks, which counts where entries fill the GPU.  Measured, delta
+    rule row by row against chunks, 16 heads of 128 x 128: one entry of 24 rows 16 and 15 us, of 40 22 and 17, of 256 104 and 48; 64
+    rows beside a portion of 40 60 and 118, of 128 109 and 124, of 512 331 and 183; 8 entries of 40 45 and 47, 32 of 17 72 and 97; 2
+    heads, 64 rows beside 128: 57 and 44.  The rule's border was placed by 546 points of chunks that took four columns a lane; with two
+    columns it holds at 51 of 57 points within 8 %, and is late for one entry of 24 to 32 rows (delta rule 19.5 and 16.4, matrix LSTM
+    24.5 and 15.8) and for the LSTM's single rows beside a portion of 40 (32.8 and 27.6)."""
     portions = S - n_single
     return portions > 0 and 8 * (T - n_single) > portions * (240 + S * H)
 
