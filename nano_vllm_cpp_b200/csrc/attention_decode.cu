@@ -86,6 +86,8 @@ constexpr int FEW_SPLITS = 8;
 // The splits of a head added up in their order: m and l of split s at part_ml[2 s], its elements at part_o[s D].  One load after
 // the other from the second-level cache was most of the time of this (eight rows of 16 heads of 256, 17 splits: 20 us).
 //
+// (a caller's scratch starts at any float, so that a pair may lie across eight bytes)
+__device__ __forceinline__ float2 split_ml(const float* p) { return make_float2(__ldcg(p), __ldcg(p + 1)); }
 // Up to eight splits: a thread asks for the weights and its element of every split at once and needs nobody else.
 __device__ __forceinline__ float few_splits_sum(const float* part_ml, const float* part_o, int splits, int D, bool has_sink, float sink,
                                                 float gate) {
@@ -93,7 +95,7 @@ __device__ __forceinline__ float few_splits_sum(const float* part_ml, const floa
   float v[FEW_SPLITS];
 #pragma unroll
   for (int i = 0; i < FEW_SPLITS; ++i) {
-    ml[i] = i < splits ? __ldcg((const float2*)part_ml + i) : make_float2(-1e30f, 0.f);
+    ml[i] = i < splits ? split_ml(part_ml + 2 * i) : make_float2(-1e30f, 0.f);
     v[i] = i < splits ? __ldcg(part_o + (size_t)i * D) : 0.f;
   }
   float mm = ml[0].x, ll = 0.f, o = 0.f;
@@ -112,7 +114,7 @@ __device__ __forceinline__ float few_splits_sum(const float* part_ml, const floa
 // More: one warp works out what the splits weigh in the output, into w[splits] ...
 __device__ __forceinline__ void split_weights(const float* part_ml, int splits, int lane, bool has_sink, float sink, float gate,
                                               float* w) {
-  const float2 ml = lane < splits ? __ldcg((const float2*)part_ml + lane) : make_float2(-1e30f, 0.f);
+  const float2 ml = lane < splits ? split_ml(part_ml + 2 * lane) : make_float2(-1e30f, 0.f);
   const float mm = warp_max(ml.x);
   const float sc = lane < splits ? __expf(ml.x - mm) : 0.f;
   float ll = warp_sum(ml.y * sc);

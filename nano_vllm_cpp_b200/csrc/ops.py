@@ -849,7 +849,8 @@ def few_experts(x, w1, w2, act, y, logits, K: int, renorm: bool, C: int, gate_lo
                 rule=None) -> None:
     """A whole mixture of experts for a handful of rows in two launches (few_experts.cu): routing (as ``router_topk``, into
     ``idx`` and ``score`` [T, K + C]) and first product into ``act`` [T (K + C), I] bfloat16, second product into ``y``
-    [T (K + C), H]; pair (t, k) stands in row t (K + C) + k of both.  ``fn``: as ``act`` of ``gemm_plain``."""
+    [T (K + C), H]; pair (t, k) stands in row t (K + C) + k of both.  ``fn``: as ``act`` of ``gemm_plain``.  The weights are read
+    before the kernel that precedes this on the stream has ended: it may not write them."""
     _cuda_contig(act, y, idx, score, w1, w2)
     T, E = logits.shape
     H, I = x.shape[1], act.shape[1]
@@ -1663,7 +1664,8 @@ def gemm_terms_usable(a, w, out) -> bool:
 def gemm_terms(a, w, out, *, err=None) -> None:
     """``out = a @ w.T`` for float32 ``a`` [T, K] and bfloat16 ``w`` [N, K] on the tensor cores: a value of ``a`` is the sum of
     three bfloat16 terms, to within 2^-132, products of bfloat16 values are exact in float32, and the terms' products are
-    added from the smallest on, in one accumulator.  Infinities and NaN of either operand come out as in ``gemm_plain``."""
+    added from the smallest on, in one accumulator.  Infinities and NaN of either operand come out as in ``gemm_plain``.
+    ``w`` is read ahead, as by ``gemm_fast``."""
     T, K = a.shape
     N = w.shape[0]
     _need(gemm_terms_usable(a, w, out) and w.shape[1] == K and out.shape == (T, N), "product of terms: operands")

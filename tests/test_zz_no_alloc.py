@@ -117,3 +117,17 @@ def test_any_number_of_splits(splits, D):
         out = torch.full((1, Hq * D), float("nan"), dtype=torch.bfloat16, device=DEV)
         assert _call(lib, name, qkv, kc, vc, bt, ent, pos, out, Hq, Hkv, D, page, splits, room) == 0
         assert bool(((out[0].double() - want).abs() <= 2.0 ** -8 * size + 2.0 ** -8 * want.abs() + 1e-5).all()), name
+
+
+@pytest.mark.parametrize("splits", [3, 20, 40])
+def test_scratch_that_starts_at_any_float(splits):
+    """The partial results' place is the caller's: four bytes off changes no bit."""
+    from nano_vllm_cpp_b200.csrc import ops
+    Hq, Hkv, D, page = 4, 2, 64, 16
+    qkv, kc, vc, bt, ent, pos = _setup([1500, 700], Hq, Hkv, D, page, seed=3)
+    room = torch.empty(2 * Hq * splits * (D + 2) + 1, dtype=torch.float32, device=DEV)
+    outs = []
+    for scratch in (room, room[1:]):
+        outs.append(torch.full((2, Hq * D), float("nan"), dtype=torch.bfloat16, device=DEV))
+        assert _call(ops.lib(), "nv_attention_decode", qkv, kc, vc, bt, ent, pos, outs[-1], Hq, Hkv, D, page, splits, scratch) == 0
+    assert torch.equal(outs[0], outs[1]) and bool(outs[0].isfinite().all())
