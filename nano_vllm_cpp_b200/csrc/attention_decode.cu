@@ -86,8 +86,6 @@ constexpr int FEW_SPLITS = 8;
 // The splits of a head added up in their order: m and l of split s at part_ml[2 s], its elements at part_o[s D].  One load after
 // the other from the second-level cache was most of the time of this (eight rows of 16 heads of 256, 17 splits: 20 us).
 //
-// (a caller's scratch starts at any float, so that a pair may lie across eight bytes)
-__device__ __forceinline__ float2 split_ml(const float* p) { return make_float2(__ldcg(p), __ldcg(p + 1)); }
 // Up to eight splits: a thread asks for the weights and its element of every split at once and needs nobody else.
 __device__ __forceinline__ float few_splits_sum(const float* part_ml, const float* part_o, int splits, int D, bool has_sink, float sink,
                                                 float gate) {
@@ -95,7 +93,7 @@ __device__ __forceinline__ float few_splits_sum(const float* part_ml, const floa
   float v[FEW_SPLITS];
 #pragma unroll
   for (int i = 0; i < FEW_SPLITS; ++i) {
-    ml[i] = i < splits ? split_ml(part_ml + 2 * i) : make_float2(-1e30f, 0.f);
+    ml[i] = i < splits ? __ldcg((const float2*)part_ml + i) : make_float2(-1e30f, 0.f);
     v[i] = i < splits ? __ldcg(part_o + (size_t)i * D) : 0.f;
   }
   float mm = ml[0].x, ll = 0.f, o = 0.f;
@@ -114,7 +112,7 @@ __device__ __forceinline__ float few_splits_sum(const float* part_ml, const floa
 // More: one warp works out what the splits weigh in the output, into w[splits] ...
 __device__ __forceinline__ void split_weights(const float* part_ml, int splits, int lane, bool has_sink, float sink, float gate,
                                               float* w) {
-  const float2 ml = lane < splits ? split_ml(part_ml + 2 * lane) : make_float2(-1e30f, 0.f);
+  const float2 ml = lane < splits ? __ldcg((const float2*)part_ml + lane) : make_float2(-1e30f, 0.f);
   const float mm = warp_max(ml.x);
   const float sc = lane < splits ? __expf(ml.x - mm) : 0.f;
   float ll = warp_sum(ml.y * sc);
@@ -134,7 +132,8 @@ __device__ __forceinline__ float split_sum(const float* part_o, const float* w, 
   }
   return o;
 }
-// A caller's choice of more splits than a warp has lanes: one after the other.
+// A caller's choice of more splits than a warp has lanes, or of scratch whose pairs lie across eight bytes: one after the other,
+// float by float.
 __device__ __forceinline__ float many_splits_sum(const float* part_ml, const float* part_o, int splits, int D, bool has_sink, float sink,
                                                  float gate) {
   float mm = -1e30f, ll = 0.f, o = 0.f;
@@ -758,22 +757,22 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __gri
 // Combines the splits of one (row, head) in split order.
 __global__ void attention_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                               const int* __restrict__ rows, void* __restrict__ out, int out_dt,
-                                              int Hq, int D, int splits, int has_sink, float sink, HeadGate gate) {
+                                              int Hq, int D, int splits, int has_sink, float sink, HeadGate gate, int one_by_one) {
   const int r = blockIdx.x, h = blockIdx.y;
   const int t = rows ? rows[r] : r;
   const size_t pi = ((size_t)r * Hq + h) * splits;
   grid_dep_wait();
   grid_dep_launch();
+  if (one_by_one) {
+    for (int d = threadIdx.x; d < D; d += blockDim.x)
+      st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d,
+            many_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
+    return;
+  }
   if (splits <= FEW_SPLITS) {
     for (int d = threadIdx.x; d < D; d += blockDim.x)
       st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d,
             few_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
-    return;
-  }
-  if (splits > MAX_SPLITS) {
-    for (int d = threadIdx.x; d < D; d += blockDim.x)
-      st_dt(out, out_dt, ((size_t)t * Hq + h) * D + d,
-            many_splits_sum(part_ml + pi * 2, part_o + pi * D + d, splits, D, has_sink, sink, head_gate_of(gate, t, h)));
     return;
   }
   __shared__ float w_s[MAX_SPLITS];
@@ -864,19 +863,19 @@ NV_API int nv_attention_decode_usable(int D, int page, int cache_dt) {
 namespace {
 // Blocks are short and all alike, so what counts is how full the last wave of resident blocks is: the split count whose blocks
 // fill whole waves best wins, with a small price per split for its start-up and the merge.  Three blocks of the kernel live on
-// a multiprocessor.  A split has at least 256 keys, or at least `one_wave_keys` while all splits run at once.
-int choose_splits(int rows, int Hq, int Hkv, int max_context, int num_sms, int one_wave_keys) {
+// a multiprocessor.  A split has at least 256 keys, or at least 128 while there are no more than `short_blocks` blocks.
+int choose_splits(int rows, int Hq, int Hkv, int max_context, int num_sms, long long short_blocks) {
   const int G = Hq / Hkv;
   const long long slots = 3LL * num_sms;
   const long long blocks = (long long)rows * Hkv * ((G + 15) / 16);
   const int usual = (max_context + 255) / 256;
-  int most = max_context / one_wave_keys > usual ? max_context / one_wave_keys : usual;
+  int most = max_context / 128 > usual ? max_context / 128 : usual;
   if (most > MAX_SPLITS) most = MAX_SPLITS;
   int best = 1;
   double best_score = -1.0;
   for (int s = 1; s <= most; ++s) {
     const long long ctas = blocks * s;
-    if (s > usual && ctas > slots) break;
+    if (s > usual && ctas > short_blocks) break;
     const long long waves = (ctas + slots - 1) / slots;
     const double score = (double)ctas / ((double)waves * (double)slots) - 0.001 * s;
     if (score > best_score + 1e-9) { best_score = score; best = s; }
@@ -887,14 +886,14 @@ int choose_splits(int rows, int Hq, int Hkv, int max_context, int num_sms, int o
 
 // Number of splits for this many rows, whatever the heads' size.
 NV_API int nv_attention_decode_splits(int rows, int Hq, int Hkv, int max_context, int num_sms) {
-  return choose_splits(rows, Hq, Hkv, max_context, num_sms, 256);
+  return choose_splits(rows, Hq, Hkv, max_context, num_sms, 0);
 }
 
-// The same for heads of D elements: up to 128, splits of 128 keys pay while all of them run at once (one row of 2,064 keys, 16
-// heads: 18.6 and 16.4 us; with several waves of them 8 rows 39 and 49).  Of larger heads one block lives on a multiprocessor,
-// and more blocks are more waves (one kv head of 256 with 16 heads: 64 rows of 500 keys in three splits 36.5 us, in two 24.3).
+// The same for heads of D elements.  Splits of 128 keys pay while all of them run at once (one row of 2,064 keys, 16 heads of 128:
+// 18.6 and 16.4 us; with several waves of them 8 rows 39 and 49).  Of heads above 128 elements that is one block a multiprocessor (16
+// heads of 256 on one kv head: two rows of 1,000 keys 22 and 18 us; 64 rows of 500 keys in three splits 36.5, in two 24.3).
 NV_API int nv_attention_decode_splits_of(int rows, int Hq, int Hkv, int D, int max_context, int num_sms) {
-  return choose_splits(rows, Hq, Hkv, max_context, num_sms, D <= 128 ? 128 : 256);
+  return choose_splits(rows, Hq, Hkv, max_context, num_sms, (D <= 128 ? 3LL : 1LL) * num_sms);
 }
 
 // The kernel is launched as a programmatic dependent of the kernel before it on the stream and reads the index
@@ -946,13 +945,14 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   // the last blocks' sums lengthen the kernel's tail by more than the second kernel's launch costs (measured per
   // decode step: batch 1 507 -> 511 tokens/s, batch 8 2,209 -> 2,212, batch 64 6,252 -> 6,192).
   a.split_count = (split_count && (long long)R * Hq <= split_count_len && R * Hq <= 256) ? split_count : nullptr;
+  const int one_by_one = splits > MAX_SPLITS || ((uintptr_t)a.part_ml & 7) != 0;
   // ... and only while the last block's sum is short: its 160 threads add the block's outputs up one after the other, each
   // with loads from the second-level cache (one row of 4,096 keys, 28 heads of 128 on 4: 33 us so and 24 with the second kernel,
   // which has a block per row and head; 8 rows of 512, 16 heads on 4: 20.5 and 17.4; one row of 2,064, 16 heads on 16: 18.6
   // and 21.5).
   {
     const int heads_per_block = Hq / Hkv < 16 ? Hq / Hkv : 16;
-    if ((long long)heads_per_block * D > 256 || splits > MAX_SPLITS) a.split_count = nullptr;
+    if ((long long)heads_per_block * D > 256 || one_by_one) a.split_count = nullptr;
   }
   a.stages = stages;
   const size_t smem = (size_t)stages * 2 * page * D * esize;
@@ -1020,7 +1020,7 @@ NV_API int nv_attention_decode(const void* qkv, int q_dt, int q_stride, const vo
   if (splits > 1 && !a.split_count) {
     dim3 grid(R, Hq);
     NV_RETURN_IF(launch_dep(attention_decode_merge_kernel, grid, dim3(128), 0, stream, (const float*)a.part_o,
-                            (const float*)a.part_ml, rows, out, out_dt, Hq, D, splits, has_sink, sink_score, a.gate));
+                            (const float*)a.part_ml, rows, out, out_dt, Hq, D, splits, has_sink, sink_score, a.gate, one_by_one));
   }
   NV_RETURN_LAST();
 }

@@ -497,9 +497,6 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
   const int kvh = h0 / (Hq / Hkv);
   const int n = positions[t] + 1;
   const int lo = window > 0 ? max(0, n - window) : 0;
-  // (a cluster is launched for what the table can hold: blocks whose row has no chunk for them leave their place to others, and
-  // nobody waits for them, a barrier of the cluster being one of the threads that have not ended)
-  if (CL > 1 && rank > 0 && lo + rank * ATT_THREADS >= n) return;
   const int* bt = block_table + (size_t)row_entry[t] * max_blocks;
   for (int i = tid; i < HB * D; i += ATT_THREADS) q[i / D][i % D] = ld_dt(qkv, dt, (size_t)t * q_stride + (size_t)h0 * D + i);
   const int slices = (D + ATT_SLICE - 1) / ATT_SLICE;
@@ -617,6 +614,10 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_plain_kernel(
     __syncthreads();
   }
   if (CL > 1) {
+    // A cluster is launched for what the table can hold: blocks whose row had no chunk for them leave their place to others, and
+    // nobody waits for them, a barrier of the cluster being one of the threads that have not ended.  (Asked before the loop, the
+    // same question made the loop a sixth slower.)
+    if (rank > 0 && lo + rank * ATT_THREADS >= n) return;
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank == 0) {
       auto there = [&](const float* at, int q) {

@@ -34,7 +34,8 @@ def test_products_split_k_where_that_is_faster(M, N, K, tile, swiglu, splits):
 
 @pytest.mark.parametrize("rows,Hq,Hkv,D,context,splits", [
     (1, 16, 16, 128, 2064, 16), (1, 28, 4, 128, 4096, 32), (8, 16, 16, 128, 2048, 3), (8, 16, 4, 128, 512, 4), (2, 8, 8, 64, 200, 1),
-    (64, 16, 1, 256, 500, 2), (32, 16, 1, 256, 1000, 4), (12, 16, 1, 256, 2048, 8), (16, 16, 1, 256, 4096, 16), (1, 8, 8, 192, 2048, 8)])
+    (64, 16, 1, 256, 500, 2), (32, 16, 1, 256, 1000, 4), (12, 16, 1, 256, 2048, 12), (16, 16, 1, 256, 4096, 16), (1, 8, 8, 192, 2048, 16),
+    (8, 8, 2, 256, 1000, 7)])
 def test_decode_splits_by_the_heads_size(rows, Hq, Hkv, D, context, splits):
     assert ops.lib().nv_attention_decode_splits_of(rows, Hq, Hkv, D, context, 148) == splits
     assert ops.lib().nv_attention_decode_splits(rows, Hq, Hkv, context, 148) <= (context + 255) // 256
