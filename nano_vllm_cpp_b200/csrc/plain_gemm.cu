@@ -439,10 +439,11 @@ int launch(GemmArgs g, int max_tiles, cudaStream_t s) {
   // rows, 576 blocks: 69, 57, 59, 54).  Then narrow ones, which leave less of a last wave (640 rows, 1,024: 91, 64, 74, 57; 896 rows:
   // 93, 79, 104, 76), until those are three and a half waves; from there wide ones again up to three and a quarter whole blocks a
   // multiprocessor (1,500 rows, 1,024: 145, 114, 121, 120; 640 rows, 2,048 -> 2,048: 277, 180, 202, 195), after which whole K fills
-  // the multiprocessors as well and needs no exchange (1,500 rows, 1,536: 148, 162, 168, 174).
+  // the multiprocessors as well and needs no exchange (1,500 rows, 1,536: 148, 162, 168, 174).  Many experts of a few rows each
+  // gain from this last rule with a long K only (20 pairs of 16 experts, 512 -> 1,024: 13.6, 13.1, 10.4, 14.3).
   const bool one_wave = 4 * narrow <= 5 * sms;
   if (g.K >= 512) {
-    if (!one_wave && (8 * wide <= 7 * sms || (2 * narrow > 7 * sms && 4 * wide <= 13 * sms)))
+    if (!one_wave && (8 * wide <= 7 * sms || (2 * narrow > 7 * sms && 4 * wide <= 13 * sms && (g.K >= 1024 || !grouped))))
       return g.swiglu ? launch_tiles<TA, TW, true, 2, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 4, 4>(g, m_tiles, s);
     if (2 * narrow <= 7 * sms)
       return g.swiglu ? launch_tiles<TA, TW, true, 1, 4>(g, m_tiles, s) : launch_tiles<TA, TW, false, 2, 4>(g, m_tiles, s);
