@@ -1,4 +1,4 @@
-// The two products of a mixture of experts for a handful of (row, expert) pairs (one or two rows while decoding), with
+// The two products of a mixture of experts for a handful of (row, expert) pairs (one to four rows while decoding), with
 // the routing inside the first of them.
 //
 // So few pairs need no permutation: a unit of work is sixteen features of one pair's expert (or of one chunk of the shared
